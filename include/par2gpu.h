@@ -91,8 +91,12 @@ int p2g_last_timing(p2g_ctx *ctx, p2g_timing *out);
  * outputs_per_group outputs (an even number), half a warp per output, and a
  * CTA builds each input's lookup tables once for up to 208 outputs; and the
  * inputs a CTA takes between two of its barriers (0 or 1; 2 in the paired
- * form, which then holds four tables).  No counterpart in par2-rs, whose
- * strategies fix their blocking (avx2.rs:700-701 DEST_BATCH / SRC_BATCH). */
+ * form, which then holds four tables).  A column tile of 256 symbols is the
+ * tensor-core kernel: warps and warps_per_group 16, outputs_per_group the rows
+ * of an output block (a multiple of 16, at most 208), inputs_per_stage 256,
+ * input_splits the parts (1 to 60) that the 60 bit products of a
+ * multiplication are dealt to.  No counterpart in par2-rs, whose strategies
+ * fix their blocking (avx2.rs:700-701 DEST_BATCH / SRC_BATCH). */
 typedef struct {
     int warps;
     int outputs_per_group;
@@ -105,9 +109,12 @@ typedef struct {
 } p2g_plan;
 
 /* Autotuner: times every compiled tile shape (and output-block / input-split
- * choice) of the multiply-accumulate kernel for nin inputs x nout outputs of
+ * choice) of the multiply-accumulate kernels for nin inputs x nout outputs of
  * slice_bytes on synthetic data in the context's scratch (best of `reps`
- * launches each) and makes the fastest the context's plan for that shape.
+ * launches each; table shapes and tensor cores are compared with the conversion
+ * of the slices that each needs) and makes the fastest the context's plan for
+ * that shape.  `ms` is the kernel's time, for the tensor cores with the
+ * conversion.
  * Untuned shapes use a heuristic plan. */
 int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int reps,
                  p2g_plan *best);
@@ -119,7 +126,9 @@ int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int 
  * 8 + 8 table kernel (8 warps x 1-13, 12 warps x 4/6/7/8, 16 warps x 2-5,
  * and 16 warps x 8/10/12 with warps_per_group 2) or its paired form
  * (tile_symbols 512: 8 warps x 14-26 even, 12 warps x 16 outputs per
- * warp; with inputs_per_stage 2: 8 warps x 14/18/22/26, 12 warps x 16). */
+ * warp; with inputs_per_stage 2: 8 warps x 14/18/22/26, 12 warps x 16), and
+ * problems of any size the tensor-core kernel (tile_symbols 256, one shape per
+ * output count: ceil(nout / 208) blocks of equal size rounded up to 16). */
 int p2g_set_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes,
                  const p2g_plan *plan);
 

@@ -217,12 +217,25 @@ static float elapsed(p2g_ctx *ctx, int a, int b)
     return ms;
 }
 
+// After a synchronisation: P2G_ETIMEOUT if a kernel's bounded wait gave up.
+int check_waits(p2g_ctx *ctx)
+{
+    volatile int *err = ctx->wait_err;
+    if (err && *err) {
+        *err = 0;
+        set_error("a bounded wait on the device gave up");
+        return P2G_ETIMEOUT;
+    }
+    return P2G_OK;
+}
+
 // Ends a call: waits for its work and collects the timing.
 static int finish(p2g_ctx *ctx)
 {
     ctx->mark(4);
     P2G_CUDA(cudaStreamSynchronize(ctx->stream));
     P2G_CUDA(cudaGetLastError());
+    P2G_TRY(check_waits(ctx));
     ctx->last = p2g_timing{};
     ctx->last.launches = ctx->launches;
     if (ctx->timing) {
@@ -250,13 +263,10 @@ static int matrix_muladd(p2g_ctx *ctx, const std::vector<uint8_t *> &src,
     memcpy(h + L.a_off, coeff, nin * nout * 2);
     P2G_TRY(upload_params(ctx, L));
     uint8_t *d = ctx->params.as<uint8_t>();
-    P2G_TRY(ctx->recs.ensure(record_bytes(nin, static_cast<int>(nout))));
-    P2G_TRY(records_from_matrix(ctx, reinterpret_cast<const uint16_t *>(d + L.a_off),
-                                static_cast<int>(nin), static_cast<int>(nout),
-                                ctx->recs.as<uint32_t>()));
-    P2G_TRY(muladd_run(ctx, reinterpret_cast<const uint8_t *const *>(d + L.src_off),
-                       static_cast<int>(nin), reinterpret_cast<uint8_t *const *>(d + L.dst_off),
-                       static_cast<int>(nout), bytes, ctx->recs.as<uint32_t>(), mode));
+    MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes);
+    P2G_TRY(mulop_matrix(ctx, op, ctx->recs, reinterpret_cast<const uint16_t *>(d + L.a_off)));
+    P2G_TRY(mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(d + L.src_off), 0,
+                      static_cast<int>(nin), reinterpret_cast<uint8_t *const *>(d + L.dst_off), bytes, mode));
     return P2G_OK;
 }
 
@@ -351,6 +361,13 @@ int p2g_create(int device, p2g_ctx **out)
             rc = P2G_ENOMEM;
             break;
         }
+        if (cudaHostAlloc(&ctx->wait_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+            ctx->wait_err = nullptr;
+            set_error("p2g_create: pinned allocation failed");
+            rc = P2G_ENOMEM;
+            break;
+        }
+        *ctx->wait_err = 0;
         static uint32_t crc_tab[4][256];
         crc32_tables(crc_tab);
         if (cudaMalloc(&ctx->d_crc, sizeof crc_tab) != cudaSuccess ||
@@ -397,6 +414,8 @@ int p2g_destroy(p2g_ctx *ctx)
         cudaFree(ctx->d_exp);
     if (ctx->d_crc)
         cudaFree(ctx->d_crc);
+    if (ctx->wait_err)
+        cudaFreeHost(ctx->wait_err);
     ctx->hash_out.release();
     ctx->wb.release();
     for (p2g::DevBuf &d : ctx->spare)
@@ -481,6 +500,10 @@ int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int 
     int tried = 0;
     P2G_TRY(muladd_autotune(ctx, static_cast<int>(nin), static_cast<int>(nout), slice_bytes,
                             reps, &p, &ms, &tried));
+    if (p.tensor) {
+        *best = p2g_plan{16, p.ereg, 16, p.nblk, p.nsplit, ms, 256, kTensorStage};
+        return P2G_OK;
+    }
     *best = p2g_plan{p.warps, p.paired ? 2 * p.ereg : p.ereg, p.psplit, p.nblk, p.nsplit, ms,
                      p.paired ? 512 : 1024, p.stage};
     return P2G_OK;
@@ -507,7 +530,10 @@ int p2g_set_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes,
     if (p.paired)
         p.ereg = plan->outputs_per_group % 2 ? -1 : plan->outputs_per_group / 2;
     p.stage = plan->inputs_per_stage == 0 ? 1 : plan->inputs_per_stage;
-    if ((plan->tile_symbols != 0 && plan->tile_symbols != 512 && plan->tile_symbols != 1024) ||
+    p.tensor = plan->tile_symbols == 256;
+    if ((p.tensor && (p.warps != 16 || p.psplit != 16 || p.stage != kTensorStage)) ||
+        (plan->tile_symbols != 0 && plan->tile_symbols != 256 && plan->tile_symbols != 512 &&
+         plan->tile_symbols != 1024) ||
         nin > 65535 || nout > 65535 ||
         !plan_valid(p, static_cast<int>(nin), static_cast<int>(nout), slice_bytes)) {
         set_error("p2g_set_plan: warps=%d outputs_per_group=%d warps_per_group=%d blocks=%d "
@@ -574,9 +600,12 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
     // blocks CTAs) about fills the device, so none leaves SMs idle.
     const size_t tiles = (slice_bytes + 2047) / 2048;
     int slabs = 1;
+    MulOp op = mulop(ctx, static_cast<int>(k), static_cast<int>(r), slice_bytes);
     if (groups >= 4 && d_staged) {
-        const p2g::MuladdPlan tp = p2g::choose_plan(ctx, static_cast<int>(k / groups * kTailGroups),
-                                                    static_cast<int>(r), slice_bytes);
+        const p2g::MuladdPlan tp =
+            op.plan.tensor ? op.plan
+                           : p2g::choose_plan(ctx, static_cast<int>(k / groups * kTailGroups),
+                                              static_cast<int>(r), slice_bytes);
         const double waves = static_cast<double>(p2g::plan_tiles(tp, slice_bytes)) * tp.nblk /
                              p2g::plan_slots(ctx, tp);
         slabs = static_cast<int>(std::min<double>(kMaxTailSlabs, std::floor(waves + 0.5)));
@@ -584,7 +613,7 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
             slabs = 1;
     }
     const bool tail = slabs >= 2;
-    const size_t t0 = tail ? k * (groups - kTailGroups) / groups : k, ntail = k - t0;
+    const size_t t0 = tail ? mulop_part(op, groups - kTailGroups, groups) : k, ntail = k - t0;
     std::vector<size_t> cut(slabs + 1);
     for (int q = 0; q <= slabs; ++q)
         cut[q] = q == slabs ? slice_bytes : tiles * q / slabs * 2048;
@@ -626,16 +655,12 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
     }
     P2G_TRY(upload_params(ctx, L));
     uint8_t *dp = ctx->params.as<uint8_t>();
-    P2G_TRY(ctx->recs.ensure(record_bytes(k, static_cast<int>(r))));
-    const size_t rw = static_cast<size_t>(record_words(static_cast<int>(r)));  // per record
-    P2G_TRY(records_par2(ctx, reinterpret_cast<const uint16_t *>(dp + L.a_off),
-                         reinterpret_cast<const uint32_t *>(dp + L.b_off), static_cast<int>(k),
-                         static_cast<int>(r), ctx->recs.as<uint32_t>()));
+    P2G_TRY(mulop_par2(ctx, op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + L.a_off),
+                       reinterpret_cast<const uint32_t *>(dp + L.b_off)));
     const uint8_t *const *d_src = reinterpret_cast<const uint8_t *const *>(dp + L.src_off);
     uint8_t *const *d_dst = reinterpret_cast<uint8_t *const *>(dp + L.dst_off);
     if (groups == 1) {
-        P2G_TRY(muladd_run(ctx, d_src, static_cast<int>(k), d_dst, static_cast<int>(r),
-                           slice_bytes, ctx->recs.as<uint32_t>(), 0));
+        P2G_TRY(mulop_run(ctx, op, d_src, 0, static_cast<int>(k), d_dst, slice_bytes, 0));
     } else {
         // The copies run on the context's side streams.  If a step below
         // fails, the ones already enqueued (some into the caller's host
@@ -643,14 +668,13 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
         const int rc = [&]() -> int {
             const int full = tail ? groups - kTailGroups : groups;
             for (int g = 0; g < full; ++g) {
-                const size_t i0 = k * g / groups, i1 = k * (g + 1) / groups;
+                const size_t i0 = mulop_part(op, g, groups), i1 = mulop_part(op, g + 1, groups);
                 P2G_TRY(copy_slices(s.data() + i0, src + i0, i1 - i0, slice_bytes,
                                     cudaMemcpyHostToDevice, ctx->copy_stream));
                 P2G_CUDA(cudaEventRecord(ctx->pipe_ev[g], ctx->copy_stream));
                 P2G_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->pipe_ev[g], 0));
-                P2G_TRY(muladd_run(ctx, d_src + i0, static_cast<int>(i1 - i0), d_dst,
-                                   static_cast<int>(r), slice_bytes,
-                                   ctx->recs.as<uint32_t>() + i0 * r * rw, g == 0 ? 0 : 1));
+                P2G_TRY(mulop_run(ctx, op, d_src + i0, static_cast<int>(i0), static_cast<int>(i1 - i0),
+                                  d_dst, slice_bytes, g == 0 ? 0 : 1));
             }
             if (tail) {
                 uint8_t *const *tab = reinterpret_cast<uint8_t *const *>(dp + tail_off);
@@ -668,9 +692,8 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
                     P2G_CUDA(cudaEventRecord(up[q], ctx->copy_stream));
                     P2G_CUDA(cudaStreamWaitEvent(ctx->stream, up[q], 0));
                     uint8_t *const *qt = tab + q * (ntail + r);
-                    P2G_TRY(muladd_run(ctx, reinterpret_cast<const uint8_t *const *>(qt),
-                                       static_cast<int>(ntail), qt + ntail, static_cast<int>(r), w,
-                                       ctx->recs.as<uint32_t>() + t0 * r * rw, 1));
+                    P2G_TRY(mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(qt),
+                                      static_cast<int>(t0), static_cast<int>(ntail), qt + ntail, w, 1));
                     P2G_CUDA(cudaEventRecord(done[q], ctx->stream));
                     P2G_CUDA(cudaStreamWaitEvent(ctx->d2h_stream, done[q], 0));
                     for (size_t e = 0; e < r; ++e) {
@@ -869,6 +892,7 @@ int p2g_reconstruction_matrix(p2g_ctx *ctx, size_t k, const uint64_t *missing, s
 struct RepairTail {
     int slabs = 0;             // 0: no slabs
     int groups = 0;            // upload groups in the tail
+    MulOp op;                  // the first pass: RHS ^= V present
     size_t t0 = 0, ntail = 0;  // the tail's present slices [t0, t0 + ntail)
     std::vector<size_t> cut;   // slab q: columns [cut[q], cut[q + 1])
     size_t tab_off = 0;        // per slab: ntail inputs, m RHS, m outputs (device pointers)
@@ -880,7 +904,7 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
                          uint8_t *dp, const ParamLayout &L, size_t exps_off,
                          const uint32_t *exps, uint8_t *const *out,
                          const std::vector<uint8_t *> &os, bool o_st, bool dev,
-                         const RepairTail &tail);
+                         RepairTail &tail);
 
 int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missing, size_t m,
                const uint8_t *const *present, const uint32_t *exps,
@@ -942,13 +966,16 @@ int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missi
     // passes and read-back instead of the whole second pass and the
     // read-back of every output.  Slabs about fill the device each.
     RepairTail tail;
+    tail.op = mulop(ctx, static_cast<int>(np), static_cast<int>(m), slice_bytes);
     const size_t tiles = (slice_bytes + 2047) / 2048;
     if (groups >= 4 && o_st) {
         // the last kTailGroups groups (measured on 2048 x 1 MiB, m = 205:
         // 45.1 ms with 2, 46.7 with 4, 47.7 with 6; 48.8 without slabs)
         const int tg = std::min(kTailGroups, groups - 1);
-        const p2g::MuladdPlan tp = p2g::choose_plan(
-            ctx, static_cast<int>(np / groups * tg), static_cast<int>(m), slice_bytes);
+        const p2g::MuladdPlan tp =
+            tail.op.plan.tensor ? tail.op.plan
+                                : p2g::choose_plan(ctx, static_cast<int>(np / groups * tg),
+                                                   static_cast<int>(m), slice_bytes);
         const double waves = static_cast<double>(p2g::plan_tiles(tp, slice_bytes)) * tp.nblk /
                              p2g::plan_slots(ctx, tp);
         int slabs = static_cast<int>(std::min<double>(kMaxTailSlabs - 1, std::floor(waves + 0.5)));
@@ -961,7 +988,7 @@ int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missi
                 tail.cut.insert(tail.cut.end() - 1, (a + (tiles - a) / 2) * 2048);
             tail.slabs = static_cast<int>(tail.cut.size()) - 1;
             tail.groups = tg;
-            tail.t0 = np * (groups - tg) / groups;
+            tail.t0 = mulop_part(tail.op, groups - tg, groups);
             tail.ntail = np - tail.t0;
             tail.present = present;
             tail.ps = &ps;
@@ -1003,7 +1030,7 @@ int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missi
         P2G_CUDA(cudaEventRecord(ctx->pipe_ev[0], ctx->stream));
         P2G_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->pipe_ev[0], 0));
         for (int g = 0; g < (tail.slabs ? groups - tail.groups : groups); ++g) {
-            const size_t i0 = np * g / groups, i1 = np * (g + 1) / groups;
+            const size_t i0 = mulop_part(tail.op, g, groups), i1 = mulop_part(tail.op, g + 1, groups);
             const int rc = copy_slices(ps.data() + i0, present + i0, i1 - i0, slice_bytes,
                                        cudaMemcpyHostToDevice, ctx->copy_stream);
             if (rc != P2G_OK || cudaEventRecord(ctx->pipe_ev[g], ctx->copy_stream) != cudaSuccess) {
@@ -1031,7 +1058,7 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
                          uint8_t *dp, const ParamLayout &L, size_t exps_off,
                          const uint32_t *exps, uint8_t *const *out,
                          const std::vector<uint8_t *> &os, bool o_st, bool dev,
-                         const RepairTail &tail)
+                         RepairTail &tail)
 {
     const uint32_t *d_exps = reinterpret_cast<const uint32_t *>(dp + exps_off);
     // 1. A^-1 on the device
@@ -1047,31 +1074,25 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
     }
     // 2. RHS = R ^ V * present (by input groups as their uploads land)
     if (np) {
-        P2G_TRY(ctx->recs.ensure(record_bytes(np, static_cast<int>(m))));
-        P2G_TRY(records_par2(ctx, reinterpret_cast<const uint16_t *>(dp + L.b_off), d_exps,
-                             static_cast<int>(np), static_cast<int>(m), ctx->recs.as<uint32_t>()));
+        P2G_TRY(mulop_par2(ctx, tail.op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + L.b_off), d_exps));
         const uint8_t *const *d_src = reinterpret_cast<const uint8_t *const *>(dp + L.src_off);
-        const size_t rw = static_cast<size_t>(record_words(static_cast<int>(m)));
         const int full = tail.slabs ? groups - tail.groups : groups;
         for (int g = 0; g < full; ++g) {
-            const size_t i0 = np * g / groups, i1 = np * (g + 1) / groups;
+            const size_t i0 = mulop_part(tail.op, g, groups), i1 = mulop_part(tail.op, g + 1, groups);
             if (groups > 1)
                 P2G_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->pipe_ev[g], 0));
-            P2G_TRY(muladd_run(ctx, d_src + i0, static_cast<int>(i1 - i0),
-                               reinterpret_cast<uint8_t *const *>(dp + L.dst_off),
-                               static_cast<int>(m), slice_bytes,
-                               ctx->recs.as<uint32_t>() + i0 * m * rw, 1));
+            P2G_TRY(mulop_run(ctx, tail.op, d_src + i0, static_cast<int>(i0), static_cast<int>(i1 - i0),
+                              reinterpret_cast<uint8_t *const *>(dp + L.dst_off), slice_bytes, 1));
         }
     }
     // 3. missing = A^-1 * RHS
-    P2G_TRY(ctx->recs2.ensure(record_bytes(m, static_cast<int>(m))));
-    P2G_TRY(records_from_matrix(ctx, ctx->inv.as<uint16_t>(), static_cast<int>(m),
-                                static_cast<int>(m), ctx->recs2.as<uint32_t>()));
+    MulOp op2 = mulop(ctx, static_cast<int>(m), static_cast<int>(m), slice_bytes);
+    P2G_TRY(mulop_matrix(ctx, op2, ctx->recs2, ctx->inv.as<uint16_t>()));
     if (!tail.slabs) {
-        P2G_TRY(muladd_run(ctx, reinterpret_cast<const uint8_t *const *>(dp + L.dst_off),
-                           static_cast<int>(m),
-                           reinterpret_cast<uint8_t *const *>(dp + L.dst_off + m * sizeof(void *)),
-                           static_cast<int>(m), slice_bytes, ctx->recs2.as<uint32_t>(), 0));
+        P2G_TRY(mulop_run(ctx, op2, reinterpret_cast<const uint8_t *const *>(dp + L.dst_off), 0,
+                          static_cast<int>(m),
+                          reinterpret_cast<uint8_t *const *>(dp + L.dst_off + m * sizeof(void *)),
+                          slice_bytes, 0));
         if (o_st)
             P2G_TRY(unstage(ctx, out, os, m, slice_bytes, dev));
         return finish(ctx);
@@ -1080,7 +1101,6 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
     // slab's right-hand sides, step 3 forms its missing columns, which go
     // back on the read-back stream while the next slab uploads.  (A failed
     // step returns after the copies already enqueued, see p2g_repair.)
-    const size_t rw = static_cast<size_t>(record_words(static_cast<int>(m)));
     uint8_t *const *tab = reinterpret_cast<uint8_t *const *>(dp + tail.tab_off);
     const size_t per = tail.ntail + 2 * m;
     std::vector<const uint8_t *> hs(tail.ntail);
@@ -1097,12 +1117,10 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
         P2G_CUDA(cudaEventRecord(up[q], ctx->copy_stream));
         P2G_CUDA(cudaStreamWaitEvent(ctx->stream, up[q], 0));
         uint8_t *const *qt = tab + q * per;
-        P2G_TRY(muladd_run(ctx, reinterpret_cast<const uint8_t *const *>(qt),
-                           static_cast<int>(tail.ntail), qt + tail.ntail, static_cast<int>(m), w,
-                           ctx->recs.as<uint32_t>() + tail.t0 * m * rw, 1));
-        P2G_TRY(muladd_run(ctx, reinterpret_cast<const uint8_t *const *>(qt + tail.ntail),
-                           static_cast<int>(m), qt + tail.ntail + m, static_cast<int>(m), w,
-                           ctx->recs2.as<uint32_t>(), 0));
+        P2G_TRY(mulop_run(ctx, tail.op, reinterpret_cast<const uint8_t *const *>(qt),
+                          static_cast<int>(tail.t0), static_cast<int>(tail.ntail), qt + tail.ntail, w, 1));
+        P2G_TRY(mulop_run(ctx, op2, reinterpret_cast<const uint8_t *const *>(qt + tail.ntail), 0,
+                          static_cast<int>(m), qt + tail.ntail + m, w, 0));
         P2G_CUDA(cudaEventRecord(done[q], ctx->stream));
         P2G_CUDA(cudaStreamWaitEvent(ctx->d2h_stream, done[q], 0));
         for (size_t j = 0; j < m; ++j) {

@@ -46,6 +46,7 @@ struct MuladdPlan {
     bool small = false;  // small-output tables (set for problems of <= kSmallOutputs outputs)
     bool paired = false; // 512-symbol tiles, two outputs per warp lookup (more than 104 outputs)
     int stage = 1;       // inputs per CTA barrier (2: paired form only)
+    bool tensor = false; // tensor-core products (ereg: rows per block, nblk and nsplit apply)
 };
 
 using PlanKey = std::tuple<int, int, size_t>;  // inputs, outputs, slice bytes
@@ -91,6 +92,8 @@ struct p2g_ctx {
             ev_marked[idx] = true;
         }
     }
+    // pinned host word that a kernel sets when a bounded wait gave up
+    int *wait_err = nullptr;
     // GF(2^16) log / antilog tables on the device (galois/core.rs:49-91)
     uint16_t *d_log = nullptr;
     uint16_t *d_exp = nullptr;
@@ -123,6 +126,8 @@ struct p2g_ctx {
 namespace p2g {
 // Frees the shuffle2x state (mirrors, staging, pool) of a context.
 void deferred_release(p2g_ctx *ctx);
+// After a synchronisation: P2G_ETIMEOUT if a kernel's bounded wait gave up.
+int check_waits(p2g_ctx *ctx);
 }  // namespace p2g
 
 #define P2G_CUDA(call)                                                                  \

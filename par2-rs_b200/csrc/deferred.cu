@@ -418,13 +418,10 @@ int launch_group(p2g_ctx *ctx, Deferred *d, const std::vector<uint8_t *> &srcs,
     uint8_t *dp = d->dpar[slot].as<uint8_t>();
     P2G_CUDA(cudaMemcpyAsync(dp, h, total, cudaMemcpyHostToDevice, ctx->stream));
     P2G_CUDA(cudaEventRecord(d->par_ev[slot], ctx->stream));
-    P2G_TRY(ctx->recs.ensure(record_bytes(nin, static_cast<int>(nout))));
-    P2G_TRY(records_from_matrix(ctx, reinterpret_cast<const uint16_t *>(dp + co),
-                                static_cast<int>(nin), static_cast<int>(nout),
-                                ctx->recs.as<uint32_t>()));
-    return muladd_run(ctx, reinterpret_cast<const uint8_t *const *>(dp + so),
-                      static_cast<int>(nin), reinterpret_cast<uint8_t *const *>(dp + dso),
-                      static_cast<int>(nout), bytes, ctx->recs.as<uint32_t>(), 1);
+    MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes);
+    P2G_TRY(mulop_matrix(ctx, op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + co)));
+    return mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(dp + so), 0, static_cast<int>(nin),
+                     reinterpret_cast<uint8_t *const *>(dp + dso), bytes, 1);
 }
 
 // Runs every recorded product.  ctx->mu held, map write-locked.
@@ -668,6 +665,7 @@ int record(p2g_ctx *ctx, uint16_t *const *dsts, size_t ndst, const uint16_t *con
         sp[i] = back[i].data();
     }
     P2G_CUDA(cudaStreamSynchronize(ctx->stream));
+    P2G_TRY(check_waits(ctx));
     wlock.unlock();
     lock.unlock();
     std::vector<uint16_t> rows(unprep.size() * nsrc);
@@ -821,6 +819,7 @@ int p2g_finish_shuffle2x(p2g_ctx *ctx, uint16_t *data, size_t n)
     P2G_CUDA(cudaMemcpyAsync(data, m.dev, std::min(n * 2, m.bytes), cudaMemcpyDeviceToHost,
                              ctx->stream));
     P2G_CUDA(cudaStreamSynchronize(ctx->stream));
+    P2G_TRY(check_waits(ctx));
     P2G_TRY(retire(ctx, d, static_cast<uint32_t>(id)));
     if (d->live_dsts == 0) {
         // no accumulator left: the remaining sources' mirrors go too

@@ -885,6 +885,8 @@ static int block_outputs(const MuladdPlan &p)
 
 int plan_tiles(const MuladdPlan &p, size_t S)
 {
+    if (p.tensor)
+        return static_cast<int>((tensor_tiles(S) + 1) / 2);
     const size_t tb = p.paired ? kPairTileBytes : kTileBytes;
     return static_cast<int>((S + tb - 1) / tb);
 }
@@ -928,14 +930,14 @@ static int resident_ctas(const MuladdPlan &p)
 int plan_slots(const p2g_ctx *ctx, const MuladdPlan &p)
 {
     const int sms = ctx && ctx->sm_count > 0 ? ctx->sm_count : 148;
-    return sms * resident_ctas(p);
+    return p.tensor ? sms : sms * resident_ctas(p);
 }
 
 MuladdPlan choose_plan(const p2g_ctx *ctx, int nin, int nout, size_t S)
 {
     if (ctx) {
         auto it = ctx->plans.find(plan_key(nin, nout, S));
-        if (it != ctx->plans.end())
+        if (it != ctx->plans.end() && !it->second.tensor)
             return it->second;
     }
     MuladdPlan p;
@@ -985,6 +987,8 @@ MuladdPlan choose_plan(const p2g_ctx *ctx, int nin, int nout, size_t S)
 
 bool plan_valid(const MuladdPlan &p, int nin, int nout, size_t S)
 {
+    if (p.tensor)
+        return p.nblk == tensor_blocks(nout) && p.ereg == tensor_rows(nout) && p.nsplit >= 1 && p.nsplit <= 60;
     if (p.psplit < 1 || p.small != (nout <= kSmallOutputs) || (p.paired && p.small) ||
         (!p.paired && p.stage != 1) || kernel_for(p) == nullptr || p.nblk < 1)
         return false;
@@ -1078,6 +1082,167 @@ int muladd_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *cons
     ctx->mark(2);
     P2G_TRY(launch_kernel(ctx->stream, p, planes, d_recs, nin, nout, T, d_dst, S, mode));
     ++ctx->launches;
+    ctx->mark(3);
+    return P2G_OK;
+}
+
+static MuladdPlan tensor_plan(int sms, int nin, int nout, size_t S)
+{
+    MuladdPlan p;
+    p.tensor = true;
+    p.ereg = tensor_rows(nout);
+    p.nblk = tensor_blocks(nout);
+    p.nsplit = tensor_splits(sms, nin, nout, S);
+    return p;
+}
+
+// SM clocks that a table plan takes (an estimate): the planes' HBM time, then
+// waves of CTAs that each run their inputs and a fixed cost of 17 inputs (20
+// when they fold), as in choose_plan.  Clocks per input of a CTA's 1024 (512)
+// symbols from launches of many waves: 460 + 52 per output with the small
+// tables, whose CTAs share an SM by two, else 1020 + 39 per output.
+static double table_clocks(const p2g_ctx *ctx, const MuladdPlan &p, int nin, int nout, size_t S)
+{
+    const int sms = ctx && ctx->sm_count > 0 ? ctx->sm_count : 148;
+    const long long ctas = static_cast<long long>(plan_tiles(p, S)) * p.nblk * p.nsplit;
+    const int slots = plan_slots(ctx, p);
+    const double per_input = p.small ? (460.0 + 52.0 * nout) * (ctas > sms ? slots / sms : 1)
+                                     : (1020.0 + 39.0 * nout) / p.nblk * (p.paired ? 0.5 : 1.0);
+    const double waves = static_cast<double>((ctas + slots - 1) / slots);
+    return waves * (static_cast<double>(nin) / p.nsplit + (p.nsplit > 1 ? 20.0 : 17.0)) * per_input +
+           45.0 * static_cast<double>(S) / 512 * nin / sms;
+}
+
+// Whether the tensor cores take a problem.  The estimates of both sides are
+// within some 20 % of the clocks measured over 8-8000 inputs, 1-205 outputs and
+// 512 B - 1 MiB, hence the margin of 12 %; the tensor side starts with 34000 more
+// (its coefficient operand, and the launches' latencies: small problems of 45 us
+// are 10-15 us shorter with tables).  On one B200, tables against tensor cores: 2048 x 64 KiB, 205
+// outputs 2300 / 402 us, 13 outputs 335 / 272, 4 outputs 210 / 268; 256 x 64 KiB,
+// 205 outputs 370 / 139, 13 outputs 81 / 81; 64 x 64 KiB, 24 outputs 69 / 77.
+static bool tensor_better(const p2g_ctx *ctx, const MuladdPlan &table, int nin, int nout, size_t S)
+{
+    const int sms = ctx && ctx->sm_count > 0 ? ctx->sm_count : 148;
+    int split = 1;
+    return 1.12 * tensor_clocks(sms, nin, nout, S, &split) + 34000.0 < table_clocks(ctx, table, nin, nout, S);
+}
+
+MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S)
+{
+    MulOp op;
+    op.nin = nin;
+    op.nout = nout;
+    op.S = S;
+    if (ctx) {
+        auto it = ctx->plans.find(plan_key(nin, nout, S));
+        if (it != ctx->plans.end()) {
+            op.plan = it->second;
+            return op;
+        }
+    }
+    const int sms = ctx && ctx->sm_count > 0 ? ctx->sm_count : 148;
+    op.plan = choose_plan(ctx, nin, nout, S);
+    if (nin > 0 && tensor_better(ctx, op.plan, nin, nout, S))
+        op.plan = tensor_plan(sms, nin, nout, S);
+    return op;
+}
+
+int mulop_matrix(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_coeff)
+{
+    P2G_TRY(buf.ensure(op.plan.tensor ? tensor_coef_bytes(op.nin, op.nout) : record_bytes(op.nin, op.nout)));
+    op.coef = buf.as<uint32_t>();
+    if (!op.plan.tensor)
+        return records_from_matrix(ctx, d_coeff, op.nin, op.nout, buf.as<uint32_t>());
+    P2G_TRY(tensor_coef_matrix(ctx->stream, d_coeff, op.nin, op.nout, buf.p));
+    ++ctx->launches;
+    return P2G_OK;
+}
+
+int mulop_par2(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_consts, const uint32_t *d_exps)
+{
+    P2G_TRY(buf.ensure(op.plan.tensor ? tensor_coef_bytes(op.nin, op.nout) : record_bytes(op.nin, op.nout)));
+    op.coef = buf.as<uint32_t>();
+    if (!op.plan.tensor)
+        return records_par2(ctx, d_consts, d_exps, op.nin, op.nout, buf.as<uint32_t>());
+    P2G_TRY(tensor_coef_par2(ctx->stream, d_consts, d_exps, ctx->d_log, ctx->d_exp, op.nin, op.nout, buf.p));
+    ++ctx->launches;
+    return P2G_OK;
+}
+
+int mulop_part(const MulOp &op, int g, int parts)
+{
+    const int i = static_cast<int>(static_cast<long long>(op.nin) * g / parts);
+    // the tensor products take inputs 64 at a time
+    return op.plan.tensor && g < parts ? i / 64 * 64 : i;
+}
+
+// Scratch of the tensor products' symbol operand, at most (larger problems
+// run in column chunks: the operand is 1.9 times the slices).
+constexpr size_t kMaxFormBytes = 12ull << 30;
+
+static int zero_outputs(p2g_ctx *ctx, uint8_t *const *d_dst, int nout, size_t S)
+{
+    dim3 g(static_cast<unsigned>(std::min<size_t>((S + 4095) / 4096, 1024)), nout);
+    zero_slices<<<g, 256, 0, ctx->stream>>>(d_dst, nout, S);
+    P2G_CUDA(cudaGetLastError());
+    ++ctx->launches;
+    return P2G_OK;
+}
+
+int mulop_run(p2g_ctx *ctx, const MulOp &op, const uint8_t *const *d_src, int i0, int n,
+              uint8_t *const *d_dst, size_t S, int mode)
+{
+    if (op.nout <= 0)
+        return P2G_OK;
+    if (!op.plan.tensor) {
+        // part of the inputs, or of the columns, has a plan of its own
+        const bool whole = i0 == 0 && n == op.nin && S == op.S;
+        return muladd_run(ctx, d_src, n, d_dst, op.nout, S,
+                          op.coef + static_cast<size_t>(i0) * op.nout * record_words(op.nout), mode,
+                          whole ? &op.plan : nullptr);
+    }
+    if (n == 0)
+        return mode == 0 ? zero_outputs(ctx, d_dst, op.nout, S) : P2G_OK;
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    TensorRun r;
+    r.src = d_src;
+    r.dst = d_dst;
+    r.nin_total = op.nin;
+    r.i0 = i0;
+    r.nin = n;
+    r.nout = op.nout;
+    r.S = S;
+    r.coef = op.coef;
+    r.mode = mode;
+    r.split = i0 == 0 && n == op.nin && S == op.S ? op.plan.nsplit : tensor_splits(sms, n, op.nout, S);
+    r.err = ctx->wait_err;
+    // column chunks: whole waves of tile pairs that fit the scratch; smaller
+    // ones when the device has no room for that
+    const size_t tiles = tensor_tiles(S), pair = tensor_form_bytes(n, 2);
+    size_t chunk = tiles;
+    if (tensor_form_bytes(n, tiles) > std::max(kMaxFormBytes, ctx->planes.cap)) {
+        const size_t pairs = std::max<size_t>(1, kMaxFormBytes / pair), wave = static_cast<size_t>(sms);
+        chunk = 2 * (pairs >= wave ? pairs / wave * wave : pairs);
+    }
+    while (ctx->planes.ensure(tensor_form_bytes(n, chunk)) != P2G_OK) {
+        if (chunk <= 2)
+            return P2G_ENOMEM;
+        chunk = std::max<size_t>(2, chunk / 4 * 2);
+        clear_error();
+    }
+    r.forms = ctx->planes.p;
+    ctx->mark(1);
+    for (size_t t0 = 0; t0 < tiles; t0 += chunk) {
+        const size_t nt = std::min(chunk, tiles - t0);
+        P2G_TRY(tensor_forms(ctx->stream, r, t0, nt));
+        if (t0 == 0) {
+            if (r.split > 1 && mode == 0)
+                P2G_TRY(zero_outputs(ctx, d_dst, op.nout, S));
+            ctx->mark(2);
+        }
+        P2G_TRY(tensor_products(ctx->stream, r, t0, nt));
+        ctx->launches += 2;
+    }
     ctx->mark(3);
     return P2G_OK;
 }
@@ -1249,13 +1414,69 @@ int muladd_autotune(p2g_ctx *ctx, int nin, int nout, size_t S, int reps, MuladdP
             best_p = p;
         }
     }
+    // The tensor products, against the best table plan with its bit planes:
+    // both sides with the conversion of the slices that each needs.
+    const int tried_tables = static_cast<int>(cands.size());
+    int tried_tensor = 0;
+    if (rc == P2G_OK) {
+        auto timed = [&](auto &&run) {
+            float t = 1e30f;
+            for (int q = 0; q <= reps && rc == P2G_OK; ++q) {
+                cudaEventRecord(e0, ctx->stream);
+                rc = run();
+                cudaEventRecord(e1, ctx->stream);
+                if (rc == P2G_OK && cudaEventSynchronize(e1) != cudaSuccess) {
+                    set_error("p2g_autotune: %s", cudaGetErrorString(cudaGetLastError()));
+                    rc = P2G_ECUDA;
+                }
+                float ms = 0.f;
+                if (rc == P2G_OK)
+                    cudaEventElapsedTime(&ms, e0, e1);
+                if (q > 0)  // the first is a warm-up
+                    t = std::min(t, ms);
+            }
+            return t;
+        };
+        const float planes_ms = timed([&] {
+            slices_to_planes<<<static_cast<unsigned>((groups + 255) / 256), 256, 0, ctx->stream>>>(
+                d_src, nin, T, S, ctx->planes.as<uint32_t>());
+            return cudaGetLastError() == cudaSuccess ? P2G_OK : P2G_ECUDA;
+        });
+        MulOp op;
+        op.nin = nin;
+        op.nout = nout;
+        op.S = S;
+        op.plan = tensor_plan(sms, nin, nout, S);
+        if (rc == P2G_OK)
+            rc = mulop_matrix(ctx, op, ctx->recs, ctx->coeffs.as<uint16_t>());
+        const int own = op.plan.nsplit;
+        float tensor_ms = 1e30f;
+        int tensor_split = own;
+        for (int ns : {own, 1, 2, 3, 4, 6, 10, 15, 30}) {
+            op.plan.nsplit = ns;
+            if (rc != P2G_OK || !plan_valid(op.plan, nin, nout, S) || (ns == own && tried_tensor))
+                continue;
+            // XOR mode: the atomic folds need no zeroed outputs
+            const float t = timed([&] { return mulop_run(ctx, op, d_src, 0, nin, d_dst, S, 1); });
+            ++tried_tensor;
+            if (t < tensor_ms) {
+                tensor_ms = t;
+                tensor_split = ns;
+            }
+        }
+        if (rc == P2G_OK && tensor_ms < best_t + planes_ms) {
+            best_p = op.plan;
+            best_p.nsplit = tensor_split;
+            best_t = tensor_ms;
+        }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     P2G_TRY(rc);
     ctx->plans[plan_key(nin, nout, S)] = best_p;
     *best = best_p;
     *best_ms = best_t;
-    *tried = static_cast<int>(cands.size());
+    *tried = tried_tables + tried_tensor;
     return P2G_OK;
 }
 

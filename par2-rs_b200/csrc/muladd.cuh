@@ -2,6 +2,7 @@
 #pragma once
 #include "bitslice.cuh"
 #include "common.cuh"
+#include "tensor.cuh"
 
 namespace p2g {
 
@@ -106,8 +107,9 @@ int batch_copy(cudaStream_t st, const uint8_t *const *src, uint8_t *const *dst,
 int batch_muladd(cudaStream_t st, int grid, const BatchProb *probs, const BatchItem *items,
                  int nitems, int *counter, const volatile int *abort);
 
-// The plan for a problem: the context's tuned plan for this shape if there
-// is one, else a heuristic (8 warps, as many outputs per warp as fit).
+// The lookup-table plan for a problem: the context's tuned plan for this
+// shape if there is one, else a heuristic (8 warps, as many outputs per warp as
+// fit).
 MuladdPlan choose_plan(const p2g_ctx *ctx, int nin, int nout, size_t slice_bytes);
 // Column tiles of plan p over slices of S bytes (1024 symbols each, 512 in
 // the paired form); a launch runs tiles x output blocks x input splits CTAs.
@@ -143,6 +145,30 @@ int records_par2(p2g_ctx *ctx, const uint16_t *d_consts, const uint32_t *d_exps,
 int muladd_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *const *d_dst,
                int nout, size_t slice_bytes, const uint32_t *d_recs, int mode,
                const MuladdPlan *plan = nullptr);
+
+// One multiply-accumulate with its coefficients on the device, in the form
+// that the kernel of its plan reads: records for the lookup-table kernels, the
+// 4-bit operand for the tensor cores.  It can be run over parts of its inputs
+// and over column ranges.
+struct MulOp {
+    int nin = 0, nout = 0;
+    size_t S = 0;  // slice bytes the plan is for
+    MuladdPlan plan;
+    const uint32_t *coef = nullptr;
+};
+// Chooses the plan of an nin x nout problem over slices of S bytes (the
+// context's own plan for that shape if it has one, else by the sizes).
+MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S);
+// Writes the coefficients into buf (grown as needed): from a device matrix
+// [nout][nin], or consts[i]^exps[o].
+int mulop_matrix(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_coeff);
+int mulop_par2(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_consts, const uint32_t *d_exps);
+// The input at which part g of `parts` parts of the inputs starts.
+int mulop_part(const MulOp &op, int g, int parts);
+// dst (^)= inputs [i0, i0 + n) of the product over slices of S bytes; d_src
+// holds those n inputs' pointers, i0 is a mulop_part of the op.
+int mulop_run(p2g_ctx *ctx, const MulOp &op, const uint8_t *const *d_src, int i0, int n,
+              uint8_t *const *d_dst, size_t S, int mode);
 
 // The same work as records_from_matrix / muladd_run (store mode) on a given
 // stream with caller-provided scratch: nothing is allocated.  d_planes must
