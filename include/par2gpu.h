@@ -313,11 +313,14 @@ int p2g_batch_destroy(p2g_batch *batch);
  * class, for this context's later batches, the default form (small tables up
  * to 24 outputs, paired above 104, wide between) unless another is at least
  * 3 % faster.  forms_out / ms_out (optional,
- * P2G_BATCH_CLASSES entries) receive the chosen forms and their times. */
+ * P2G_BATCH_CLASSES entries) receive the chosen forms and their times.
+ * Problems that the tensor cores are estimated to be faster on go to them,
+ * whatever the tuned form of their class. */
 int p2g_batch_autotune(p2g_ctx *ctx, int reps, int *forms_out, float *ms_out);
 /* Pins the form per class (P2G_BATCH_CLASSES entries; -1, or forms NULL,
  * restores the heuristic: small tables up to 24 outputs, paired above 104,
- * wide between).  P2G_EINVAL for the small form on a class above 24
+ * wide between, the tensor cores where they are estimated to be faster; no
+ * problem of a context with pinned forms uses the tensor cores).  P2G_EINVAL for the small form on a class above 24
  * outputs. */
 int p2g_batch_set_forms(p2g_ctx *ctx, const int *forms);
 

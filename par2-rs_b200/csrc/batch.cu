@@ -55,6 +55,10 @@ struct Phase {
            zero_len_off = 0;
     int nplanes = 0, nrec = 0, nitems = 0, nzero = 0, grid = 0;
     unsigned long long planes_total = 0, rec_total = 0;
+    // the problems that the tensor cores take
+    size_t tform_off = 0, tcoef_off = 0, tprob_off = 0, titem_off = 0;
+    int ntens = 0, ntitems = 0, trows = 0;
+    unsigned long long tform_ctas = 0, tcoef_threads = 0;
 };
 
 }  // namespace
@@ -163,8 +167,11 @@ int enqueue(p2g_batch *b)
     Phase *ph[2] = {&b->A, &b->B};
     for (int x = 0; x < 2; ++x) {
         Phase &P = *ph[x];
-        if (!P.nitems)
-            continue;
+        P2G_TRY(tensor_batch_forms(st, reinterpret_cast<const TensorFormProb *>(dp(b, P.tform_off)),
+                                   P.ntens, P.tform_ctas));
+        P2G_TRY(tensor_batch_coefs(st, ctx->d_log, ctx->d_exp,
+                                   reinterpret_cast<const TensorCoefProb *>(dp(b, P.tcoef_off)),
+                                   P.ntens, P.tcoef_threads));
         P2G_TRY(batch_planes(st, reinterpret_cast<const PlanesProb *>(dp(b, P.planes_off)),
                              P.nplanes, P.planes_total));
         P2G_TRY(batch_records(st, ctx->d_log, ctx->d_exp,
@@ -175,10 +182,13 @@ int enqueue(p2g_batch *b)
                            P.nzero));
         if (x == 0)
             ctx->mark(2);
+        P2G_TRY(tensor_batch(st, reinterpret_cast<const TensorArgs *>(dp(b, P.tprob_off)),
+                             reinterpret_cast<const TensorItem *>(dp(b, P.titem_off)), P.ntitems,
+                             P.trows, b->abort_dev));
         P2G_TRY(batch_muladd(st, P.grid, reinterpret_cast<const BatchProb *>(dp(b, P.prob_off)),
                              reinterpret_cast<const BatchItem *>(dp(b, P.item_off)), P.nitems,
                              reinterpret_cast<int *>(dp(b, b->counter_off)) + x, b->abort_dev));
-        ctx->launches += 4;
+        ctx->launches += (P.nitems ? 3 : 0) + (P.ntitems ? 3 : 0) + (P.nzero ? 1 : 0);
     }
     ctx->mark(3);
     for (const HashGroup &g : b->hash) {
@@ -200,12 +210,9 @@ struct Prob {
     size_t consts_off, exps_off;
     const uint16_t *coeff;  // device
     int form;               // tile form of the persistent kernel (BatchForm)
+    bool tensor;            // taken by the tensor cores instead
 };
 
-// The tile form for a problem: the context's tuned form for its class if
-// there is one, else small tables up to 24 outputs, the paired form above
-// 104 (one table build per input serves up to 208 outputs) and the 8 + 8
-// tables over 1024-symbol tiles between.
 // Input splits of an item of `unit` cost when the queue aims at items of
 // `target` cost (whole aligned words: S % 4 == 0; at least 16 inputs each).
 int split_for(double unit, double target, int nin, size_t S)
@@ -216,12 +223,59 @@ int split_for(double unit, double target, int nin, size_t S)
     return std::max(1, static_cast<int>(ns));
 }
 
+// The tile form for a problem: the context's tuned form for its class if
+// there is one, else small tables up to 24 outputs, the paired form above
+// 104 (one table build per input serves up to 208 outputs) and the 8 + 8
+// tables over 1024-symbol tiles between.
 int form_for(const p2g_ctx *ctx, int nout, size_t S)
 {
     const int f = ctx->batch_forms[batch_class(nout, S)];
     if (batch_form_valid(f, nout))
         return f;
     return nout <= 24 ? kFormSmall : nout > 104 ? kFormPaired : kFormWide;
+}
+
+// SM clocks per 256 symbols of a problem in the persistent kernel, planes
+// included, from launches of many waves: per input 160 + 13 per output with the
+// small tables, else 300 + 9.7 per output.
+double table_pair_clocks(int nin, int nout)
+{
+    return nin * (nout <= 24 ? 160.0 + 13.0 * nout : 300.0 + 9.7 * nout);
+}
+
+// Marks the problems of a phase that the tensor cores take: those they are
+// estimated at least 12 % faster on (as in the rule of the single calls, without
+// the part-filled waves that a batch does not have), if together they save more
+// than the 20 us of their three further launches.
+void mark_tensor(const p2g_ctx *ctx, std::vector<Prob> &probs, int phase)
+{
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    double saved = 0;
+    for (Prob &p : probs) {
+        if (p.phase != phase)
+            continue;
+        const double pairs = static_cast<double>((p.S + 511) / 512);
+        const double gain = table_pair_clocks(p.nin, p.nout) - 1.12 * tensor_pair_clocks(p.nin, p.nout);
+        p.tensor = gain > 0 && !ctx->batch_pinned;
+        if (p.tensor)
+            saved += gain * pairs / sms;
+    }
+    if (saved < 40000.0)
+        for (Prob &p : probs)
+            if (p.phase == phase)
+                p.tensor = false;
+}
+
+// Bytes of a problem's converted slices and of its coefficients.
+size_t planes_need(const Prob &p)
+{
+    return p.tensor ? tensor_form_bytes(p.nin, tensor_tiles(p.S))
+                    : static_cast<size_t>(p.nin) * ((p.S + 2047) / 2048) * 2048;
+}
+size_t recs_need(const Prob &p)
+{
+    return p.tensor ? tensor_coef_bytes(p.nin, p.nout)
+                    : al256(static_cast<size_t>(p.nin) * p.nout * batch_record_words(p.form) * 4);
 }
 
 // Times each valid form of the persistent kernel on `copies` synthetic
@@ -622,21 +676,31 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     for (Prob &p : probs)
         p.form = form_for(ctx, p.nout, p.S);
-    size_t plane_need = 0, rec_need = 0;
-    for (int x = 0; x < 2; ++x) {
-        size_t pl = 0, rc = 0;
-        for (const Prob &p : probs)
-            if (p.phase == x) {
-                pl += static_cast<size_t>(p.nin) * ((p.S + 2047) / 2048) * 2048;
-                rc += static_cast<size_t>(p.nin) * p.nout * batch_record_words(p.form) * 4;
-            }
-        plane_need = std::max(plane_need, pl);
-        rec_need = std::max(rec_need, rc);
+    mark_tensor(ctx, probs, 0);
+    mark_tensor(ctx, probs, 1);
+    auto scratch = [&] {
+        size_t plane_need = 0, rec_need = 0;
+        for (int x = 0; x < 2; ++x) {
+            size_t pl = 0, rc = 0;
+            for (const Prob &p : probs)
+                if (p.phase == x) {
+                    pl += planes_need(p);
+                    rc += recs_need(p);
+                }
+            plane_need = std::max(plane_need, pl);
+            rec_need = std::max(rec_need, rc);
+        }
+        P2G_TRY(take(ctx, b->planes, plane_need + 256));
+        return take(ctx, b->recs, rec_need + 256);
+    };
+    if (scratch() != P2G_OK) {
+        // the tensor cores' operands take up to twice the planes' room
+        for (Prob &p : probs)
+            p.tensor = false;
+        clear_error();
+        if (int rc = scratch())
+            return fail(rc);
     }
-    if (int rc = take(ctx, b->planes, plane_need + 256))
-        return fail(rc);
-    if (int rc = take(ctx, b->recs, rec_need + 256))
-        return fail(rc);
     b->copy_src_off = img.put(copy_src.data(), copy_src.size() * sizeof(void *));
     b->copy_dst_off = img.put(copy_dst.data(), copy_dst.size() * sizeof(void *));
     b->copy_len_off = img.put(copy_len.data(), copy_len.size() * 8);
@@ -651,6 +715,11 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         std::vector<BatchItem> items;
         std::vector<uint8_t *> zptr;
         std::vector<unsigned long long> zlen;
+        std::vector<TensorFormProb> tf;
+        std::vector<TensorCoefProb> tc;
+        std::vector<TensorArgs> tp;
+        std::vector<TensorItem> titems;
+        int trows = 0;
     } ph[2];
     // the params buffer must exist before pointers into it are formed: the
     // image grows below, so reserve generously and fix the base afterwards
@@ -659,9 +728,12 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         Pending &P = ph[x];
         size_t pl_off = 0, rc_off = 0;
         unsigned long long pl_first = 0, rc_first = 0;
-        double total_cost = 0;
+        unsigned long long tf_first = 0, tc_first = 0;
+        double total_cost = 0, total_clocks = 0;
         for (const Prob &p : probs)
-            if (p.phase == x) {
+            if (p.phase == x && p.tensor) {
+                total_clocks += static_cast<double>((p.S + 511) / 512) * tensor_pair_clocks(p.nin, p.nout);
+            } else if (p.phase == x) {
                 const int blk = batch_block(p.form);
                 const size_t tb = batch_tile_bytes(p.form);
                 total_cost += static_cast<double>(p.nin) * ((p.S + tb - 1) / tb) *
@@ -673,6 +745,67 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
             const Prob &p = probs[pi];
             if (p.phase != x)
                 continue;
+            // outputs that are folded with atomic XOR start at zero
+            auto zero_outputs = [&] {
+                for (int e = 0; e < p.nout; ++e) {
+                    uint8_t *ptr;
+                    memcpy(&ptr, img.bytes.data() + p.dst_off + e * sizeof(void *), sizeof ptr);
+                    P.zptr.push_back(ptr);
+                    P.zlen.push_back(p.S);
+                }
+            };
+            if (p.tensor) {
+                // as above: pointer fields hold image offsets for now
+                TensorFormProb tf{};
+                tf.src = reinterpret_cast<const uint8_t *const *>(p.src_off);
+                tf.forms = reinterpret_cast<uint32_t *>(b->planes.as<uint8_t>() + pl_off);
+                tf.S = p.S;
+                tf.nin = p.nin;
+                tf.first = tf_first;
+                P.tf.push_back(tf);
+                TensorCoefProb tc{};
+                tc.coeff = p.coeff;
+                tc.consts = p.coeff ? nullptr : reinterpret_cast<const uint16_t *>(p.consts_off);
+                tc.exps = p.coeff ? nullptr : reinterpret_cast<const uint32_t *>(p.exps_off);
+                tc.coef = reinterpret_cast<uint4 *>(b->recs.as<uint8_t>() + rc_off);
+                tc.nin = p.nin;
+                tc.nout = p.nout;
+                tc.first = tc_first;
+                P.tc.push_back(tc);
+                TensorArgs a{};
+                a.forms = tf.forms;
+                a.coef = tc.coef;
+                a.dst = reinterpret_cast<uint8_t *const *>(p.dst_off);
+                a.S = p.S;
+                a.tiles = static_cast<int>(tensor_tiles(p.S));
+                a.steps = (p.nin + 63) / 64;
+                a.cwords = tensor_words(p.nin);
+                a.rows = tensor_rows(p.nout);
+                a.nblk = tensor_blocks(p.nout);
+                a.nout = p.nout;
+                a.mode = p.mode;
+                a.err = ctx->wait_err;
+                // parts: items of at most half of an SM's share of the phase
+                a.split = 1;
+                const double share = total_clocks / (2.0 * sms);
+                for (int parts : {2, 3, 4, 5, 6, 10, 12, 15, 20, 30})
+                    if (tensor_item_clocks(p.nin, p.nout, 60 / a.split) > share)
+                        a.split = parts;
+                const int prob = static_cast<int>(P.tp.size());
+                P.tp.push_back(a);
+                for (int pair = 0; pair < (a.tiles + 1) / 2; ++pair)
+                    for (int nb = 0; nb < a.nblk; ++nb)
+                        for (int part = 0; part < a.split; ++part)
+                            P.titems.push_back(TensorItem{prob, pair, nb, part});
+                if (a.split > 1 && p.mode == 0)
+                    zero_outputs();
+                P.trows = std::max(P.trows, a.rows);
+                pl_off += planes_need(p);
+                rc_off += recs_need(p);
+                tf_first += tensor_form_ctas(p.nin, p.S);
+                tc_first += tensor_coef_threads(p.nin, p.nout);
+                continue;
+            }
             const int T = static_cast<int>((p.S + 2047) / 2048);
             PlanesProb pp{};
             pp.S = p.S;
@@ -716,17 +849,10 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
                 for (int ob = 0; ob < bp.nblk; ++ob)
                     for (int sp = 0; sp < bp.nsplit; ++sp)
                         P.items.push_back(BatchItem{bpi, t, ob, sp});
-            if (bp.nsplit > 1 && bp.mode == 0) {
-                // outputs are folded with atomic XOR: start them at zero
-                for (int e = 0; e < p.nout; ++e) {
-                    uint8_t *ptr;
-                    memcpy(&ptr, img.bytes.data() + p.dst_off + e * sizeof(void *), sizeof ptr);
-                    P.zptr.push_back(ptr);
-                    P.zlen.push_back(p.S);
-                }
-            }
-            pl_off += static_cast<size_t>(p.nin) * T * 2048;
-            rc_off += static_cast<size_t>(p.nin) * p.nout * batch_record_words(p.form) * 4;
+            if (bp.nsplit > 1 && bp.mode == 0)
+                zero_outputs();
+            pl_off += planes_need(p);
+            rc_off += recs_need(p);
             pl_first += static_cast<unsigned long long>(p.nin) * T * 32;
             rc_first += static_cast<unsigned long long>(p.nin) * p.nout;
         }
@@ -748,7 +874,19 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         for (size_t i = 0; i < order.size(); ++i)
             sorted[i] = P.items[order[i]];
         P.items.swap(sorted);
+        std::stable_sort(P.titems.begin(), P.titems.end(), [&](const TensorItem &l, const TensorItem &r) {
+            auto clocks = [&](const TensorItem &it) {
+                const TensorArgs &a = P.tp[it.prob];
+                return tensor_item_clocks(a.steps * 64, a.nout, 60 / a.split);
+            };
+            return clocks(l) > clocks(r);
+        });
         Phase &D = x == 0 ? b->A : b->B;
+        D.ntens = static_cast<int>(P.tp.size());
+        D.ntitems = static_cast<int>(P.titems.size());
+        D.trows = P.trows;
+        D.tform_ctas = tf_first;
+        D.tcoef_threads = tc_first;
         D.nplanes = static_cast<int>(P.pl.size());
         D.nrec = static_cast<int>(P.rc.size());
         D.nitems = static_cast<int>(P.items.size());
@@ -765,6 +903,10 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         D.rec_off = img.put(nullptr, ph[x].rc.size() * sizeof(RecProb));
         D.prob_off = img.put(nullptr, ph[x].bp.size() * sizeof(BatchProb));
         D.item_off = img.put(ph[x].items.data(), ph[x].items.size() * sizeof(BatchItem));
+        D.tform_off = img.put(nullptr, ph[x].tf.size() * sizeof(TensorFormProb));
+        D.tcoef_off = img.put(nullptr, ph[x].tc.size() * sizeof(TensorCoefProb));
+        D.tprob_off = img.put(nullptr, ph[x].tp.size() * sizeof(TensorArgs));
+        D.titem_off = img.put(ph[x].titems.data(), ph[x].titems.size() * sizeof(TensorItem));
         D.zero_ptr_off = img.put(ph[x].zptr.data(), ph[x].zptr.size() * sizeof(void *));
         D.zero_len_off = img.put(ph[x].zlen.data(), ph[x].zlen.size() * 8);
     }
@@ -791,6 +933,22 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         }
         for (BatchProb &q : ph[x].bp)
             q.dst = reinterpret_cast<uint8_t *const *>(rebase(q.dst));
+        for (TensorFormProb &q : ph[x].tf)
+            q.src = reinterpret_cast<const uint8_t *const *>(rebase(q.src));
+        for (TensorCoefProb &q : ph[x].tc)
+            if (!q.coeff) {
+                q.consts = reinterpret_cast<const uint16_t *>(rebase(q.consts));
+                q.exps = reinterpret_cast<const uint32_t *>(rebase(q.exps));
+            }
+        for (TensorArgs &q : ph[x].tp)
+            q.dst = reinterpret_cast<uint8_t *const *>(rebase(q.dst));
+        auto table = [&](size_t off, const auto &v) {
+            if (!v.empty())
+                memcpy(img.bytes.data() + off, v.data(), v.size() * sizeof(v[0]));
+        };
+        table(D.tform_off, ph[x].tf);
+        table(D.tcoef_off, ph[x].tc);
+        table(D.tprob_off, ph[x].tp);
         memcpy(img.bytes.data() + D.planes_off, ph[x].pl.data(), ph[x].pl.size() * sizeof(PlanesProb));
         memcpy(img.bytes.data() + D.rec_off, ph[x].rc.data(), ph[x].rc.size() * sizeof(RecProb));
         memcpy(img.bytes.data() + D.prob_off, ph[x].bp.data(), ph[x].bp.size() * sizeof(BatchProb));
@@ -908,6 +1066,7 @@ int p2g_batch_wait(p2g_batch *b)
     P2G_CUDA(cudaEventSynchronize(b->done));
     P2G_CUDA(cudaGetLastError());
     b->launched = false;
+    P2G_TRY(check_waits(ctx));
     if (b->cancelled) {
         for (size_t j = 0; j < b->njobs; ++j)
             b->jobs[j].status = P2G_ECANCELED;
@@ -1005,6 +1164,7 @@ int p2g_batch_set_forms(p2g_ctx *ctx, const int *forms)
     }
     for (int c = 0; c < 8; ++c)
         ctx->batch_forms[c] = forms ? forms[c] : -1;
+    ctx->batch_pinned = forms != nullptr;
     return P2G_OK;
 }
 
@@ -1026,6 +1186,7 @@ int p2g_batch_autotune(p2g_ctx *ctx, int reps, int *forms_out, float *ms_out)
         set_error("p2g_batch_autotune: cudaEventCreate failed");
         return P2G_ECUDA;
     }
+    ctx->batch_pinned = false;
     // representative outputs per class pair, ten inputs per output (a set
     // of 10 % redundancy)
     static const int kOut[4] = {8, 64, 160, 420};

@@ -63,6 +63,7 @@ struct p2g_ctx {
     // tile form of the persistent batch kernel per problem class
     // (p2g_batch_autotune / p2g_batch_set_forms); -1: the heuristic's
     int batch_forms[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
+    bool batch_pinned = false;  // the forms are the caller's, not the tuner's
     int device = 0;
     int sm_count = 0;
     cudaStream_t own_stream = nullptr;  // created with the context

@@ -134,3 +134,63 @@ def test_set_plan_rejects_other_tensor_shapes(ctx):
             ctx.set_plan(300, 205, 4096, warps, rows, blocks, parts, wpg, tile_symbols=256,
                          inputs_per_stage=stage)
         assert ei.value.code == par2gpu.EINVAL
+
+
+def test_batch_problems_on_the_tensor_cores(ctx):
+    """A batch whose large problems go to the tensor cores (in parts, with
+    odd last symbols, next to problems that stay with the tables and to a
+    column range); every job equals the oracle."""
+    import par2gpu
+    import torch
+
+    rng = np.random.default_rng(77)
+    jobs, want, outs, keep = [], [], [], []
+    for k, S, r, cols in [(700, 16386, 120, None), (1500, 4098, 209, None), (64, 2050, 30, None),
+                          (520, 8192, 90, (2048, 6144)), (5, 4096, 1, None)]:
+        src = rng.integers(0, 256, (k, S), dtype=np.uint8)
+        exps = np.arange(r, dtype=np.uint32)
+        pitch = (S + 15) // 16 * 16
+        d = torch.zeros((k, pitch), dtype=torch.uint8, device="cuda")
+        d[:, :S] = torch.from_numpy(src).cuda()
+        o = torch.full((r, pitch), 7, dtype=torch.uint8, device="cuda")
+        job = {"kind": par2gpu.JOB_CREATE, "k": k, "slice_bytes": S,
+               "src": [d[i] for i in range(k)], "exps": exps, "out": [o[e] for e in range(r)]}
+        full = oracle.encode(src, exps)
+        expect = np.full((r, pitch), 7, np.uint8)
+        a, b = cols or (0, S)
+        expect[:, a:b] = full[:, a:b]
+        if cols:
+            job["col_begin"], job["col_end"] = cols
+        jobs.append(job)
+        want.append(expect)
+        outs.append(o)
+        keep.append(d)
+    k, S, m = 900, 8190, 100
+    data = rng.integers(0, 256, (k, S), dtype=np.uint8)
+    exps = np.arange(m, dtype=np.uint32)
+    rec = oracle.encode(data, exps)
+    missing = np.sort(rng.choice(k, m, replace=False))
+    pitch = (S + 15) // 16 * 16
+    d = torch.zeros((k, pitch), dtype=torch.uint8, device="cuda")
+    d[:, :S] = torch.from_numpy(data).cuda()
+    d_rec = torch.zeros((m, pitch), dtype=torch.uint8, device="cuda")
+    d_rec[:, :S] = torch.from_numpy(rec).cuda()
+    o = torch.full((m, pitch), 7, dtype=torch.uint8, device="cuda")
+    lost = set(missing.tolist())
+    jobs.append({"kind": par2gpu.JOB_REPAIR, "k": k, "slice_bytes": S,
+                 "src": [d[i] for i in range(k) if i not in lost], "missing": missing, "exps": exps,
+                 "recovery": [d_rec[j] for j in range(m)], "out": [o[j] for j in range(m)]})
+    expect = np.full((m, pitch), 7, np.uint8)
+    expect[:, :S] = data[missing]
+    want.append(expect)
+    outs.append(o)
+    for graph in (False, True):
+        for o in outs:
+            o.fill_(7)
+        torch.cuda.synchronize()
+        batch = par2gpu.Batch(ctx, jobs, graph=graph)
+        for _ in range(2):
+            assert batch.run() == [par2gpu.OK] * len(jobs)
+        for j, (o, w) in enumerate(zip(outs, want)):
+            assert np.array_equal(o.cpu().numpy(), w), (graph, j)
+        batch.close()
