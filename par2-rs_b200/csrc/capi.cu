@@ -435,6 +435,14 @@ int p2g_destroy(p2g_ctx *ctx)
         cudaStreamSynchronize(ctx->d2h_stream);
         cudaStreamDestroy(ctx->d2h_stream);
     }
+    if (ctx->side_stream) {
+        cudaStreamSynchronize(ctx->side_stream);
+        cudaStreamDestroy(ctx->side_stream);
+    }
+    if (ctx->fork_ev)
+        cudaEventDestroy(ctx->fork_ev);
+    if (ctx->join_ev)
+        cudaEventDestroy(ctx->join_ev);
     if (ctx->cancel_stream) {
         cudaStreamSynchronize(ctx->cancel_stream);
         cudaStreamDestroy(ctx->cancel_stream);

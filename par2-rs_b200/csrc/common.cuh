@@ -74,6 +74,10 @@ struct p2g_ctx {
     cudaStream_t d2h_stream = nullptr;
     // the copy that raises a running batch's abort word (p2g_batch_cancel)
     cudaStream_t cancel_stream = nullptr;
+    // verification beside a batch's multiply-accumulate work (created on
+    // first use, with the events that fork and join it)
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     static constexpr int kPipe = 16;        // input groups of a host encode
     static constexpr int kPipeEvents = 56;  // group events + slab events
     cudaEvent_t pipe_ev[kPipeEvents] = {};

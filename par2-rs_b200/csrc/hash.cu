@@ -153,35 +153,30 @@ __device__ __forceinline__ void hash_block(const uint32_t *stab, uint32_t st[4],
     md5_block(st, x);
 }
 
-__global__ void __launch_bounds__(kHashThreads, 1)
-    hash_slices_kernel(const uint8_t *const *__restrict__ slices, int n, int per_cta, size_t S,
-                       const uint32_t *__restrict__ crc_tables, uint8_t *__restrict__ md5_out,
-                       uint32_t *__restrict__ crc_out)
+// Fills the CTA's copy of the CRC tables (all threads; ends with a barrier).
+__device__ __forceinline__ void load_crc_tables(uint32_t *stab, const uint32_t *__restrict__ crc_tables)
 {
-    extern __shared__ __align__(16) uint32_t stab[];
     for (int idx = threadIdx.x; idx < kCrcTabWords; idx += blockDim.x) {
         const int L = idx & 31, e = (idx >> 5) & 255, T = idx >> 13;
         stab[(crc_base(T, L) | e << 8) >> 2] = crc_tables[T * 256 + e];
     }
     __syncthreads();
+}
+
+// One warp hashes `count` (1 to 32) slices of S bytes, lane L slices[L]; md5
+// and crc are the results' places of slices[0].
+__device__ __forceinline__ void hash_warp(const uint32_t *stab, uint8_t *ring, const uint8_t *const *slices,
+                                          int count, size_t S, uint8_t *md5, uint32_t *crc_out)
+{
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    // this CTA hashes slices [blockIdx * per_cta, end), 32 to a warp
-    const int first = blockIdx.x * per_cta + warp * 32;
-    const int end = min(n, (blockIdx.x + 1) * per_cta);
-    if (first >= end)
-        return;
     const CrcLanes CL{crc_base(0, lane), crc_base(1, lane), crc_base(2, lane), crc_base(3, lane)};
-    uint8_t *ring = reinterpret_cast<uint8_t *>(stab + kCrcTabWords) +
-                    static_cast<size_t>(warp) * kStages * kStageBytes;
     const uint8_t *ptr[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int g = first + 4 * i + (lane >> 3);
-        ptr[i] = g < end ? slices[g] : nullptr;
+        const int g = 4 * i + (lane >> 3);
+        ptr[i] = g < count ? slices[g] : nullptr;
     }
-    const int me = first + lane;
-    const bool active = me < end;
+    const bool active = lane < count;
     uint32_t st[4] = {0x67452301u, 0xefcdab89u, 0x98badcfeu, 0x10325476u};
     uint32_t crc = 0xFFFFFFFFu;
     const size_t nch = S / kChunk;
@@ -223,7 +218,7 @@ __global__ void __launch_bounds__(kHashThreads, 1)
         return;
     // the last S % 128 bytes: one more full 64-byte block if there is one,
     // then the remaining bytes, 0x80, zeros, 64-bit bit length (RFC 1321 3.1-3.2)
-    const uint8_t *t = slices[me] + nch * kChunk;
+    const uint8_t *t = slices[lane] + nch * kChunk;
     size_t rem = S - nch * kChunk;
     uint32_t x[16];
     if (rem >= 64) {
@@ -259,9 +254,43 @@ __global__ void __launch_bounds__(kHashThreads, 1)
     x[14] = static_cast<uint32_t>(bits);
     x[15] = static_cast<uint32_t>(bits >> 32);
     md5_block(st, x);
-    uint4 *o = reinterpret_cast<uint4 *>(md5_out + static_cast<size_t>(me) * 16);
-    *o = make_uint4(st[0], st[1], st[2], st[3]);
-    crc_out[me] = crc ^ 0xFFFFFFFFu;
+    *reinterpret_cast<uint4 *>(md5 + lane * 16) = make_uint4(st[0], st[1], st[2], st[3]);
+    crc_out[lane] = crc ^ 0xFFFFFFFFu;
+}
+
+__device__ __forceinline__ uint8_t *warp_ring(uint32_t *stab)
+{
+    return reinterpret_cast<uint8_t *>(stab + kCrcTabWords) +
+           static_cast<size_t>(threadIdx.x >> 5) * kStages * kStageBytes;
+}
+
+__global__ void __launch_bounds__(kHashThreads, 1)
+    hash_slices_kernel(const uint8_t *const *__restrict__ slices, int n, int per_cta, size_t S,
+                       const uint32_t *__restrict__ crc_tables, uint8_t *__restrict__ md5_out,
+                       uint32_t *__restrict__ crc_out)
+{
+    extern __shared__ __align__(16) uint32_t stab[];
+    load_crc_tables(stab, crc_tables);
+    // this CTA hashes slices [blockIdx * per_cta, end), 32 to a warp
+    const int first = blockIdx.x * per_cta + (threadIdx.x >> 5) * 32;
+    const int end = min(n, (blockIdx.x + 1) * per_cta);
+    if (first < end)
+        hash_warp(stab, warp_ring(stab), slices + first, min(32, end - first), S,
+                  md5_out + static_cast<size_t>(first) * 16, crc_out + first);
+}
+
+// Slices of several sizes in one launch: warps take groups of up to 32 slices
+// of one size, longest first, dealt over the CTAs.
+__global__ void __launch_bounds__(kHashThreads, 1)
+    hash_groups_kernel(const HashWarp *__restrict__ groups, int n, const uint32_t *__restrict__ crc_tables)
+{
+    extern __shared__ __align__(16) uint32_t stab[];
+    load_crc_tables(stab, crc_tables);
+    for (int g = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; g < n; g += gridDim.x * kHashWarps) {
+        const HashWarp h = groups[g];
+        hash_warp(stab, warp_ring(stab), h.slices, h.count, h.S, h.md5, h.crc);
+        __syncwarp();
+    }
 }
 
 void crc32_tables(uint32_t tab[4][256])
@@ -295,6 +324,21 @@ int hash_run(p2g_ctx *ctx, const uint8_t *const *d_slices, int n, size_t S, uint
                                                                   ctx->d_crc, d_md5, d_crc);
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
+    return P2G_OK;
+}
+
+// A group's time is its slices' chain of MD5 blocks whatever else runs, as long
+// as an SM holds no more than about one warp per scheduler: four to a CTA, so
+// that the launch leaves the other SMs to the work it runs beside.
+int hash_groups(cudaStream_t st, int sms, const uint32_t *crc_tables, const HashWarp *d_groups, int n)
+{
+    if (n <= 0)
+        return P2G_OK;
+    const size_t smem = hash_smem_bytes();
+    P2G_CUDA(cudaFuncSetAttribute(hash_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)));
+    hash_groups_kernel<<<std::min(sms, (n + 3) / 4), kHashThreads, smem, st>>>(d_groups, n, crc_tables);
+    P2G_CUDA(cudaGetLastError());
     return P2G_OK;
 }
 

@@ -13,4 +13,16 @@ size_t hash_smem_bytes();
 int hash_run(p2g_ctx *ctx, const uint8_t *const *d_slices, int n, size_t S, uint8_t *d_md5,
              uint32_t *d_crc);
 
+// Up to 32 slices of one size, hashed by one warp; results at md5 (16-byte
+// aligned, 16 bytes a slice) and crc.
+struct HashWarp {
+    const uint8_t *const *slices;
+    size_t S;
+    uint8_t *md5;
+    uint32_t *crc;
+    int count;
+};
+// All groups (a DEVICE array, longest first) in one launch.
+int hash_groups(cudaStream_t st, int sms, const uint32_t *crc_tables, const HashWarp *d_groups, int n);
+
 }  // namespace p2g
