@@ -42,13 +42,19 @@ __constant__ uint32_t kMd5T[64] = {
 
 __device__ __forceinline__ uint32_t rotl(uint32_t x, int s) { return __funnelshift_l(x, x, s); }
 
-// One RFC 1321 block transform of the 16 little-endian words x.
+// One RFC 1321 block transform of the 16 little-endian words x.  The chain
+// through a step is the function of b, an addition, the rotation and the
+// addition of b; the other addends are summed ahead, behind an asm barrier
+// without which the compiler puts them back into the chain (300 slices of 1 MiB:
+// 9.88 -> 9.68 ms, 32000 of 64 KiB: 0.855 -> 0.839).
 __device__ __forceinline__ void md5_block(uint32_t st[4], const uint32_t x[16])
 {
     uint32_t a = st[0], b = st[1], c = st[2], d = st[3];
 #define P2G_STEP(f, a, b, c, d, k, s, i)              \
     {                                                 \
-        a = b + rotl(a + (f) + x[k] + kMd5T[i], s);   \
+        uint32_t p_ = a + x[k] + kMd5T[i];            \
+        asm("" : "+r"(p_));                           \
+        a = b + rotl(p_ + (f), s);                    \
     }
 #pragma unroll
     for (int i = 0; i < 16; i += 4) {
