@@ -198,6 +198,11 @@ __device__ bool cta_gauss_jordan(uint16_t *S, int n, int ld, uint32_t *fcol, uin
     return true;
 }
 
+// Above this size gj_small first copies the antilogarithms into shared memory:
+// the copy takes 15 us of a CTA's time, which a small matrix's few lookups do
+// not repay (3 x 3: 27 us with it, 13 without).
+constexpr int kCopyTableM = 16;
+
 // Whole inversion of a small matrix (m <= kSmallM) by one CTA.
 __global__ void __launch_bounds__(kGjThreads)
     gj_small(const uint16_t *__restrict__ M, int m, int W, uint16_t *__restrict__ inv,
@@ -208,13 +213,15 @@ __global__ void __launch_bounds__(kGjThreads)
     uint16_t *sexp = dyn, *S = dyn + 65536;
     __shared__ uint32_t fcol[kSmallM];
     __shared__ uint32_t lrow[2 * kSmallM];
-    load_exp_table(sexp, gexp);
+    const bool copied = m > kCopyTableM;
+    if (copied)
+        load_exp_table(sexp, gexp);
     for (int idx = threadIdx.x; idx < m * 2 * m; idx += blockDim.x) {
         const int r = idx / (2 * m), j = idx - r * 2 * m;
         S[idx] = M[static_cast<size_t>(r) * W + j];
     }
     __syncthreads();
-    if (!cta_gauss_jordan(S, m, 2 * m, fcol, lrow, sexp, glog, gexp)) {
+    if (!cta_gauss_jordan(S, m, 2 * m, fcol, lrow, copied ? sexp : gexp, glog, gexp)) {
         if (threadIdx.x == 0)
             *status = 1;
         return;
@@ -538,28 +545,16 @@ __global__ void vdm_leaves(const uint16_t *__restrict__ x, int m, uint16_t *__re
     }
 }
 
-// One level of the product tree.  Pin holds monic polynomials of degree G
-// (the last one shorter), each as its G low coefficients at offset g*G;
-// pairs are multiplied into Pout (degree 2G at offset q*2G).  One thread per
-// output coefficient; LP/LPout are the logs of the coefficients.
-__global__ void vdm_level(const uint16_t *__restrict__ Pin, const uint16_t *__restrict__ LPin,
-                          uint16_t *__restrict__ Pout, uint16_t *__restrict__ LPout, int m, int G,
-                          const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp)
+// The products A_i B_j of one output coefficient (level G of the product tree:
+// monic polynomials of degree G, the last one shorter, each as its G low
+// coefficients at offset g*G; pairs are multiplied into degree 2G at offset
+// q*2G): those with i = first, first + step, ...
+__device__ __forceinline__ uint32_t vdm_coefficient(const uint16_t *LA, const uint16_t *LB, int a, int b, int u,
+                                                    int first, int step, const uint16_t *__restrict__ gexp)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m)
-        return;
-    const int base = (t / (2 * G)) * 2 * G, u = t - base;
-    const int a = min(G, m - base), b = max(0, min(G, m - base - G));
-    if (b == 0) {
-        Pout[t] = Pin[t];
-        LPout[t] = LPin[t];
-        return;
-    }
     // c_u = sum_{i+j=u} A_i B_j with A_a = B_b = 1 (u < a + b)
-    const uint16_t *LA = LPin + base, *LB = LPin + base + G;
     uint32_t acc = 0;
-    for (int i = max(0, u - b); i <= min(u, a); ++i) {
+    for (int i = max(0, u - b) + first; i <= min(u, a); i += step) {
         const int j = u - i;
         const uint32_t la = i == a ? 0u : LA[i], lb = j == b ? 0u : LB[j];
         if (la != kNoLog && lb != kNoLog) {
@@ -569,54 +564,212 @@ __global__ void vdm_level(const uint16_t *__restrict__ Pin, const uint16_t *__re
             acc ^= gexp[l];
         }
     }
-    Pout[t] = static_cast<uint16_t>(acc);
-    LPout[t] = acc ? glog[acc] : kNoLog;
+    return acc;
 }
 
-// y * q for a fixed y given as X[i] = y * 2^i (i < 16): the XOR of the X[i]
-// selected by the bits of q, summed in four independent chains.
-__device__ __forceinline__ uint32_t gmul_fixed(const uint32_t X[16], uint32_t q)
+// One level of the product tree, LANES threads per output coefficient (1 for
+// short polynomials; a warp from degree 16 on, where one thread's sum of up to
+// m lookups was the level's time: 43 us for the last of m = 1600).  LP/LPout
+// are the logs of the coefficients.
+template <int LANES>
+__global__ void vdm_level(const uint16_t *__restrict__ Pin, const uint16_t *__restrict__ LPin,
+                          uint16_t *__restrict__ Pout, uint16_t *__restrict__ LPout, int m, int G,
+                          const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp)
 {
-    uint32_t r[4] = {0, 0, 0, 0};
+    const int id = blockIdx.x * blockDim.x + threadIdx.x, t = id / LANES, lane = id % LANES;
+    if (t >= m)
+        return;
+    const int base = (t / (2 * G)) * 2 * G, u = t - base;
+    const int a = min(G, m - base), b = max(0, min(G, m - base - G));
+    uint32_t acc = Pin[t], lacc = LPin[t];
+    if (b != 0) {
+        acc = vdm_coefficient(LPin + base, LPin + base + G, a, b, u, lane, LANES, gexp);
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-        r[i & 3] ^= X[i] & (0u - ((q >> i) & 1u));
-    return (r[0] ^ r[1]) ^ (r[2] ^ r[3]);
+        for (int o = LANES / 2; o > 0; o /= 2)
+            acc ^= __shfl_xor_sync(0xffffffffu, acc, o);
+        lacc = acc ? glog[acc] : kNoLog;
+    }
+    if (lane == 0) {
+        Pout[t] = static_cast<uint16_t>(acc);
+        LPout[t] = static_cast<uint16_t>(lacc);
+    }
 }
 
-// Thread j: Q_j = P / (z + x_j) by synthetic division (q_{m-1} = 1,
-// q_{i-1} = p_i + x_j q_i), written transposed (QT[i][j]), and Q_j(x_j) by
-// Horner in the same pass; scale[j] = x_j^-s / Q_j(x_j).
-__global__ void vdm_quotients(const uint16_t *__restrict__ P, const uint16_t *__restrict__ x,
-                              int m, uint32_t s, uint16_t *__restrict__ QT,
-                              uint16_t *__restrict__ scale, int *__restrict__ status,
-                              const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp)
+// Products by a fixed y: four tables of 16 entries (y times each value of a
+// nibble) in shared memory, one 32-bit column per lane, so that the four
+// lookups of a product are independent and never conflict.  (Sixteen masked
+// XORs per product took 150 clocks of a serial chain; four lookups take 50.)
+constexpr int kNibbleWords = 64 * 32;  // per warp
+__device__ __forceinline__ void nibble_tables(uint32_t *T, int lane, uint32_t y)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= m)
-        return;
-    const uint32_t xj = x[j];
-    uint32_t X[16];
-    X[0] = xj;
 #pragma unroll
-    for (int i = 1; i < 16; ++i)
-        X[i] = ((X[i - 1] << 1) ^ ((X[i - 1] & 0x8000u) ? 0x1100Bu : 0u)) & 0xFFFFu;
-    uint32_t q = 1, h = 1;
-    QT[static_cast<size_t>(m - 1) * m + j] = 1;
-    for (int i = m - 1; i >= 1; --i) {
-        q = __ldg(P + i) ^ gmul_fixed(X, q);
-        QT[static_cast<size_t>(i - 1) * m + j] = static_cast<uint16_t>(q);
-        h = gmul_fixed(X, h) ^ q;
+    for (int t = 0; t < 4; ++t) {
+        T[t * 512 + lane] = 0;
+#pragma unroll
+        for (int bit = 0; bit < 4; ++bit) {
+            for (int e = 0; e < (1 << bit); ++e)
+                T[(t * 16 + (1 << bit) + e) * 32 + lane] = T[(t * 16 + e) * 32 + lane] ^ y;
+            y = (y << 1) ^ ((y & 0x8000u) ? 0x1100Bu : 0u);
+        }
     }
-    if (h == 0 || (xj == 0 && s != 0)) {
-        atomicExch(status, 1);
-        scale[j] = 0;
-        return;
-    }
-    // x_j^-s / h = 2^(-(s log x_j) - log h)  (mod 65535)
+}
+__device__ __forceinline__ uint32_t nibble_product(const uint32_t *T, int lane, uint32_t q)
+{
+    const uint8_t *p = reinterpret_cast<const uint8_t *>(T + lane);
+    auto at = [p](uint32_t off) { return *reinterpret_cast<const uint32_t *>(p + off); };
+    return (at((q << 7) & 0x780u) ^ at(2048 + ((q << 3) & 0x780u))) ^
+           (at(4096 + ((q >> 1) & 0x780u)) ^ at(6144 + ((q >> 5) & 0x780u)));
+}
+
+// x_j^-s / Q_j(x_j), 0 when there is none (singular)
+__device__ __forceinline__ uint32_t vdm_scale(uint32_t xj, uint32_t h, uint32_t s,
+                                              const uint16_t *__restrict__ glog,
+                                              const uint16_t *__restrict__ gexp)
+{
+    if (h == 0 || (xj == 0 && s != 0))
+        return 0;
+    // 2^(-(s log x_j) - log h)  (mod 65535)
     const uint64_t lx = xj ? glog[xj] : 0;
     const uint64_t neg = (lx * s + glog[h]) % 65535u;
-    scale[j] = gexp[neg == 0 ? 0 : 65535u - neg];
+    return gexp[neg == 0 ? 0 : 65535u - neg];
+}
+
+// Q_j = P / (z + x_j) by synthetic division (q_{m-1} = 1, q_{i-1} = p_i + x_j
+// q_i), written transposed (QT[i][j], row stride ld), and Q_j(x_j) by Horner in
+// the same pass; returns vdm_scale.
+__device__ __forceinline__ uint32_t vdm_quotient(const uint16_t *P, uint32_t xj, int j, int m, uint32_t s,
+                                                 uint16_t *QT, int ld, uint32_t *T, int lane,
+                                                 const uint16_t *__restrict__ glog,
+                                                 const uint16_t *__restrict__ gexp)
+{
+    nibble_tables(T, lane, xj);
+    uint32_t q = 1, h = 1;
+    QT[static_cast<size_t>(m - 1) * ld + j] = 1;
+    for (int i = m - 1; i >= 1; --i) {
+        q = P[i] ^ nibble_product(T, lane, q);
+        QT[static_cast<size_t>(i - 1) * ld + j] = static_cast<uint16_t>(q);
+        h = nibble_product(T, lane, h) ^ q;
+    }
+    return vdm_scale(xj, h, s, glog, gexp);
+}
+
+// 32 quotients Q_j and scale[j] per CTA.  Both recurrences are linear, so warp w
+// runs the w-th of kSegs segments of the m - 1 steps: once from zero to learn
+// what the segment adds, and, with the carry x_j^len times the one before plus
+// that, once more to write the coefficients.  (One warp over all steps is a
+// chain of two dependent lookups a step: 92 us for m = 1600.)
+constexpr int kSegs = 16;
+__global__ void __launch_bounds__(kSegs * 32)
+    vdm_quotients(const uint16_t *__restrict__ P, const uint16_t *__restrict__ x, int m, uint32_t s,
+                  uint16_t *__restrict__ QT, uint16_t *__restrict__ scale, int *__restrict__ status,
+                  const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp)
+{
+    __shared__ uint32_t T[kNibbleWords];
+    __shared__ uint32_t part[2][kSegs][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;
+    const uint32_t xj = j < m ? x[j] : 0;
+    if (w == 0)
+        nibble_tables(T, lane, xj);
+    __syncthreads();
+    // segment w: steps i = top, top - 1, ..., top - n + 1
+    const int len = (m - 1 + kSegs - 1) / kSegs;
+    const int top = m - 1 - w * len, n = max(0, min(len, top));
+    uint32_t q = 0;
+    for (int i = top; i > top - n; --i)
+        q = P[i] ^ nibble_product(T, lane, q);
+    part[0][w][lane] = q;
+    __syncthreads();
+    const uint32_t xlen =
+        xj ? gexp[static_cast<uint64_t>(glog[xj]) * static_cast<uint32_t>(len) % 65535u] : 0;
+    q = 1;
+    for (int v = 0; v < w; ++v)
+        q = gmul_alu(xlen, q) ^ part[0][v][lane];
+    if (j < m) {
+        if (w == 0)
+            QT[static_cast<size_t>(m - 1) * m + j] = 1;
+        uint32_t h = 0;
+        for (int i = top; i > top - n; --i) {
+            q = P[i] ^ nibble_product(T, lane, q);
+            QT[static_cast<size_t>(i - 1) * m + j] = static_cast<uint16_t>(q);
+            h = nibble_product(T, lane, h) ^ q;
+        }
+        part[1][w][lane] = h;
+    }
+    __syncthreads();
+    if (w != 0 || j >= m)
+        return;
+    uint32_t h = 1;
+    for (int v = 0; v < kSegs; ++v) {
+        // the last segments may be short or empty
+        const int nv = max(0, min(len, m - 1 - v * len));
+        if (nv == len) {
+            h = gmul_alu(xlen, h);
+        } else {
+            for (int i = 0; i < nv; ++i)
+                h = nibble_product(T, lane, h);
+        }
+        h ^= part[1][v][lane];
+    }
+    const uint32_t sc = vdm_scale(xj, h, s, glog, gexp);
+    scale[j] = static_cast<uint16_t>(sc);
+    if (sc == 0)
+        atomicExch(status, 1);
+}
+
+// The whole inverse for m <= kVdmSmall in one launch of one CTA: the product
+// tree, the quotients and the scaled transpose in shared memory (13 rows: 7
+// launches of 3-7 us each before, 20 us in one).
+constexpr int kVdmSmall = 128;
+constexpr int kVdmQtLd = kVdmSmall + 2;
+struct VdmSmallSmem {
+    uint16_t P[2][kVdmSmall], L[2][kVdmSmall], scale[kVdmSmall];
+    uint32_t T[kVdmSmall / 32 * kNibbleWords];
+    uint16_t QT[kVdmSmall * kVdmQtLd];
+};
+__global__ void __launch_bounds__(kVdmSmall)
+    vdm_small(const uint16_t *__restrict__ x, const uint32_t *__restrict__ exps, uint32_t s, int m, int ld,
+              uint16_t *__restrict__ inv, int *__restrict__ status, const uint16_t *__restrict__ glog,
+              const uint16_t *__restrict__ gexp)
+{
+    extern __shared__ __align__(16) uint8_t raw[];
+    VdmSmallSmem &sm = *reinterpret_cast<VdmSmallSmem *>(raw);
+    const int j = threadIdx.x, lane = j & 31;
+    const uint32_t xj = j < m ? x[j] : 0;
+    if (j < m) {
+        sm.P[0][j] = static_cast<uint16_t>(xj);
+        sm.L[0][j] = xj ? glog[xj] : kNoLog;
+    }
+    __syncthreads();
+    int cur = 0;
+    for (int G = 1; G < m; G *= 2, cur ^= 1) {
+        if (j < m) {
+            const int base = (j / (2 * G)) * 2 * G;
+            const int a = min(G, m - base), b = max(0, min(G, m - base - G));
+            uint32_t acc = sm.P[cur][j], lacc = sm.L[cur][j];
+            if (b != 0) {
+                acc = vdm_coefficient(sm.L[cur] + base, sm.L[cur] + base + G, a, b, j - base, 0, 1, gexp);
+                lacc = acc ? glog[acc] : kNoLog;
+            }
+            sm.P[cur ^ 1][j] = static_cast<uint16_t>(acc);
+            sm.L[cur ^ 1][j] = static_cast<uint16_t>(lacc);
+        }
+        __syncthreads();
+    }
+    uint32_t sc = 1;
+    if (j < m) {
+        sc = vdm_quotient(sm.P[cur], xj, j, m, s, sm.QT, kVdmQtLd, sm.T + (j >> 5) * kNibbleWords, lane, glog, gexp);
+        sm.scale[j] = static_cast<uint16_t>(sc);
+    }
+    const int bad = __syncthreads_or(sc == 0);
+    if (j == 0)
+        *status = bad;
+    // inv[r'][r] = scale[r'] * QT[e_r - s][r']
+    for (int idx = j; idx < m * m; idx += blockDim.x) {
+        const int row = idx / m, r = idx - row * m;
+        inv[static_cast<size_t>(row) * ld + r] =
+            static_cast<uint16_t>(gmul(sm.scale[row], sm.QT[static_cast<int>(exps[r] - s) * kVdmQtLd + row], glog, gexp));
+    }
 }
 
 // inv[j][r] (row stride ld) = scale[j] * QT[e_r - s][j], through a 32 x 32 shared-memory tile
@@ -667,6 +820,15 @@ static int vdm_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x, const
 {
     const size_t vec = (static_cast<size_t>(m) * 2 + 255) & ~static_cast<size_t>(255);
     P2G_TRY(w.status.ensure(256 + 5 * vec));
+    if (m <= kVdmSmall) {
+        P2G_CUDA(cudaFuncSetAttribute(vdm_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(sizeof(VdmSmallSmem))));
+        vdm_small<<<1, kVdmSmall, sizeof(VdmSmallSmem), ctx->stream>>>(
+            d_x, d_exps, s, m, ld, d_inv, w.status.as<int>(), ctx->d_log, ctx->d_exp);
+        P2G_CUDA(cudaGetLastError());
+        ++ctx->launches;
+        return P2G_OK;
+    }
     P2G_TRY(w.M.ensure(static_cast<size_t>(m) * m * 2 + 16));
     uint8_t *aux = w.status.as<uint8_t>();
     int *status = reinterpret_cast<int *>(aux);
@@ -682,14 +844,18 @@ static int vdm_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x, const
     ++ctx->launches;
     int cur = 0;
     for (int G = 1; G < m; G *= 2) {
-        vdm_level<<<nb, tb, 0, ctx->stream>>>(P[cur], LP[cur], P[cur ^ 1], LP[cur ^ 1], m, G,
-                                              ctx->d_log, ctx->d_exp);
+        if (G < 16)
+            vdm_level<1><<<nb, tb, 0, ctx->stream>>>(P[cur], LP[cur], P[cur ^ 1], LP[cur ^ 1], m, G,
+                                                     ctx->d_log, ctx->d_exp);
+        else
+            vdm_level<32><<<(m + 7) / 8, 256, 0, ctx->stream>>>(P[cur], LP[cur], P[cur ^ 1], LP[cur ^ 1], m,
+                                                                G, ctx->d_log, ctx->d_exp);
         P2G_CUDA(cudaGetLastError());
         ++ctx->launches;
         cur ^= 1;
     }
     uint16_t *QT = w.M.as<uint16_t>();
-    vdm_quotients<<<(m + 31) / 32, 32, 0, ctx->stream>>>(P[cur], d_x, m, s, QT, scale, status,
+    vdm_quotients<<<(m + 31) / 32, kSegs * 32, 0, ctx->stream>>>(P[cur], d_x, m, s, QT, scale, status,
                                                          ctx->d_log, ctx->d_exp);
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
@@ -804,6 +970,40 @@ __global__ void wb_cols_kernel(const uint16_t *__restrict__ Vinv, int ldv, const
     }
 }
 
+// A fixed factor's products from one column of four 16-entry tables (64 words,
+// the entries of a table in 16 banks: lanes with one factor and any values never
+// conflict); entry e of the 64 is nibble_entry(y, e).
+__device__ __forceinline__ uint32_t nibble_entry(uint32_t y, int e)
+{
+    return gmul_alu(y, static_cast<uint32_t>(e & 15) << (4 * (e >> 4)));
+}
+__device__ __forceinline__ uint32_t column_product(const uint32_t *T, uint32_t q)
+{
+    return (T[q & 15] ^ T[16 + ((q >> 4) & 15)]) ^ (T[32 + ((q >> 8) & 15)] ^ T[48 + ((q >> 12) & 15)]);
+}
+
+// inv[j][r] = Vinv[j][r] + sum_q Vinv[j][rows[q]] Z[q][r] for a few replaced rows
+// (one CTA per row j; the multiply-accumulate kernels need g inputs to be many:
+// 60 us for 3 inputs and 1600 outputs; logarithm lookups in global memory 46)
+constexpr int kDirectRows = 8;
+__global__ void __launch_bounds__(256)
+    wb_correct_kernel(const uint16_t *__restrict__ Vinv, int ldv, const uint16_t *__restrict__ Z, int ldz,
+                      const int *__restrict__ rows, int m, int g, uint16_t *__restrict__ inv)
+{
+    __shared__ uint32_t T[kDirectRows][64];
+    const int j = blockIdx.x;
+    const uint16_t *v = Vinv + static_cast<size_t>(j) * ldv;
+    for (int e = threadIdx.x; e < 64 * g; e += blockDim.x)
+        T[e >> 6][e & 63] = nibble_entry(v[rows[e >> 6]], e & 63);
+    __syncthreads();
+    for (int r = threadIdx.x; r < m; r += blockDim.x) {
+        uint32_t acc = v[r];
+        for (int q = 0; q < g; ++q)
+            acc ^= column_product(T[q], Z[static_cast<size_t>(q) * ldz + r]);
+        inv[static_cast<size_t>(j) * m + r] = static_cast<uint16_t>(acc);
+    }
+}
+
 static int woodbury_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x,
                            const WoodburyPlan &wp, uint16_t *d_inv)
 {
@@ -871,6 +1071,13 @@ static int woodbury_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x,
     P2G_TRY(records_from_matrix(ctx, Cinv, g, g, recs));
     P2G_TRY(muladd_run(ctx, const_cast<const uint8_t *const *>(py), g, pz, g, bytes, recs, 0));
     // V^-1 += (V^-1 U) Z
+    if (g <= kDirectRows) {
+        wb_correct_kernel<<<m, 256, 0, ctx->stream>>>(Vinv, ld, reinterpret_cast<const uint16_t *>(b + o_z), ld,
+                                                      d_rows, m, g, d_inv);
+        P2G_CUDA(cudaGetLastError());
+        ctx->launches += 4;
+        return P2G_OK;
+    }
     const size_t nvc = static_cast<size_t>(m) * g;
     wb_cols_kernel<<<static_cast<unsigned>((nvc + 255) / 256), 256, 0, ctx->stream>>>(Vinv, ld, d_rows,
                                                                                    m, g, Vc);
