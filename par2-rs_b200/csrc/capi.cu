@@ -66,6 +66,7 @@ static size_t round16(size_t n) { return (n + 15) & ~static_cast<size_t>(15); }
 struct HostTables {
     uint16_t log[65536];
     uint16_t exp[65535];
+    uint16_t constant[32768];  // 2^n, n prime to 65535 = 3 * 5 * 17 * 257, in order
     HostTables()
     {
         uint32_t b = 1;
@@ -77,6 +78,10 @@ struct HostTables {
                 b ^= 0x1100Bu;
         }
         log[0] = 0;
+        size_t have = 0;
+        for (uint32_t n = 1; n < 65535; ++n)
+            if (n % 3 && n % 5 && n % 17 && n % 257)
+                constant[have++] = exp[n];
     }
 };
 
@@ -89,10 +94,8 @@ static const HostTables &tables()
 void par2_constants(size_t k, uint16_t *out)
 {
     const HostTables &t = tables();
-    size_t have = 0;
-    for (uint64_t n = 1; have < k; ++n)
-        if (n % 3 && n % 5 && n % 17 && n % 257)
-            out[have++] = t.exp[n % 65535];
+    for (size_t i = 0; i < k; ++i)
+        out[i] = t.constant[i % 32768];
 }
 
 // Layout of the per-call parameter block (device + pinned mirror).
