@@ -72,8 +72,8 @@ int p2g_set_stream(p2g_ctx *ctx, void *cuda_stream);
  * stream the kernels run on when timing is enabled.  No counterpart in
  * par2-rs (its tracing is host-side, par2_rs.rs:220-226). */
 typedef struct {
-    float ms_records;  /* coefficient records */
-    float ms_planes;   /* slices -> bit planes */
+    float ms_records;  /* parameters (and, in pipelined host calls, coefficients) */
+    float ms_planes;   /* operands: slices -> bit planes or forms, coefficients */
     float ms_kernel;   /* the main kernel: multiply-accumulate, or hashing */
     float ms_total;    /* first to last event of the call */
     int launches;      /* kernels launched by the call */

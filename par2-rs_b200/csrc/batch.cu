@@ -58,7 +58,7 @@ struct Phase {
     // the problems that the tensor cores take
     size_t tform_off = 0, tcoef_off = 0, tprob_off = 0, titem_off = 0;
     int ntens = 0, ntitems = 0, trows = 0;
-    unsigned long long tform_ctas = 0, tcoef_threads = 0;
+    unsigned long long tform_ctas = 0, tcoef_ctas = 0;
 };
 
 }  // namespace
@@ -168,7 +168,7 @@ int enqueue_phases(p2g_batch *b)
                                    P.ntens, P.tform_ctas));
         P2G_TRY(tensor_batch_coefs(st, ctx->d_log, ctx->d_exp,
                                    reinterpret_cast<const TensorCoefProb *>(dp(b, P.tcoef_off)),
-                                   P.ntens, P.tcoef_threads));
+                                   P.ntens, P.tcoef_ctas));
         P2G_TRY(batch_planes(st, reinterpret_cast<const PlanesProb *>(dp(b, P.planes_off)),
                              P.nplanes, P.planes_total));
         P2G_TRY(batch_records(st, ctx->d_log, ctx->d_exp,
@@ -824,7 +824,7 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
                 pl_off += planes_need(p);
                 rc_off += recs_need(p);
                 tf_first += tensor_form_ctas(p.nin, p.S);
-                tc_first += tensor_coef_threads(p.nin, p.nout);
+                tc_first += tensor_coef_ctas(p.nin, p.nout);
                 continue;
             }
             const int T = static_cast<int>((p.S + 2047) / 2048);
@@ -907,7 +907,7 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         D.ntitems = static_cast<int>(P.titems.size());
         D.trows = P.trows;
         D.tform_ctas = tf_first;
-        D.tcoef_threads = tc_first;
+        D.tcoef_ctas = tc_first;
         D.nplanes = static_cast<int>(P.pl.size());
         D.nrec = static_cast<int>(P.rc.size());
         D.nitems = static_cast<int>(P.items.size());

@@ -267,7 +267,7 @@ static int matrix_muladd(p2g_ctx *ctx, const std::vector<uint8_t *> &src,
     P2G_TRY(upload_params(ctx, L));
     uint8_t *d = ctx->params.as<uint8_t>();
     MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes);
-    P2G_TRY(mulop_matrix(ctx, op, ctx->recs, reinterpret_cast<const uint16_t *>(d + L.a_off)));
+    P2G_TRY(mulop_matrix(op, ctx->recs, reinterpret_cast<const uint16_t *>(d + L.a_off)));
     P2G_TRY(mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(d + L.src_off), 0,
                       static_cast<int>(nin), reinterpret_cast<uint8_t *const *>(d + L.dst_off), bytes, mode));
     return P2G_OK;
@@ -666,10 +666,12 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
     }
     P2G_TRY(upload_params(ctx, L));
     uint8_t *dp = ctx->params.as<uint8_t>();
-    P2G_TRY(mulop_par2(ctx, op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + L.a_off),
+    P2G_TRY(mulop_par2(op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + L.a_off),
                        reinterpret_cast<const uint32_t *>(dp + L.b_off)));
     const uint8_t *const *d_src = reinterpret_cast<const uint8_t *const *>(dp + L.src_off);
     uint8_t *const *d_dst = reinterpret_cast<uint8_t *const *>(dp + L.dst_off);
+    if (groups > 1)
+        P2G_TRY(mulop_prepare(ctx, op));
     if (groups == 1) {
         P2G_TRY(mulop_run(ctx, op, d_src, 0, static_cast<int>(k), d_dst, slice_bytes, 0));
     } else {
@@ -1085,7 +1087,9 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
     }
     // 2. RHS = R ^ V * present (by input groups as their uploads land)
     if (np) {
-        P2G_TRY(mulop_par2(ctx, tail.op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + L.b_off), d_exps));
+        P2G_TRY(mulop_par2(tail.op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + L.b_off), d_exps));
+        if (groups > 1)
+            P2G_TRY(mulop_prepare(ctx, tail.op));
         const uint8_t *const *d_src = reinterpret_cast<const uint8_t *const *>(dp + L.src_off);
         const int full = tail.slabs ? groups - tail.groups : groups;
         for (int g = 0; g < full; ++g) {
@@ -1098,7 +1102,9 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
     }
     // 3. missing = A^-1 * RHS
     MulOp op2 = mulop(ctx, static_cast<int>(m), static_cast<int>(m), slice_bytes);
-    P2G_TRY(mulop_matrix(ctx, op2, ctx->recs2, ctx->inv.as<uint16_t>()));
+    P2G_TRY(mulop_matrix(op2, ctx->recs2, ctx->inv.as<uint16_t>()));
+    if (tail.slabs)
+        P2G_TRY(mulop_prepare(ctx, op2));
     if (!tail.slabs) {
         P2G_TRY(mulop_run(ctx, op2, reinterpret_cast<const uint8_t *const *>(dp + L.dst_off), 0,
                           static_cast<int>(m),

@@ -419,7 +419,7 @@ int launch_group(p2g_ctx *ctx, Deferred *d, const std::vector<uint8_t *> &srcs,
     P2G_CUDA(cudaMemcpyAsync(dp, h, total, cudaMemcpyHostToDevice, ctx->stream));
     P2G_CUDA(cudaEventRecord(d->par_ev[slot], ctx->stream));
     MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes);
-    P2G_TRY(mulop_matrix(ctx, op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + co)));
+    P2G_TRY(mulop_matrix(op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + co)));
     return mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(dp + so), 0, static_cast<int>(nin),
                      reinterpret_cast<uint8_t *const *>(dp + dso), bytes, 1);
 }

@@ -142,10 +142,9 @@ __device__ __forceinline__ void store_group(uint8_t *base, size_t S, size_t off,
 }
 
 // LE symbols -> planes[i][t][b][lane]; one thread per group of 32 symbols.
-__global__ void slices_to_planes(const uint8_t *const *__restrict__ src, int nin, int T,
-                                 size_t S, uint32_t *__restrict__ planes)
+__device__ __forceinline__ void planes_of_group(const uint8_t *const *__restrict__ src, int nin, int T,
+                                                size_t S, uint32_t *__restrict__ planes, size_t gid)
 {
-    size_t gid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     size_t total = static_cast<size_t>(nin) * T * 32;
     if (gid >= total)
         return;
@@ -162,39 +161,51 @@ __global__ void slices_to_planes(const uint8_t *const *__restrict__ src, int nin
         P[b * 32] = x[b];
 }
 
-__global__ void records_matrix_kernel(const uint16_t *__restrict__ coeff, int nin, int nout,
-                                      uint32_t *__restrict__ recs)
+__global__ void slices_to_planes(const uint8_t *const *__restrict__ src, int nin, int T,
+                                 size_t S, uint32_t *__restrict__ planes)
 {
-    size_t gid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (gid >= static_cast<size_t>(nin) * nout)
-        return;
-    int o = static_cast<int>(gid % nout);
-    size_t i = gid / nout;
-    write_record(recs, gid, coeff[static_cast<size_t>(o) * nin + i], nout <= kSmallOutputs);
+    planes_of_group(src, nin, T, S, planes, static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x);
 }
 
-// c_i^e by the log / antilog tables: (log c * e) mod 65535 (galois/core.rs:242-258)
-__global__ void records_par2_kernel(const uint16_t *__restrict__ consts,
-                                    const uint32_t *__restrict__ exps,
-                                    const uint16_t *__restrict__ glog,
-                                    const uint16_t *__restrict__ gexp, int nin, int nout,
-                                    uint32_t *__restrict__ recs)
+// Record of coefficient gid = i * nout + o.
+__device__ __forceinline__ void record_of(const CoefSource &c, const uint16_t *__restrict__ glog,
+                                          const uint16_t *__restrict__ gexp, int nin, int nout,
+                                          uint32_t *__restrict__ recs, size_t gid)
 {
-    size_t gid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (gid >= static_cast<size_t>(nin) * nout)
         return;
-    int o = static_cast<int>(gid % nout);
-    int i = static_cast<int>(gid / nout);
-    uint32_t base = consts[i];
-    uint32_t e = exps[o];
-    uint32_t c;
-    if (base == 0)
-        c = e == 0 ? 1u : 0u;
-    else if (e == 0)
-        c = 1u;
+    const int o = static_cast<int>(gid % nout), i = static_cast<int>(gid / nout);
+    write_record(recs, gid, coefficient(c, nin, i, o, glog, gexp), nout <= kSmallOutputs);
+}
+
+__global__ void records_kernel(const CoefSource c, const uint16_t *__restrict__ glog,
+                               const uint16_t *__restrict__ gexp, int nin, int nout,
+                               uint32_t *__restrict__ recs)
+{
+    record_of(c, glog, gexp, nin, nout, recs, static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x);
+}
+
+// All that a launch of the table kernels needs, in one launch: blocks of 256
+// threads for the records, then the planes, then the outputs that partial
+// results are XORed into.  (Three launches in a row are 4-6 us each on a small
+// problem, mostly their latency: 20 slices of 4 KiB, 2 outputs, 4.6 + 3.5 + 2.5
+// us against 5.1 in one, the call 36 -> 29.)
+__global__ void __launch_bounds__(256)
+    prepare_tables(const CoefSource c, const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp,
+                   int cnin, int nout, uint32_t *__restrict__ recs, unsigned rec_blocks,
+                   const uint8_t *const *__restrict__ src, int nin, int T, size_t S,
+                   uint32_t *__restrict__ planes, unsigned plane_blocks, const ZeroOutputs z)
+{
+    unsigned b = blockIdx.x;
+    if (b < rec_blocks) {
+        record_of(c, glog, gexp, cnin, nout, recs, static_cast<size_t>(b) * 256 + threadIdx.x);
+        return;
+    }
+    b -= rec_blocks;
+    if (b < plane_blocks)
+        planes_of_group(src, nin, T, S, planes, static_cast<size_t>(b) * 256 + threadIdx.x);
     else
-        c = gexp[static_cast<uint32_t>((static_cast<uint64_t>(glog[base]) * e) % 65535u)];
-    write_record(recs, gid, c, nout <= kSmallOutputs);
+        zero_block(z, b - plane_blocks);
 }
 
 // WARPS warps per CTA; each output group of EREG outputs is held by PSPLIT
@@ -796,22 +807,8 @@ __global__ void __launch_bounds__(kBatchWarps * 32, 1)
     }
 }
 
-// Zeroes nout slices before a split (atomic-XOR) run in store mode.
-__global__ void zero_slices(uint8_t *const *__restrict__ dst, int nout, size_t S)
-{
-    int o = blockIdx.y;
-    if (o >= nout)
-        return;
-    uint8_t *d = dst[o];
-    for (size_t x = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 16; x < S;
-         x += static_cast<size_t>(gridDim.x) * blockDim.x * 16) {
-        if (x + 16 <= S)
-            *reinterpret_cast<uint4 *>(d + x) = make_uint4(0, 0, 0, 0);
-        else
-            for (size_t y = x; y < S; y += 2)
-                *reinterpret_cast<uint16_t *>(d + y) = 0;
-    }
-}
+// Zeroes outputs before a split (atomic-XOR) run in store mode.
+__global__ void __launch_bounds__(256) zero_slices(const ZeroOutputs z) { zero_block(z, blockIdx.x); }
 
 using KernelFn = void (*)(const uint32_t *, const uint32_t *, int, int, int, int, int,
                           uint8_t *const *, size_t, int);
@@ -997,29 +994,31 @@ bool plan_valid(const MuladdPlan &p, int nin, int nout, size_t S)
            (p.nsplit == 1 || (S % 4 == 0 && p.nsplit <= std::max(1, nin)));
 }
 
-int records_from_matrix(p2g_ctx *ctx, const uint16_t *d_coeff, int nin, int nout,
-                        uint32_t *d_recs)
+static int launch_records(cudaStream_t st, const CoefSource &c, const uint16_t *glog,
+                          const uint16_t *gexp, int nin, int nout, uint32_t *d_recs)
 {
-    size_t n = static_cast<size_t>(nin) * nout;
+    const size_t n = static_cast<size_t>(nin) * nout;
     if (n == 0)
         return P2G_OK;
-    records_matrix_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, ctx->stream>>>(
-        d_coeff, nin, nout, d_recs);
+    records_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(c, glog, gexp, nin, nout, d_recs);
     P2G_CUDA(cudaGetLastError());
-    ++ctx->launches;
     return P2G_OK;
 }
 
-int records_par2(p2g_ctx *ctx, const uint16_t *d_consts, const uint32_t *d_exps, int nin,
-                 int nout, uint32_t *d_recs)
+int records_from_matrix(p2g_ctx *ctx, const uint16_t *d_coeff, int nin, int nout,
+                        uint32_t *d_recs)
 {
-    size_t n = static_cast<size_t>(nin) * nout;
-    if (n == 0)
-        return P2G_OK;
-    records_par2_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, ctx->stream>>>(
-        d_consts, d_exps, ctx->d_log, ctx->d_exp, nin, nout, d_recs);
+    CoefSource c;
+    c.coeff = d_coeff;
+    ctx->launches += nin > 0 && nout > 0;
+    return launch_records(ctx->stream, c, ctx->d_log, ctx->d_exp, nin, nout, d_recs);
+}
+
+static int launch_zero(cudaStream_t st, uint8_t *const *d_dst, int nout, size_t S)
+{
+    const ZeroOutputs z = zero_blocks(d_dst, nout, S);
+    zero_slices<<<z.blocks, 256, 0, st>>>(z);
     P2G_CUDA(cudaGetLastError());
-    ++ctx->launches;
     return P2G_OK;
 }
 
@@ -1043,8 +1042,11 @@ static int launch_kernel(cudaStream_t stream, const MuladdPlan &p, const uint32_
     return P2G_OK;
 }
 
-int muladd_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *const *d_dst,
-               int nout, size_t S, const uint32_t *d_recs, int mode, const MuladdPlan *plan)
+// muladd_run, after which the records of `todo` (op's, when not null) are
+// written as well.
+static int tables_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *const *d_dst,
+                      int nout, size_t S, const uint32_t *d_recs, int mode, const MuladdPlan *plan,
+                      MulOp *todo)
 {
     if (nout <= 0)
         return P2G_OK;
@@ -1057,9 +1059,7 @@ int muladd_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *cons
     }
     if (nin == 0) {
         if (mode == 0) {
-            dim3 g(static_cast<unsigned>(std::min<size_t>((S + 4095) / 4096, 1024)), nout);
-            zero_slices<<<g, 256, 0, ctx->stream>>>(d_dst, nout, S);
-            P2G_CUDA(cudaGetLastError());
+            P2G_TRY(launch_zero(ctx->stream, d_dst, nout, S));
             ++ctx->launches;
         }
         return P2G_OK;
@@ -1067,23 +1067,29 @@ int muladd_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *cons
     size_t plane_bytes = static_cast<size_t>(nin) * T * kTileBytes;
     P2G_TRY(ctx->planes.ensure(plane_bytes));
     uint32_t *planes = ctx->planes.as<uint32_t>();
-    size_t groups = static_cast<size_t>(nin) * T * 32;
+    const size_t groups = static_cast<size_t>(nin) * T * 32;
+    const size_t recs = todo ? static_cast<size_t>(todo->nin) * nout : 0;
+    const ZeroOutputs z = p.nsplit > 1 && mode == 0 ? zero_blocks(d_dst, nout, S) : ZeroOutputs{};
+    const unsigned rec_blocks = static_cast<unsigned>((recs + 255) / 256),
+                   plane_blocks = static_cast<unsigned>((groups + 255) / 256);
     ctx->mark(1);
-    slices_to_planes<<<static_cast<unsigned>((groups + 255) / 256), 256, 0, ctx->stream>>>(
-        d_src, nin, T, S, planes);
+    prepare_tables<<<rec_blocks + plane_blocks + z.blocks, 256, 0, ctx->stream>>>(
+        todo ? todo->todo : CoefSource{}, ctx->d_log, ctx->d_exp, todo ? todo->nin : 0, nout,
+        todo ? const_cast<uint32_t *>(todo->coef) : nullptr, rec_blocks, d_src, nin, T, S, planes, plane_blocks,
+        z);
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
-    if (p.nsplit > 1 && mode == 0) {
-        dim3 g(static_cast<unsigned>(std::min<size_t>((S + 4095) / 4096, 1024)), nout);
-        zero_slices<<<g, 256, 0, ctx->stream>>>(d_dst, nout, S);
-        P2G_CUDA(cudaGetLastError());
-        ++ctx->launches;
-    }
     ctx->mark(2);
     P2G_TRY(launch_kernel(ctx->stream, p, planes, d_recs, nin, nout, T, d_dst, S, mode));
     ++ctx->launches;
     ctx->mark(3);
     return P2G_OK;
+}
+
+int muladd_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *const *d_dst,
+               int nout, size_t S, const uint32_t *d_recs, int mode, const MuladdPlan *plan)
+{
+    return tables_run(ctx, d_src, nin, d_dst, nout, S, d_recs, mode, plan, nullptr);
 }
 
 static MuladdPlan tensor_plan(int sms, int nin, int nout, size_t S)
@@ -1147,26 +1153,40 @@ MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S)
     return op;
 }
 
-int mulop_matrix(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_coeff)
+static int mulop_coefs(MulOp &op, DevBuf &buf, const CoefSource &c)
 {
     P2G_TRY(buf.ensure(op.plan.tensor ? tensor_coef_bytes(op.nin, op.nout) : record_bytes(op.nin, op.nout)));
     op.coef = buf.as<uint32_t>();
-    if (!op.plan.tensor)
-        return records_from_matrix(ctx, d_coeff, op.nin, op.nout, buf.as<uint32_t>());
-    P2G_TRY(tensor_coef_matrix(ctx->stream, d_coeff, op.nin, op.nout, buf.p));
-    ++ctx->launches;
+    op.todo = c;
+    op.pending = op.nin > 0 && op.nout > 0;
     return P2G_OK;
 }
 
-int mulop_par2(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_consts, const uint32_t *d_exps)
+int mulop_matrix(MulOp &op, DevBuf &buf, const uint16_t *d_coeff)
 {
-    P2G_TRY(buf.ensure(op.plan.tensor ? tensor_coef_bytes(op.nin, op.nout) : record_bytes(op.nin, op.nout)));
-    op.coef = buf.as<uint32_t>();
-    if (!op.plan.tensor)
-        return records_par2(ctx, d_consts, d_exps, op.nin, op.nout, buf.as<uint32_t>());
-    P2G_TRY(tensor_coef_par2(ctx->stream, d_consts, d_exps, ctx->d_log, ctx->d_exp, op.nin, op.nout, buf.p));
+    CoefSource c;
+    c.coeff = d_coeff;
+    return mulop_coefs(op, buf, c);
+}
+
+int mulop_par2(MulOp &op, DevBuf &buf, const uint16_t *d_consts, const uint32_t *d_exps)
+{
+    CoefSource c;
+    c.consts = d_consts;
+    c.exps = d_exps;
+    return mulop_coefs(op, buf, c);
+}
+
+int mulop_prepare(p2g_ctx *ctx, MulOp &op)
+{
+    if (!op.pending)
+        return P2G_OK;
+    op.pending = false;
     ++ctx->launches;
-    return P2G_OK;
+    uint32_t *buf = const_cast<uint32_t *>(op.coef);
+    return op.plan.tensor
+               ? tensor_coefs(ctx->stream, op.todo, ctx->d_log, ctx->d_exp, op.nin, op.nout, buf)
+               : launch_records(ctx->stream, op.todo, ctx->d_log, ctx->d_exp, op.nin, op.nout, buf);
 }
 
 int mulop_part(const MulOp &op, int g, int parts)
@@ -1180,16 +1200,7 @@ int mulop_part(const MulOp &op, int g, int parts)
 // run in column chunks: the operand is 1.9 times the slices).
 constexpr size_t kMaxFormBytes = 12ull << 30;
 
-static int zero_outputs(p2g_ctx *ctx, uint8_t *const *d_dst, int nout, size_t S)
-{
-    dim3 g(static_cast<unsigned>(std::min<size_t>((S + 4095) / 4096, 1024)), nout);
-    zero_slices<<<g, 256, 0, ctx->stream>>>(d_dst, nout, S);
-    P2G_CUDA(cudaGetLastError());
-    ++ctx->launches;
-    return P2G_OK;
-}
-
-int mulop_run(p2g_ctx *ctx, const MulOp &op, const uint8_t *const *d_src, int i0, int n,
+int mulop_run(p2g_ctx *ctx, MulOp &op, const uint8_t *const *d_src, int i0, int n,
               uint8_t *const *d_dst, size_t S, int mode)
 {
     if (op.nout <= 0)
@@ -1197,12 +1208,20 @@ int mulop_run(p2g_ctx *ctx, const MulOp &op, const uint8_t *const *d_src, int i0
     if (!op.plan.tensor) {
         // part of the inputs, or of the columns, has a plan of its own
         const bool whole = i0 == 0 && n == op.nin && S == op.S;
-        return muladd_run(ctx, d_src, n, d_dst, op.nout, S,
-                          op.coef + static_cast<size_t>(i0) * op.nout * record_words(op.nout), mode,
-                          whole ? &op.plan : nullptr);
+        const bool pending = op.pending && n > 0;
+        P2G_TRY(tables_run(ctx, d_src, n, d_dst, op.nout, S,
+                           op.coef + static_cast<size_t>(i0) * op.nout * record_words(op.nout), mode,
+                           whole ? &op.plan : nullptr, pending ? &op : nullptr));
+        op.pending = op.pending && !pending;
+        return P2G_OK;
     }
-    if (n == 0)
-        return mode == 0 ? zero_outputs(ctx, d_dst, op.nout, S) : P2G_OK;
+    if (n == 0) {
+        if (mode == 0) {
+            P2G_TRY(launch_zero(ctx->stream, d_dst, op.nout, S));
+            ++ctx->launches;
+        }
+        return P2G_OK;
+    }
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
     TensorRun r;
     r.src = d_src;
@@ -1234,12 +1253,12 @@ int mulop_run(p2g_ctx *ctx, const MulOp &op, const uint8_t *const *d_src, int i0
     ctx->mark(1);
     for (size_t t0 = 0; t0 < tiles; t0 += chunk) {
         const size_t nt = std::min(chunk, tiles - t0);
-        P2G_TRY(tensor_forms(ctx->stream, r, t0, nt));
-        if (t0 == 0) {
-            if (r.split > 1 && mode == 0)
-                P2G_TRY(zero_outputs(ctx, d_dst, op.nout, S));
+        const ZeroOutputs z =
+            t0 == 0 && r.split > 1 && mode == 0 ? zero_blocks(d_dst, op.nout, S) : ZeroOutputs{};
+        P2G_TRY(tensor_prepare(ctx->stream, r, t0, nt, op.pending ? &op.todo : nullptr, ctx->d_log, ctx->d_exp, z));
+        op.pending = false;
+        if (t0 == 0)
             ctx->mark(2);
-        }
         P2G_TRY(tensor_products(ctx->stream, r, t0, nt));
         ctx->launches += 2;
     }
@@ -1448,7 +1467,9 @@ int muladd_autotune(p2g_ctx *ctx, int nin, int nout, size_t S, int reps, MuladdP
         op.S = S;
         op.plan = tensor_plan(sms, nin, nout, S);
         if (rc == P2G_OK)
-            rc = mulop_matrix(ctx, op, ctx->recs, ctx->coeffs.as<uint16_t>());
+            rc = mulop_matrix(op, ctx->recs, ctx->coeffs.as<uint16_t>());
+        if (rc == P2G_OK)
+            rc = mulop_prepare(ctx, op);
         const int own = op.plan.nsplit;
         float tensor_ms = 1e30f;
         int tensor_split = own;
@@ -1528,19 +1549,7 @@ __global__ void batch_records_kernel(const RecProb *__restrict__ probs, int np,
     const unsigned long long local = gid - p.first;
     const int o = static_cast<int>(local % p.nout);
     const int i = static_cast<int>(local / p.nout);
-    uint32_t c;
-    if (p.coeff) {
-        c = p.coeff[static_cast<size_t>(o) * p.nin + i];
-    } else {
-        const uint32_t base = p.consts[i], e = p.exps[o];
-        if (base == 0)
-            c = e == 0 ? 1u : 0u;
-        else if (e == 0)
-            c = 1u;
-        else
-            c = gexp[static_cast<uint32_t>((static_cast<uint64_t>(glog[base]) * e) % 65535u)];
-    }
-    write_record(p.recs, local, c, p.small != 0);
+    write_record(p.recs, local, coefficient({p.coeff, p.consts, p.exps}, p.nin, i, o, glog, gexp), p.small != 0);
 }
 
 __global__ void batch_zero_kernel(uint8_t *const *__restrict__ ptrs,
@@ -1657,13 +1666,9 @@ size_t planes_bytes_fixed(int nin, size_t S)
 int records_matrix_fixed(cudaStream_t stream, const uint16_t *d_coeff, int nin, int nout,
                          uint32_t *d_recs)
 {
-    size_t n = static_cast<size_t>(nin) * nout;
-    if (n == 0)
-        return P2G_OK;
-    records_matrix_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
-        d_coeff, nin, nout, d_recs);
-    P2G_CUDA(cudaGetLastError());
-    return P2G_OK;
+    CoefSource c;
+    c.coeff = d_coeff;
+    return launch_records(stream, c, nullptr, nullptr, nin, nout, d_recs);
 }
 
 int muladd_run_fixed(cudaStream_t stream, int sm_count, const uint8_t *const *d_src, int nin,
@@ -1676,13 +1681,10 @@ int muladd_run_fixed(cudaStream_t stream, int sm_count, const uint8_t *const *d_
     probe.sm_count = sm_count;
     const MuladdPlan p = choose_plan(&probe, nin, nout, S);
     const int T = static_cast<int>((S + kTileBytes - 1) / kTileBytes);
-    dim3 zg(static_cast<unsigned>(std::min<size_t>((S + 4095) / 4096, 1024)), nout);
-    if (nin == 0 || p.nsplit > 1) {
-        zero_slices<<<zg, 256, 0, stream>>>(d_dst, nout, S);
-        P2G_CUDA(cudaGetLastError());
-        if (nin == 0)
-            return P2G_OK;
-    }
+    if (nin == 0 || p.nsplit > 1)
+        P2G_TRY(launch_zero(stream, d_dst, nout, S));
+    if (nin == 0)
+        return P2G_OK;
     size_t groups = static_cast<size_t>(nin) * T * 32;
     slices_to_planes<<<static_cast<unsigned>((groups + 255) / 256), 256, 0, stream>>>(
         d_src, nin, T, S, d_planes);

@@ -2,6 +2,7 @@
 #pragma once
 #include "bitslice.cuh"
 #include "common.cuh"
+#include "prep.cuh"
 #include "tensor.cuh"
 
 namespace p2g {
@@ -134,11 +135,6 @@ int muladd_autotune(p2g_ctx *ctx, int nin, int nout, size_t S, int reps, MuladdP
 int records_from_matrix(p2g_ctx *ctx, const uint16_t *d_coeff, int nin, int nout,
                         uint32_t *d_recs);
 
-// Records of the PAR2 encoding matrix: coefficient (i, o) = consts[i]^exps[o]
-// (par2_rs.rs:707-719).
-int records_par2(p2g_ctx *ctx, const uint16_t *d_consts, const uint32_t *d_exps, int nin,
-                 int nout, uint32_t *d_recs);
-
 // dst[o] (^)= sum_i coeff(i, o) * src[i] over slices of slice_bytes.
 // d_src / d_dst are DEVICE arrays of 16-byte aligned device pointers.
 // mode 0 stores, mode 1 XORs into the existing contents.
@@ -155,19 +151,25 @@ struct MulOp {
     size_t S = 0;  // slice bytes the plan is for
     MuladdPlan plan;
     const uint32_t *coef = nullptr;
+    CoefSource todo;       // what the coefficients are written from
+    bool pending = false;  // not written yet
 };
 // Chooses the plan of an nin x nout problem over slices of S bytes (the
 // context's own plan for that shape if it has one, else by the sizes).
 MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S);
-// Writes the coefficients into buf (grown as needed): from a device matrix
-// [nout][nin], or consts[i]^exps[o].
-int mulop_matrix(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_coeff);
-int mulop_par2(p2g_ctx *ctx, MulOp &op, DevBuf &buf, const uint16_t *d_consts, const uint32_t *d_exps);
+// The coefficients, which go into buf (grown as needed): a device matrix
+// [nout][nin], or consts[i]^exps[o] (the PAR2 encoding matrix,
+// par2_rs.rs:707-719).  The first mulop_run writes them, in the launch that
+// prepares its inputs; mulop_prepare writes them now, for a call whose inputs
+// are still on their way.
+int mulop_matrix(MulOp &op, DevBuf &buf, const uint16_t *d_coeff);
+int mulop_par2(MulOp &op, DevBuf &buf, const uint16_t *d_consts, const uint32_t *d_exps);
+int mulop_prepare(p2g_ctx *ctx, MulOp &op);
 // The input at which part g of `parts` parts of the inputs starts.
 int mulop_part(const MulOp &op, int g, int parts);
 // dst (^)= inputs [i0, i0 + n) of the product over slices of S bytes; d_src
 // holds those n inputs' pointers, i0 is a mulop_part of the op.
-int mulop_run(p2g_ctx *ctx, const MulOp &op, const uint8_t *const *d_src, int i0, int n,
+int mulop_run(p2g_ctx *ctx, MulOp &op, const uint8_t *const *d_src, int i0, int n,
               uint8_t *const *d_dst, size_t S, int mode);
 
 // The same work as records_from_matrix / muladd_run (store mode) on a given

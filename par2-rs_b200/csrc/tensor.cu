@@ -18,9 +18,9 @@
 // multiply-adds, of which an SM does 16384 per clock; the table kernels spend
 // 4 bytes of shared-memory reads on it, of which an SM does 128 per clock.
 //
-//   * symbol_forms reads the slices once and writes the 30 forms that all 60
+//   * forms_of_pair reads the slices once and writes the 30 forms that all 60
 //     phi_e are sums of (1, 2 or 4 of them) as bits, 32 inputs to a word.
-//   * coef_forms writes the coefficients' 60 forms as the 4-bit B operand.
+//   * coef_block writes the coefficients' 60 forms as the 4-bit B operand.
 //   * tensor_muladd: a CTA owns 256 symbols (two accumulator tiles of 128
 //     rows) and up to 208 outputs (columns).  For each e it runs over all
 //     inputs in stages of 256: four warps per tile turn the form words of 128
@@ -45,7 +45,7 @@
 // product takes less than 48 clocks; the small tables 4.2 ms).  What remains
 // is latency: with one stage of A per tile at 208 columns its refill is only
 // partly hidden by the other tile's products, and a tile stands still while its
-// accumulators are read.  symbol_forms: 1.0 ms for 2 GiB, 6.4 of 6.55 TB/s.
+// accumulators are read.  The symbol forms: 1.0 ms for 2 GiB, 6.4 of 6.55 TB/s.
 //
 // The place of an input in an operand word: bit j of a form word (input j of
 // 32) becomes nibble j / 4 of word j % 4 of the 16-byte group.  The A side
@@ -355,14 +355,7 @@ __device__ __forceinline__ void forms_of_pair(const uint8_t *const *__restrict__
     store_forms<0>(x, x + 16, out, plane);
 }
 
-__global__ void __launch_bounds__(256)
-    symbol_forms(const uint8_t *const *__restrict__ src, int nin, size_t S, size_t byte0,
-                 uint32_t *__restrict__ forms)
-{
-    forms_of_pair(src, nin, S, byte0, forms, blockIdx.x, blockIdx.y);
-}
-
-// the problem that CTA or thread `id` of a batched launch works for
+// the problem that CTA `id` of a batched launch works for
 template <class P>
 __device__ __forceinline__ int problem_of(const P *probs, int np, unsigned long long id)
 {
@@ -423,71 +416,98 @@ __device__ __forceinline__ void store_coef(const uint32_t *x, uint4 *out, size_t
     }
 }
 
-// coef[block][e][word][row] (16 bytes: 32 inputs of one output).  One thread
-// takes one output's 32 coefficients of a word and the products of one of the
-// ten places (blockIdx.y); coefficients come from a matrix or are powers
-// c_i^e (par2_rs.rs:707-719).
-__device__ __forceinline__ void coef_of_word(const TensorCoefProb &p, const uint16_t *__restrict__ glog,
-                                             const uint16_t *__restrict__ gexp, int rows, int nblk,
-                                             unsigned long long id, int place)
+// coef[block][e][word][row] (16 bytes: 32 inputs of one output).  A block of
+// 256 threads takes 32 rows (of all output blocks' rows, padding included) of 4
+// words: its threads find 16 coefficients each, 128 of them transpose 32
+// coefficients' bits, and then a warp takes a word's products of one of the ten
+// places at a time.  (With one thread for all of an output's coefficients and
+// one place, the ten of a word found them all ten times: 32000 inputs and 1600
+// outputs took 1.36 ms; now they and the forms of 64 KiB slices, 0.96 ms alone,
+// take 1.31 in one launch.)
+constexpr int kCoefWords = 4;
+__device__ __forceinline__ void coef_block(const TensorCoefProb &p, const uint16_t *__restrict__ glog,
+                                           const uint16_t *__restrict__ gexp, unsigned block)
 {
-    const int all = rows * nblk, words = (p.nin + 63) / 64 * 2;
-    const int kw = static_cast<int>(id / all), ro = static_cast<int>(id % all);
+    __shared__ uint32_t bits[kCoefWords][16][32];
+    const int nblk = (p.nout + kTensorMaxN - 1) / kTensorMaxN, per = (p.nout + nblk - 1) / nblk;
+    const int rows = (per + 15) / 16 * 16, all = rows * nblk, words = (p.nin + 63) / 64 * 2;
+    const unsigned groups = (all + 31) / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ro = static_cast<int>(block % groups) * 32 + lane, kw0 = static_cast<int>(block / groups) * kCoefWords;
     const int nb = ro / rows, row = ro % rows;
     // blocks of equal size: block nb holds outputs [nb * per, ...)
-    const int per = (p.nout + nblk - 1) / nblk;
     const int o = nb * per + row;
-    const bool live = row < per && o < p.nout;
-    uint32_t x[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        x[j] = 0;
-    if (live) {
-        const uint32_t e = p.coeff ? 0u : p.exps[o];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const int in = kw * 32 + i;
-            uint32_t c = 0;
-            if (in < p.nin) {
-                if (p.coeff) {
-                    c = p.coeff[static_cast<size_t>(o) * p.nin + in];
-                } else {
-                    const uint32_t base = p.consts[in];
-                    if (e == 0)
-                        c = 1;
-                    else if (base != 0)
-                        c = gexp[static_cast<uint32_t>((static_cast<uint64_t>(glog[base]) * e) % 65535u)];
-                }
-            }
-            x[i & 15] |= c << (i & 16);
+    const bool live = ro < all && row < per && o < p.nout;
+    const CoefSource c = {p.coeff, p.consts, p.exps};
+    {
+        const int w = warp & 3, j0 = (warp >> 2) * 8, in0 = (kw0 + w) * 32;
+#pragma unroll 4
+        for (int j = j0; j < j0 + 8; ++j) {
+            uint32_t x = 0;
+            if (live && in0 + j < p.nin)
+                x = coefficient(c, p.nin, in0 + j, o, glog, gexp);
+            if (live && in0 + j + 16 < p.nin)
+                x |= coefficient(c, p.nin, in0 + j + 16, o, glog, gexp) << 16;
+            bits[w][j][lane] = x;
         }
     }
-    transpose16x2(x);
+    __syncthreads();
+    if (warp < kCoefWords) {
+        uint32_t x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            x[j] = bits[warp][j][lane];
+        transpose16x2(x);
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            bits[warp][j][lane] = x[j];
+    }
+    __syncthreads();
     const size_t stride = static_cast<size_t>(words) * rows;
-    uint4 *out = p.coef + (static_cast<size_t>(nb) * kProds * words + kw) * rows + row;
-    store_coef<0>(x, out, stride, place);
+    for (int job = warp; job < 10 * kCoefWords; job += 8) {
+        const int w = job / 10, kw = kw0 + w;
+        if (ro >= all || kw >= words)
+            continue;
+        uint32_t x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            x[j] = bits[w][j][lane];
+        store_coef<0>(x, p.coef + (static_cast<size_t>(nb) * kProds * words + kw) * rows + row, stride, job % 10);
+    }
 }
 
-__global__ void __launch_bounds__(128)
-    coef_forms(const TensorCoefProb p, const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp,
-               int rows, int nblk, unsigned long long total)
+__global__ void __launch_bounds__(256)
+    coef_forms(const TensorCoefProb p, const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp)
 {
-    const unsigned long long id = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (id < total)
-        coef_of_word(p, glog, gexp, rows, nblk, id, blockIdx.y);
+    coef_block(p, glog, gexp, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
     batch_coef_forms(const TensorCoefProb *__restrict__ probs, int np, const uint16_t *__restrict__ glog,
-                     const uint16_t *__restrict__ gexp, unsigned long long total)
+                     const uint16_t *__restrict__ gexp)
 {
-    const unsigned long long id = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (id >= total)
+    const TensorCoefProb p = probs[problem_of(probs, np, blockIdx.x)];
+    coef_block(p, glog, gexp, static_cast<unsigned>(blockIdx.x - p.first));
+}
+
+// Both operands, and the outputs that partial results are XORed into, in one
+// launch: blocks for the coefficients, then the symbols (pairs x 64 inputs), then
+// the outputs.
+__global__ void __launch_bounds__(256)
+    prepare_tensor(const TensorCoefProb p, const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp,
+                   unsigned coef_blocks, const uint8_t *const *__restrict__ src, int nin, size_t S, size_t byte0,
+                   uint32_t *__restrict__ forms, unsigned pairs, unsigned form_blocks, const ZeroOutputs z)
+{
+    unsigned b = blockIdx.x;
+    if (b < coef_blocks) {
+        coef_block(p, glog, gexp, b);
         return;
-    const TensorCoefProb p = probs[problem_of(probs, np, id)];
-    const int nblk = (p.nout + kTensorMaxN - 1) / kTensorMaxN;
-    const int rows = ((p.nout + nblk - 1) / nblk + 15) / 16 * 16;
-    coef_of_word(p, glog, gexp, rows, nblk, id - p.first, blockIdx.y);
+    }
+    b -= coef_blocks;
+    if (b < form_blocks)
+        forms_of_pair(src, nin, S, byte0, forms, b % pairs, b / pairs);
+    else
+        zero_block(z, b - form_blocks);
 }
 
 // ---- the products ----------------------------------------------------------
@@ -1055,17 +1075,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 size_t tensor_smem(int rows) { return kOffB + static_cast<size_t>(kRingB) * rows * kStageWords * 16; }
 
-int launch_coef(cudaStream_t st, const TensorCoefProb &p, const uint16_t *glog, const uint16_t *gexp)
-{
-    const unsigned long long n = tensor_coef_threads(p.nin, p.nout);
-    if (n == 0)
-        return P2G_OK;
-    coef_forms<<<dim3(static_cast<unsigned>((n + 127) / 128), 10), 128, 0, st>>>(
-        p, glog, gexp, tensor_rows(p.nout), tensor_blocks(p.nout), n);
-    P2G_CUDA(cudaGetLastError());
-    return P2G_OK;
-}
-
 // clocks of one product of a CTA's two tiles (see tensor_clocks)
 double product_clocks(int nin, int nout)
 {
@@ -1085,21 +1094,15 @@ size_t tensor_form_bytes(int nin, size_t tiles)
     return (tiles + 1) / 2 * static_cast<size_t>(tensor_stages(nin)) * kForms * kFormBytes;
 }
 
-int tensor_coef_matrix(cudaStream_t st, const uint16_t *d_coeff, int nin, int nout, void *coef)
+int tensor_coefs(cudaStream_t st, const CoefSource &c, const uint16_t *glog, const uint16_t *gexp,
+                 int nin, int nout, void *coef)
 {
     if (nin <= 0 || nout <= 0)
         return P2G_OK;
-    return launch_coef(st, TensorCoefProb{d_coeff, nullptr, nullptr, static_cast<uint4 *>(coef), nin, nout, 0},
-                       nullptr, nullptr);
-}
-
-int tensor_coef_par2(cudaStream_t st, const uint16_t *d_consts, const uint32_t *d_exps,
-                     const uint16_t *glog, const uint16_t *gexp, int nin, int nout, void *coef)
-{
-    if (nin <= 0 || nout <= 0)
-        return P2G_OK;
-    return launch_coef(st, TensorCoefProb{nullptr, d_consts, d_exps, static_cast<uint4 *>(coef), nin, nout, 0},
-                       glog, gexp);
+    const TensorCoefProb p{c.coeff, c.consts, c.exps, static_cast<uint4 *>(coef), nin, nout, 0};
+    coef_forms<<<static_cast<unsigned>(tensor_coef_ctas(nin, nout)), 256, 0, st>>>(p, glog, gexp);
+    P2G_CUDA(cudaGetLastError());
+    return P2G_OK;
 }
 
 // SM clocks of a problem's two launches, and the parts of the 60 products (CTAs
@@ -1148,12 +1151,11 @@ int tensor_batch_forms(cudaStream_t st, const TensorFormProb *d, int np, unsigne
 }
 
 int tensor_batch_coefs(cudaStream_t st, const uint16_t *glog, const uint16_t *gexp,
-                       const TensorCoefProb *d, int np, unsigned long long threads)
+                       const TensorCoefProb *d, int np, unsigned long long ctas)
 {
-    if (!threads)
+    if (!ctas)
         return P2G_OK;
-    batch_coef_forms<<<dim3(static_cast<unsigned>((threads + 127) / 128), 10), 128, 0, st>>>(d, np, glog, gexp,
-                                                                                             threads);
+    batch_coef_forms<<<static_cast<unsigned>(ctas), 256, 0, st>>>(d, np, glog, gexp);
     P2G_CUDA(cudaGetLastError());
     return P2G_OK;
 }
@@ -1171,12 +1173,26 @@ int tensor_batch(cudaStream_t st, const TensorArgs *probs, const TensorItem *ite
     return P2G_OK;
 }
 
-int tensor_forms(cudaStream_t st, const TensorRun &r, size_t t0, size_t n)
+int tensor_prepare(cudaStream_t st, const TensorRun &r, size_t t0, size_t n, const CoefSource *todo,
+                   const uint16_t *glog, const uint16_t *gexp, const ZeroOutputs &z)
 {
     const size_t byte0 = t0 * kTensorM * 2;
-    symbol_forms<<<dim3(static_cast<unsigned>((n + 1) / 2), static_cast<unsigned>((r.nin + 63) / 64)), 256, 0, st>>>(
-        r.src, r.nin, std::min(r.S, byte0 + n * kTensorM * 2), byte0,
-        static_cast<uint32_t *>(r.forms));
+    TensorCoefProb p{};
+    unsigned long long coef_blocks = 0;
+    if (todo) {
+        p = TensorCoefProb{todo->coeff, todo->consts, todo->exps,
+                           static_cast<uint4 *>(const_cast<void *>(r.coef)), r.nin_total, r.nout, 0};
+        coef_blocks = tensor_coef_ctas(r.nin_total, r.nout);
+    }
+    const unsigned long long pairs = (n + 1) / 2, form_blocks = pairs * ((r.nin + 63) / 64),
+                             grid = coef_blocks + form_blocks + z.blocks;
+    if (grid > 0x7fffffffull) {
+        set_error("tensor multiply-accumulate: grid too large");
+        return P2G_ERANGE;
+    }
+    prepare_tensor<<<static_cast<unsigned>(grid), 256, 0, st>>>(
+        p, glog, gexp, static_cast<unsigned>(coef_blocks), r.src, r.nin, std::min(r.S, byte0 + n * kTensorM * 2),
+        byte0, static_cast<uint32_t *>(r.forms), static_cast<unsigned>(pairs), static_cast<unsigned>(form_blocks), z);
     P2G_CUDA(cudaGetLastError());
     return P2G_OK;
 }

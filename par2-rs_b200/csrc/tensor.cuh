@@ -1,6 +1,7 @@
 // tensor.cuh -- host launchers of the tensor-core multiply-accumulate.
 #pragma once
 #include "common.cuh"
+#include "prep.cuh"
 
 namespace p2g {
 
@@ -24,11 +25,9 @@ size_t tensor_coef_bytes(int nin, int nout);
 // Bytes of the symbol operand for `tiles` tiles of 128 symbols of nin inputs.
 size_t tensor_form_bytes(int nin, size_t tiles);
 
-// The coefficient operand from a row-major matrix coeff[nout][nin], or of the
-// PAR2 matrix consts[i]^exps[o].
-int tensor_coef_matrix(cudaStream_t st, const uint16_t *d_coeff, int nin, int nout, void *coef);
-int tensor_coef_par2(cudaStream_t st, const uint16_t *d_consts, const uint32_t *d_exps,
-                     const uint16_t *glog, const uint16_t *gexp, int nin, int nout, void *coef);
+// The coefficient operand.
+int tensor_coefs(cudaStream_t st, const CoefSource &c, const uint16_t *glog, const uint16_t *gexp,
+                 int nin, int nout, void *coef);
 
 // SM clocks that a problem takes (an estimate), and the parts its work is split
 // into for that (folded with atomic XOR).
@@ -55,8 +54,11 @@ struct TensorRun {
     int *err;     // device-visible word, set when a bounded wait gave up
 };
 inline size_t tensor_tiles(size_t S) { return (S / 2 + kTensorM - 1) / kTensorM; }
-// The forms of tiles [t0, t0 + n), then the products of the same tiles.
-int tensor_forms(cudaStream_t st, const TensorRun &r, size_t t0, size_t n);
+// The forms of tiles [t0, t0 + n), the coefficient operand (r.coef, of the whole
+// problem) where `todo` is given, and zeroed outputs; then the products of the
+// same tiles.
+int tensor_prepare(cudaStream_t st, const TensorRun &r, size_t t0, size_t n, const CoefSource *todo,
+                   const uint16_t *glog, const uint16_t *gexp, const ZeroOutputs &z);
 int tensor_products(cudaStream_t st, const TensorRun &r, size_t t0, size_t n);
 
 // ---- batches: the same three kernels over many problems -------------------
@@ -79,8 +81,8 @@ struct TensorArgs {
 struct TensorItem {
     int prob, pair, nb, part;
 };
-// `first`: the problem's first CTA (forms: tile pairs x 64-input groups) or
-// thread (coefficients: rows x blocks x words) of the batched launch.
+// `first`: the problem's first CTA of the batched launch (forms: tile pairs x
+// 64-input groups; coefficients: 32 rows x 4 words).
 struct TensorFormProb {
     const uint8_t *const *src;
     uint32_t *forms;
@@ -100,9 +102,10 @@ inline unsigned long long tensor_form_ctas(int nin, size_t S)
 {
     return static_cast<unsigned long long>((tensor_tiles(S) + 1) / 2) * ((nin + 63) / 64);
 }
-inline unsigned long long tensor_coef_threads(int nin, int nout)
+inline unsigned long long tensor_coef_ctas(int nin, int nout)
 {
-    return static_cast<unsigned long long>(tensor_rows(nout)) * tensor_blocks(nout) * tensor_words(nin);
+    return static_cast<unsigned long long>((tensor_rows(nout) * tensor_blocks(nout) + 31) / 32) *
+           ((tensor_words(nin) + 3) / 4);
 }
 // SM clocks per tile pair of a problem that runs among others: the products of
 // all its output blocks, and the forms.
@@ -112,7 +115,7 @@ double tensor_item_clocks(int nin, int nout, int products);
 
 int tensor_batch_forms(cudaStream_t st, const TensorFormProb *d, int np, unsigned long long ctas);
 int tensor_batch_coefs(cudaStream_t st, const uint16_t *glog, const uint16_t *gexp,
-                       const TensorCoefProb *d, int np, unsigned long long threads);
+                       const TensorCoefProb *d, int np, unsigned long long ctas);
 // One CTA per item, in the order given (longest first); `rows` the largest of
 // the problems'.  A CTA that starts once *abort is set does nothing.
 int tensor_batch(cudaStream_t st, const TensorArgs *probs, const TensorItem *items, int nitems, int rows,
