@@ -946,14 +946,9 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
     }
     b->hash_warps_off = img.put(nullptr, hwarps * sizeof(HashWarp));
     b->nhash_warps = hwarps;
-    if (hwarps && !ctx->side_stream) {
-        if (cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->join_ev, cudaEventDisableTiming) != cudaSuccess) {
-            set_error("p2g_batch_create: cudaStreamCreate failed");
-            return fail(P2G_ECUDA);
-        }
-    }
+    if (hwarps)
+        if (int rc = ensure_side(ctx))
+            return fail(rc);
     if (int rc = take(ctx, b->hashbuf, hbytes + 256))
         return fail(rc);
     if (int rc = take(ctx, b->params, img.bytes.size() + 256))

@@ -74,8 +74,9 @@ struct p2g_ctx {
     cudaStream_t d2h_stream = nullptr;
     // the copy that raises a running batch's abort word (p2g_batch_cancel)
     cudaStream_t cancel_stream = nullptr;
-    // verification beside a batch's multiply-accumulate work (created on
-    // first use, with the events that fork and join it)
+    // verification beside a batch's multiply-accumulate work, a small inversion
+    // beside a repair's first pass (ensure_side, with the events that fork and
+    // join it)
     cudaStream_t side_stream = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     static constexpr int kPipe = 16;        // input groups of a host encode
@@ -133,6 +134,8 @@ namespace p2g {
 void deferred_release(p2g_ctx *ctx);
 // After a synchronisation: P2G_ETIMEOUT if a kernel's bounded wait gave up.
 int check_waits(p2g_ctx *ctx);
+// Creates the context's side stream and its events on first use.
+int ensure_side(p2g_ctx *ctx);
 }  // namespace p2g
 
 #define P2G_CUDA(call)                                                                  \

@@ -1191,6 +1191,8 @@ int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uin
     return P2G_OK;
 }
 
+bool gj_one_cta(int m) { return m <= kSmallM; }
+
 int gj_status(p2g_ctx *ctx, GjWork &w, int *singular)
 {
     int h = 0;

@@ -19,6 +19,10 @@ struct GjWork {
 int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uint32_t *d_exps,
               const uint32_t *h_exps, const uint16_t *d_A, uint16_t *d_inv);
 
+// Whether an inversion of m rows runs in one CTA, without the multiply-accumulate
+// kernels and their scratch: it can then run beside them, on another stream.
+bool gj_one_cta(int m);
+
 // Waits for the inversion and reads its status (1 = singular).
 int gj_status(p2g_ctx *ctx, GjWork &w, int *singular);
 

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256)
     prepare_tables(const CoefSource c, const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp,
                    int cnin, int nout, uint32_t *__restrict__ recs, unsigned rec_blocks,
                    const uint8_t *const *__restrict__ src, int nin, int T, size_t S,
-                   uint32_t *__restrict__ planes, unsigned plane_blocks, const ZeroOutputs z)
+                   uint32_t *__restrict__ planes, unsigned plane_blocks, const OutputPrep z)
 {
     unsigned b = blockIdx.x;
     if (b < rec_blocks) {
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256)
     if (b < plane_blocks)
         planes_of_group(src, nin, T, S, planes, static_cast<size_t>(b) * 256 + threadIdx.x);
     else
-        zero_block(z, b - plane_blocks);
+        output_block(z, b - plane_blocks);
 }
 
 // WARPS warps per CTA; each output group of EREG outputs is held by PSPLIT
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(kBatchWarps * 32, 1)
 }
 
 // Zeroes outputs before a split (atomic-XOR) run in store mode.
-__global__ void __launch_bounds__(256) zero_slices(const ZeroOutputs z) { zero_block(z, blockIdx.x); }
+__global__ void __launch_bounds__(256) zero_slices(const OutputPrep z) { output_block(z, blockIdx.x); }
 
 using KernelFn = void (*)(const uint32_t *, const uint32_t *, int, int, int, int, int,
                           uint8_t *const *, size_t, int);
@@ -1016,7 +1016,7 @@ int records_from_matrix(p2g_ctx *ctx, const uint16_t *d_coeff, int nin, int nout
 
 static int launch_zero(cudaStream_t st, uint8_t *const *d_dst, int nout, size_t S)
 {
-    const ZeroOutputs z = zero_blocks(d_dst, nout, S);
+    const OutputPrep z = output_prep(d_dst, nout, S, true);
     zero_slices<<<z.blocks, 256, 0, st>>>(z);
     P2G_CUDA(cudaGetLastError());
     return P2G_OK;
@@ -1042,11 +1042,11 @@ static int launch_kernel(cudaStream_t stream, const MuladdPlan &p, const uint32_
     return P2G_OK;
 }
 
-// muladd_run, after which the records of `todo` (op's, when not null) are
-// written as well.
+// muladd_run for op (when not null), whose records are written as well while
+// they are pending.
 static int tables_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_t *const *d_dst,
                       int nout, size_t S, const uint32_t *d_recs, int mode, const MuladdPlan *plan,
-                      MulOp *todo)
+                      const MulOp *op)
 {
     if (nout <= 0)
         return P2G_OK;
@@ -1068,14 +1068,15 @@ static int tables_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_
     P2G_TRY(ctx->planes.ensure(plane_bytes));
     uint32_t *planes = ctx->planes.as<uint32_t>();
     const size_t groups = static_cast<size_t>(nin) * T * 32;
-    const size_t recs = todo ? static_cast<size_t>(todo->nin) * nout : 0;
-    const ZeroOutputs z = p.nsplit > 1 && mode == 0 ? zero_blocks(d_dst, nout, S) : ZeroOutputs{};
+    const size_t recs = op && op->pending ? static_cast<size_t>(op->nin) * nout : 0;
+    const OutputPrep z = output_prep(d_dst, nout, S, p.nsplit > 1 && mode == 0, op ? op->status : nullptr,
+                                     op ? op->alt : nullptr);
     const unsigned rec_blocks = static_cast<unsigned>((recs + 255) / 256),
                    plane_blocks = static_cast<unsigned>((groups + 255) / 256);
     ctx->mark(1);
     prepare_tables<<<rec_blocks + plane_blocks + z.blocks, 256, 0, ctx->stream>>>(
-        todo ? todo->todo : CoefSource{}, ctx->d_log, ctx->d_exp, todo ? todo->nin : 0, nout,
-        todo ? const_cast<uint32_t *>(todo->coef) : nullptr, rec_blocks, d_src, nin, T, S, planes, plane_blocks,
+        op ? op->todo : CoefSource{}, ctx->d_log, ctx->d_exp, op ? op->nin : 0, nout,
+        op ? const_cast<uint32_t *>(op->coef) : nullptr, rec_blocks, d_src, nin, T, S, planes, plane_blocks,
         z);
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
@@ -1208,11 +1209,10 @@ int mulop_run(p2g_ctx *ctx, MulOp &op, const uint8_t *const *d_src, int i0, int 
     if (!op.plan.tensor) {
         // part of the inputs, or of the columns, has a plan of its own
         const bool whole = i0 == 0 && n == op.nin && S == op.S;
-        const bool pending = op.pending && n > 0;
         P2G_TRY(tables_run(ctx, d_src, n, d_dst, op.nout, S,
                            op.coef + static_cast<size_t>(i0) * op.nout * record_words(op.nout), mode,
-                           whole ? &op.plan : nullptr, pending ? &op : nullptr));
-        op.pending = op.pending && !pending;
+                           whole ? &op.plan : nullptr, &op));
+        op.pending = op.pending && n == 0;
         return P2G_OK;
     }
     if (n == 0) {
@@ -1253,8 +1253,8 @@ int mulop_run(p2g_ctx *ctx, MulOp &op, const uint8_t *const *d_src, int i0, int 
     ctx->mark(1);
     for (size_t t0 = 0; t0 < tiles; t0 += chunk) {
         const size_t nt = std::min(chunk, tiles - t0);
-        const ZeroOutputs z =
-            t0 == 0 && r.split > 1 && mode == 0 ? zero_blocks(d_dst, op.nout, S) : ZeroOutputs{};
+        const OutputPrep z =
+            t0 == 0 ? output_prep(d_dst, op.nout, S, r.split > 1 && mode == 0, op.status, op.alt) : OutputPrep{};
         P2G_TRY(tensor_prepare(ctx->stream, r, t0, nt, op.pending ? &op.todo : nullptr, ctx->d_log, ctx->d_exp, z));
         op.pending = false;
         if (t0 == 0)

@@ -153,6 +153,10 @@ struct MulOp {
     const uint32_t *coef = nullptr;
     CoefSource todo;       // what the coefficients are written from
     bool pending = false;  // not written yet
+    // a device word that, when set by the time a run starts, sends the results
+    // to the slices of the device array `alt` (a run with at least one input)
+    const int *status = nullptr;
+    uint8_t *const *alt = nullptr;
 };
 // Chooses the plan of an nin x nout problem over slices of S bytes (the
 // context's own plan for that shape if it has one, else by the sizes).

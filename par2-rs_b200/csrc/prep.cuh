@@ -14,27 +14,44 @@ struct CoefSource {
     const uint32_t *exps = nullptr;
 };
 
-// Zeroes nout outputs of S bytes (for partial results that are XORed in).
-struct ZeroOutputs {
-    uint8_t *const *dst = nullptr;
+// The outputs: zeroed where partial results are XORed in; and, if *status is
+// set by the time the launch runs, put aside -- the device array of their
+// addresses gets the addresses `alt` instead, so that nothing is written to them.
+struct OutputPrep {
+    uint8_t **dst = nullptr;
     size_t S = 0;
-    int per = 0;  // blocks of 256 threads per output
-    unsigned blocks = 0;
+    int n = 0, per = 0;                   // outputs; zeroing blocks of each
+    unsigned zero_blocks = 0, blocks = 0;  // of 256 threads
+    const int *status = nullptr;
+    uint8_t *const *alt = nullptr;
 };
-inline ZeroOutputs zero_blocks(uint8_t *const *dst, int nout, size_t S)
+inline OutputPrep output_prep(uint8_t *const *dst, int n, size_t S, bool zero, const int *status = nullptr,
+                              uint8_t *const *alt = nullptr)
 {
-    ZeroOutputs z;
-    z.dst = dst;
+    OutputPrep z;
+    z.dst = const_cast<uint8_t **>(dst);
     z.S = S;
+    z.n = n;
     z.per = static_cast<int>(std::min<size_t>((S + 4095) / 4096, 1024));
-    z.blocks = static_cast<unsigned>(z.per) * static_cast<unsigned>(nout);
+    z.zero_blocks = zero ? static_cast<unsigned>(z.per) * static_cast<unsigned>(n) : 0;
+    z.blocks = z.zero_blocks + (status ? 1 : 0);
+    z.status = status;
+    z.alt = alt;
     return z;
 }
 
 #ifdef __CUDACC__
 // Block b of the z.blocks (256 threads each).
-__device__ __forceinline__ void zero_block(const ZeroOutputs &z, unsigned b)
+__device__ __forceinline__ void output_block(const OutputPrep &z, unsigned b)
 {
+    const bool aside = z.status && *z.status != 0;
+    if (b >= z.zero_blocks) {
+        for (int i = threadIdx.x; aside && i < z.n; i += 256)
+            z.dst[i] = z.alt[i];
+        return;
+    }
+    if (aside)
+        return;
     uint8_t *d = z.dst[b / z.per];
     for (size_t x = (static_cast<size_t>(b % z.per) * 256 + threadIdx.x) * 16; x < z.S;
          x += static_cast<size_t>(z.per) * 4096) {

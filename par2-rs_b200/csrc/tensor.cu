@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     prepare_tensor(const TensorCoefProb p, const uint16_t *__restrict__ glog, const uint16_t *__restrict__ gexp,
                    unsigned coef_blocks, const uint8_t *const *__restrict__ src, int nin, size_t S, size_t byte0,
-                   uint32_t *__restrict__ forms, unsigned pairs, unsigned form_blocks, const ZeroOutputs z)
+                   uint32_t *__restrict__ forms, unsigned pairs, unsigned form_blocks, const OutputPrep z)
 {
     unsigned b = blockIdx.x;
     if (b < coef_blocks) {
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(256)
     if (b < form_blocks)
         forms_of_pair(src, nin, S, byte0, forms, b % pairs, b / pairs);
     else
-        zero_block(z, b - form_blocks);
+        output_block(z, b - form_blocks);
 }
 
 // ---- the products ----------------------------------------------------------
@@ -1174,7 +1174,7 @@ int tensor_batch(cudaStream_t st, const TensorArgs *probs, const TensorItem *ite
 }
 
 int tensor_prepare(cudaStream_t st, const TensorRun &r, size_t t0, size_t n, const CoefSource *todo,
-                   const uint16_t *glog, const uint16_t *gexp, const ZeroOutputs &z)
+                   const uint16_t *glog, const uint16_t *gexp, const OutputPrep &z)
 {
     const size_t byte0 = t0 * kTensorM * 2;
     TensorCoefProb p{};

@@ -55,10 +55,10 @@ struct TensorRun {
 };
 inline size_t tensor_tiles(size_t S) { return (S / 2 + kTensorM - 1) / kTensorM; }
 // The forms of tiles [t0, t0 + n), the coefficient operand (r.coef, of the whole
-// problem) where `todo` is given, and zeroed outputs; then the products of the
+// problem) where `todo` is given, and the outputs' start; then the products of the
 // same tiles.
 int tensor_prepare(cudaStream_t st, const TensorRun &r, size_t t0, size_t n, const CoefSource *todo,
-                   const uint16_t *glog, const uint16_t *gexp, const ZeroOutputs &z);
+                   const uint16_t *glog, const uint16_t *gexp, const OutputPrep &z);
 int tensor_products(cudaStream_t st, const TensorRun &r, size_t t0, size_t n);
 
 // ---- batches: the same three kernels over many problems -------------------
