@@ -11,15 +11,23 @@
 //     final XOR 0xFFFFFFFF, computed four bytes at a time with four 256-entry
 //     tables ("slicing by 4").
 //
-// One lane owns one slice (MD5 is a serial chain over the slice) and computes
-// both checksums from the same registers.  The 32 slices of a warp stream
-// through a 3-stage shared-memory ring filled by cp.async: eight lanes copy
-// 128 contiguous bytes of one slice (coalesced), the 16-byte units of each
-// slice row are XOR-swizzled by the slice index so that the lanes' 16-byte
-// reads of their own rows never conflict, and the copy of chunk c+2 is in
-// flight while chunk c is hashed.  The four CRC tables are replicated 32 times
-// in shared memory so that lane L always reads bank L: data-dependent table
-// reads never conflict.
+// One lane owns one slice (MD5 is a serial chain over the slice), in a team of
+// two warps: one computes the MD5s and does nothing else, the other copies the
+// slices for both and computes the CRCs, on another scheduler as long as there
+// are one or two teams on the SM.  The 32 slices of a team stream through a
+// 3-stage shared-memory ring filled by cp.async: eight lanes copy 128 contiguous
+// bytes of one slice (coalesced), the 16-byte units of each slice row are
+// XOR-swizzled by the slice index so that the lanes' 16-byte reads of their own
+// rows never conflict, and the copy of chunk c+2 is in flight while chunk c is
+// hashed.  The four CRC tables are replicated 32 times in shared memory so that
+// lane L always reads bank L: data-dependent table reads never conflict.
+//
+// Bounds, on one B200: few slices, by MD5's chain: a block of 64 bytes takes 990
+// clocks, of which its 64 steps alone 909 (300 slices of 1 MiB 8.28 ms; 9.68 with
+// one warp for copies, CRC and MD5, which issues 496 instructions a block; 9.40
+// with the team's warps on one scheduler).  Many, by the integer pipe: 32000
+// slices of 64 KiB 0.84 ms, at about 70 % of its rate on average over the SM's
+// schedulers, some of which have two MD5 warps and others one.
 #include <algorithm>
 
 #include "async.cuh"
@@ -45,8 +53,8 @@ __device__ __forceinline__ uint32_t rotl(uint32_t x, int s) { return __funnelshi
 // One RFC 1321 block transform of the 16 little-endian words x.  The chain
 // through a step is the function of b, an addition, the rotation and the
 // addition of b; the other addends are summed ahead, behind an asm barrier
-// without which the compiler puts them back into the chain (300 slices of 1 MiB:
-// 9.88 -> 9.68 ms, 32000 of 64 KiB: 0.855 -> 0.839).
+// without which the compiler puts them back into the chain (300 slices of 1 MiB
+// with copies, CRC and MD5 in one warp: 9.88 -> 9.68 ms).
 __device__ __forceinline__ void md5_block(uint32_t st[4], const uint32_t x[16])
 {
     uint32_t a = st[0], b = st[1], c = st[2], d = st[3];
@@ -91,14 +99,14 @@ __device__ __forceinline__ void md5_block(uint32_t st[4], const uint32_t x[16])
     st[3] += d;
 }
 
-constexpr int kHashThreads = 256;
-constexpr int kHashWarps = kHashThreads / 32;
+constexpr int kHashTeams = 8;  // of an MD5 and a CRC warp, 32 slices each
+constexpr int kHashThreads = kHashTeams * 64;
 constexpr int kCrcTabWords = 4 * 256 * 32;  // 4 tables x 256 entries x 32 bank copies
 constexpr int kChunk = 128;                 // bytes of every slice per ring stage
 constexpr int kStages = 3;
-constexpr int kStageBytes = 32 * kChunk;    // one warp's 32 slices
+constexpr int kStageBytes = 32 * kChunk;    // one team's 32 slices
 constexpr size_t kHashSmem =
-    static_cast<size_t>(kCrcTabWords) * 4 + static_cast<size_t>(kHashWarps) * kStages * kStageBytes;
+    static_cast<size_t>(kCrcTabWords) * 4 + static_cast<size_t>(kHashTeams) * kStages * kStageBytes;
 
 // CRC table layout in shared memory: tables 2p and 2p+1 share a 64 KiB
 // region p, whose row e (256 bytes) holds entry e of table 2p in its first
@@ -136,7 +144,7 @@ __device__ __forceinline__ uint32_t crc_byte(const uint32_t *stab, uint32_t crc,
 // byte offset of 16-byte unit u of slice row s inside a stage
 __device__ __forceinline__ int stage_pos(int s, int u) { return s * kChunk + ((u ^ (s & 7)) << 4); }
 
-// Copies bytes [off, off + kChunk) of the warp's slices into a stage: lane L
+// Copies bytes [off, off + kChunk) of a team's slices into a stage: lane L
 // moves unit L % 8 of slices L / 8, 4 + L / 8, ... (null pointer: no slice).
 __device__ __forceinline__ void stage_chunk(uint8_t *stage, const uint8_t *const ptr[8], size_t off,
                                             int lane)
@@ -150,15 +158,6 @@ __device__ __forceinline__ void stage_chunk(uint8_t *stage, const uint8_t *const
     }
 }
 
-__device__ __forceinline__ void hash_block(const uint32_t *stab, uint32_t st[4], uint32_t &crc,
-                                           const uint32_t x[16], const CrcLanes &L)
-{
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        crc = crc_word(stab, crc, x[j], L);
-    md5_block(st, x);
-}
-
 // Fills the CTA's copy of the CRC tables (all threads; ends with a barrier).
 __device__ __forceinline__ void load_crc_tables(uint32_t *stab, const uint32_t *__restrict__ crc_tables)
 {
@@ -169,10 +168,31 @@ __device__ __forceinline__ void load_crc_tables(uint32_t *stab, const uint32_t *
     __syncthreads();
 }
 
-// One warp hashes `count` (1 to 32) slices of S bytes, lane L slices[L]; md5
-// and crc are the results' places of slices[0].
-__device__ __forceinline__ void hash_warp(const uint32_t *stab, uint8_t *ring, const uint8_t *const *slices,
-                                          int count, size_t S, uint8_t *md5, uint32_t *crc_out)
+// 16 words of block b of this lane's slice in a stage
+__device__ __forceinline__ void load_block(const uint8_t *stage, int lane, int b, uint32_t x[16])
+{
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(stage + stage_pos(lane, 4 * b + v));
+        x[4 * v] = q.x;
+        x[4 * v + 1] = q.y;
+        x[4 * v + 2] = q.z;
+        x[4 * v + 3] = q.w;
+    }
+}
+
+// Both warps of a team: what the CRC warp copied is there for both, and what
+// both have read may be written again.
+__device__ __forceinline__ void team_barrier(int team)
+{
+    __syncwarp();
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + team) : "memory");
+}
+
+// The CRC warp of a team: copies the slices' chunks for both warps, and lane L
+// computes the CRC32 of slices[L].
+__device__ __forceinline__ void crc_warp(const uint32_t *stab, uint8_t *ring, const uint8_t *const *slices,
+                                         int count, size_t S, uint32_t *crc_out, int team)
 {
     const int lane = threadIdx.x & 31;
     const CrcLanes CL{crc_base(0, lane), crc_base(1, lane), crc_base(2, lane), crc_base(3, lane)};
@@ -183,7 +203,6 @@ __device__ __forceinline__ void hash_warp(const uint32_t *stab, uint8_t *ring, c
         ptr[i] = g < count ? slices[g] : nullptr;
     }
     const bool active = lane < count;
-    uint32_t st[4] = {0x67452301u, 0xefcdab89u, 0x98badcfeu, 0x10325476u};
     uint32_t crc = 0xFFFFFFFFu;
     const size_t nch = S / kChunk;
 #pragma unroll
@@ -195,31 +214,54 @@ __device__ __forceinline__ void hash_warp(const uint32_t *stab, uint8_t *ring, c
     int cur = 0;
     for (size_t c = 0; c < nch; ++c) {
         cp_async_wait<kStages - 2>();  // this lane's copies of chunk c have landed
-        __syncwarp();                  // ... and every other lane's; chunk c-1 is consumed
+        team_barrier(team);            // ... and every other lane's; chunk c-1 is consumed
         const size_t pre = c + kStages - 1;
         const int pst = cur == 0 ? kStages - 1 : cur - 1;
         if (pre < nch)
             stage_chunk(ring + pst * kStageBytes, ptr, pre * kChunk, lane);
         cp_async_commit();
         if (active) {
-            const uint8_t *row = ring + cur * kStageBytes;
 #pragma unroll
             for (int b = 0; b < kChunk / 64; ++b) {
                 uint32_t x[16];
+                load_block(ring + cur * kStageBytes, lane, b, x);
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const uint4 q = *reinterpret_cast<const uint4 *>(row + stage_pos(lane, 4 * b + v));
-                    x[4 * v] = q.x;
-                    x[4 * v + 1] = q.y;
-                    x[4 * v + 2] = q.z;
-                    x[4 * v + 3] = q.w;
-                }
-                hash_block(stab, st, crc, x, CL);
+                for (int j = 0; j < 16; ++j)
+                    crc = crc_word(stab, crc, x[j], CL);
             }
         }
         cur = cur == kStages - 1 ? 0 : cur + 1;
     }
     cp_async_wait<0>();
+    if (!active)
+        return;
+    const uint8_t *t = slices[lane] + nch * kChunk;
+    for (size_t b = 0; b < S - nch * kChunk; ++b)
+        crc = crc_byte(stab, crc, t[b], CL);
+    crc_out[lane] = crc ^ 0xFFFFFFFFu;
+}
+
+// The MD5 warp of a team: lane L computes the MD5 of slices[L].
+__device__ __forceinline__ void md5_warp(const uint8_t *ring, const uint8_t *const *slices, int count,
+                                         size_t S, uint8_t *md5, int team)
+{
+    const int lane = threadIdx.x & 31;
+    const bool active = lane < count;
+    uint32_t st[4] = {0x67452301u, 0xefcdab89u, 0x98badcfeu, 0x10325476u};
+    const size_t nch = S / kChunk;
+    int cur = 0;
+    for (size_t c = 0; c < nch; ++c) {
+        team_barrier(team);
+        if (active) {
+#pragma unroll
+            for (int b = 0; b < kChunk / 64; ++b) {
+                uint32_t x[16];
+                load_block(ring + cur * kStageBytes, lane, b, x);
+                md5_block(st, x);
+            }
+        }
+        cur = cur == kStages - 1 ? 0 : cur + 1;
+    }
     if (!active)
         return;
     // the last S % 128 bytes: one more full 64-byte block if there is one,
@@ -237,18 +279,15 @@ __device__ __forceinline__ void hash_warp(const uint32_t *stab, uint8_t *ring, c
             x[4 * v + 2] = u.z;
             x[4 * v + 3] = u.w;
         }
-        hash_block(stab, st, crc, x, CL);
+        md5_block(st, x);
         t += 64;
         rem -= 64;
     }
 #pragma unroll
     for (int j = 0; j < 16; ++j)
         x[j] = 0;
-    for (size_t b = 0; b < rem; ++b) {
-        uint32_t v = t[b];
-        crc = crc_byte(stab, crc, v, CL);
-        x[b >> 2] |= v << (8 * (b & 3));
-    }
+    for (size_t b = 0; b < rem; ++b)
+        x[b >> 2] |= static_cast<uint32_t>(t[b]) << (8 * (b & 3));
     x[rem >> 2] |= 0x80u << (8 * (rem & 3));
     const uint64_t bits = static_cast<uint64_t>(S) * 8;
     if (rem >= 56) {
@@ -261,13 +300,29 @@ __device__ __forceinline__ void hash_warp(const uint32_t *stab, uint8_t *ring, c
     x[15] = static_cast<uint32_t>(bits >> 32);
     md5_block(st, x);
     *reinterpret_cast<uint4 *>(md5 + lane * 16) = make_uint4(st[0], st[1], st[2], st[3]);
-    crc_out[lane] = crc ^ 0xFFFFFFFFu;
 }
 
-__device__ __forceinline__ uint8_t *warp_ring(uint32_t *stab)
+// This warp's team: warps 0-7 are the MD5 warps of teams 0-7, warps 8-15 the CRC
+// warps of teams 6, 7, 0, ... 5, so that the two warps of a team are on different
+// schedulers (warp % 4).
+__device__ __forceinline__ int warp_team()
 {
-    return reinterpret_cast<uint8_t *>(stab + kCrcTabWords) +
-           static_cast<size_t>(threadIdx.x >> 5) * kStages * kStageBytes;
+    const int warp = threadIdx.x >> 5;
+    return warp < kHashTeams ? warp : (warp + 6) % kHashTeams;
+}
+
+// A team of two warps hashes `count` (1 to 32) slices of S bytes; md5 and crc
+// are the results' places of slices[0].
+__device__ __forceinline__ void hash_team(uint32_t *stab, const uint8_t *const *slices, int count, size_t S,
+                                          uint8_t *md5, uint32_t *crc)
+{
+    const int team = warp_team();
+    uint8_t *ring = reinterpret_cast<uint8_t *>(stab + kCrcTabWords) +
+                    static_cast<size_t>(team) * kStages * kStageBytes;
+    if (threadIdx.x < kHashTeams * 32)
+        md5_warp(ring, slices, count, S, md5, team);
+    else
+        crc_warp(stab, ring, slices, count, S, crc, team);
 }
 
 __global__ void __launch_bounds__(kHashThreads, 1)
@@ -277,25 +332,26 @@ __global__ void __launch_bounds__(kHashThreads, 1)
 {
     extern __shared__ __align__(16) uint32_t stab[];
     load_crc_tables(stab, crc_tables);
-    // this CTA hashes slices [blockIdx * per_cta, end), 32 to a warp
-    const int first = blockIdx.x * per_cta + (threadIdx.x >> 5) * 32;
+    // this CTA hashes slices [blockIdx * per_cta, end), 32 to a team
+    const int first = blockIdx.x * per_cta + warp_team() * 32;
     const int end = min(n, (blockIdx.x + 1) * per_cta);
     if (first < end)
-        hash_warp(stab, warp_ring(stab), slices + first, min(32, end - first), S,
-                  md5_out + static_cast<size_t>(first) * 16, crc_out + first);
+        hash_team(stab, slices + first, min(32, end - first), S, md5_out + static_cast<size_t>(first) * 16,
+                  crc_out + first);
 }
 
-// Slices of several sizes in one launch: warps take groups of up to 32 slices
+// Slices of several sizes in one launch: teams take groups of up to 32 slices
 // of one size, longest first, dealt over the CTAs.
 __global__ void __launch_bounds__(kHashThreads, 1)
     hash_groups_kernel(const HashWarp *__restrict__ groups, int n, const uint32_t *__restrict__ crc_tables)
 {
     extern __shared__ __align__(16) uint32_t stab[];
     load_crc_tables(stab, crc_tables);
-    for (int g = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; g < n; g += gridDim.x * kHashWarps) {
+    const int team = warp_team();
+    for (int g = blockIdx.x + team * gridDim.x; g < n; g += gridDim.x * kHashTeams) {
         const HashWarp h = groups[g];
-        hash_warp(stab, warp_ring(stab), h.slices, h.count, h.S, h.md5, h.crc);
-        __syncwarp();
+        hash_team(stab, h.slices, h.count, h.S, h.md5, h.crc);
+        team_barrier(team);  // the ring is free for the next group
     }
 }
 
@@ -324,7 +380,7 @@ int hash_run(p2g_ctx *ctx, const uint8_t *const *d_slices, int n, size_t S, uint
                                   static_cast<int>(smem)));
     // spread the slices over every SM (one CTA per SM fits), at most 256 per CTA
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
-    const int per_cta = std::min(kHashThreads, std::max(1, (n + sms - 1) / sms));
+    const int per_cta = std::min(kHashTeams * 32, std::max(1, (n + sms - 1) / sms));
     const int grid = (n + per_cta - 1) / per_cta;
     hash_slices_kernel<<<grid, kHashThreads, smem, ctx->stream>>>(d_slices, n, per_cta, S,
                                                                   ctx->d_crc, d_md5, d_crc);
@@ -334,7 +390,7 @@ int hash_run(p2g_ctx *ctx, const uint8_t *const *d_slices, int n, size_t S, uint
 }
 
 // A group's time is its slices' chain of MD5 blocks whatever else runs, as long
-// as an SM holds no more than about one warp per scheduler: four to a CTA, so
+// as an SM holds no more than about one team per scheduler: four to a CTA, so
 // that the launch leaves the other SMs to the work it runs beside.
 int hash_groups(cudaStream_t st, int sms, const uint32_t *crc_tables, const HashWarp *d_groups, int n)
 {
