@@ -727,10 +727,10 @@ struct VdmSmallSmem {
     uint32_t T[kVdmSmall / 32 * kNibbleWords];
     uint16_t QT[kVdmSmall * kVdmQtLd];
 };
-__global__ void __launch_bounds__(kVdmSmall)
-    vdm_small(const uint16_t *__restrict__ x, const uint32_t *__restrict__ exps, uint32_t s, int m, int ld,
-              uint16_t *__restrict__ inv, int *__restrict__ status, const uint16_t *__restrict__ glog,
-              const uint16_t *__restrict__ gexp)
+__device__ __forceinline__ void vdm_small_cta(const uint16_t *__restrict__ x, const uint32_t *__restrict__ exps,
+                                              uint32_t s, int m, int ld, uint16_t *__restrict__ inv,
+                                              int *__restrict__ status, const uint16_t *__restrict__ glog,
+                                              const uint16_t *__restrict__ gexp)
 {
     extern __shared__ __align__(16) uint8_t raw[];
     VdmSmallSmem &sm = *reinterpret_cast<VdmSmallSmem *>(raw);
@@ -770,6 +770,24 @@ __global__ void __launch_bounds__(kVdmSmall)
         inv[static_cast<size_t>(row) * ld + r] =
             static_cast<uint16_t>(gmul(sm.scale[row], sm.QT[static_cast<int>(exps[r] - s) * kVdmQtLd + row], glog, gexp));
     }
+}
+
+__global__ void __launch_bounds__(kVdmSmall)
+    vdm_small(const SmallInverse one, const SmallInverse *__restrict__ items, const uint16_t *__restrict__ glog,
+              const uint16_t *__restrict__ gexp)
+{
+    const SmallInverse t = items ? items[blockIdx.x] : one;
+    vdm_small_cta(t.x, t.exps, t.s, t.m, t.ld, t.inv, t.status, glog, gexp);
+}
+
+static int launch_vdm_small(p2g_ctx *ctx, const SmallInverse &one, const SmallInverse *d_items, int n)
+{
+    P2G_CUDA(cudaFuncSetAttribute(vdm_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(VdmSmallSmem))));
+    vdm_small<<<n, kVdmSmall, sizeof(VdmSmallSmem), ctx->stream>>>(one, d_items, ctx->d_log, ctx->d_exp);
+    P2G_CUDA(cudaGetLastError());
+    ++ctx->launches;
+    return P2G_OK;
 }
 
 // inv[j][r] (row stride ld) = scale[j] * QT[e_r - s][j], through a 32 x 32 shared-memory tile
@@ -820,15 +838,8 @@ static int vdm_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x, const
 {
     const size_t vec = (static_cast<size_t>(m) * 2 + 255) & ~static_cast<size_t>(255);
     P2G_TRY(w.status.ensure(256 + 5 * vec));
-    if (m <= kVdmSmall) {
-        P2G_CUDA(cudaFuncSetAttribute(vdm_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(sizeof(VdmSmallSmem))));
-        vdm_small<<<1, kVdmSmall, sizeof(VdmSmallSmem), ctx->stream>>>(
-            d_x, d_exps, s, m, ld, d_inv, w.status.as<int>(), ctx->d_log, ctx->d_exp);
-        P2G_CUDA(cudaGetLastError());
-        ++ctx->launches;
-        return P2G_OK;
-    }
+    if (m <= kVdmSmall)
+        return launch_vdm_small(ctx, SmallInverse{d_x, d_exps, d_inv, w.status.as<int>(), s, m, ld}, nullptr, 1);
     P2G_TRY(w.M.ensure(static_cast<size_t>(m) * m * 2 + 16));
     uint8_t *aux = w.status.as<uint8_t>();
     int *status = reinterpret_cast<int *>(aux);
@@ -1189,6 +1200,16 @@ int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uin
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
     return P2G_OK;
+}
+
+bool small_inverse(const uint32_t *h_exps, int m, uint32_t *s)
+{
+    return m > 0 && m <= kVdmSmall && exps_are_run(h_exps, m, s);
+}
+
+int small_inverses(p2g_ctx *ctx, const SmallInverse *d_items, int n)
+{
+    return n > 0 ? launch_vdm_small(ctx, SmallInverse{}, d_items, n) : P2G_OK;
 }
 
 bool gj_one_cta(int m) { return m <= kSmallM; }

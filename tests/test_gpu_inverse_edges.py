@@ -55,3 +55,39 @@ def test_repeated_constant_is_singular(ctx, m):
     with pytest.raises(par2gpu.Par2GpuError) as ei:
         ctx.reconstruction_matrix(40000, missing, np.arange(m))
     assert ei.value.code == par2gpu.ESINGULAR
+
+
+def test_inverses_of_a_batch(ctx):
+    """Repairs whose inverses share a launch (up to 128 consecutive exponents),
+    among larger and gapped ones and an unrepairable one."""
+    import par2gpu
+    import torch
+
+    rng = np.random.default_rng(9)
+    S, jobs, want = 64, [], []
+    for m, first, gap in [(1, 0, 0), (31, 3, 0), (32, 0, 0), (33, 7, 0), (40, 0, 1), (128, 0, 0), (129, 1, 0)]:
+        k = m + 9
+        src = rng.integers(0, 256, (k, S), dtype=np.uint8)
+        exps = first + np.arange(m) + (np.arange(m) >= m // 2) * gap
+        rng.shuffle(exps)
+        missing = np.sort(rng.choice(k, m, replace=False))
+        d = torch.from_numpy(np.delete(src, missing, axis=0)).cuda()
+        rec = torch.from_numpy(oracle.encode(src, exps.astype(np.uint32))).cuda()
+        out = torch.full((m, S), 0x5A, dtype=torch.uint8, device="cuda")
+        jobs.append({"kind": par2gpu.JOB_REPAIR, "k": k, "slice_bytes": S, "src": list(d), "missing": missing,
+                     "exps": exps, "recovery": list(rec), "out": list(out)})
+        want.append((out, src[missing], d, rec))
+    k = 32780
+    d = torch.zeros((1, S), dtype=torch.uint8, device="cuda")
+    out = torch.full((2, S), 0x5A, dtype=torch.uint8, device="cuda")
+    jobs.insert(3, {"kind": par2gpu.JOB_REPAIR, "k": k, "slice_bytes": S, "src": [d[0]] * (k - 2),
+                    "missing": np.array([5, 5 + 32768]), "exps": np.arange(2), "recovery": [d[0], d[0]],
+                    "out": list(out)})
+    b = par2gpu.Batch(ctx, jobs)
+    st = b.run()
+    assert [s != 0 for s in st] == [j == 3 for j in range(len(jobs))], st
+    assert st[3] == par2gpu.ESINGULAR
+    assert bool((out == 0x5A).all())
+    for o, w, _, _ in want:
+        assert np.array_equal(o.cpu().numpy(), w)
+    b.close()
