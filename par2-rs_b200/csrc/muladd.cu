@@ -1122,16 +1122,17 @@ static double table_clocks(const p2g_ctx *ctx, const MuladdPlan &p, int nin, int
 
 // Whether the tensor cores take a problem.  The estimates of both sides are
 // within some 20 % of the clocks measured over 8-8000 inputs, 1-205 outputs and
-// 512 B - 1 MiB, hence the margin of 12 %; the tensor side starts with 34000 more
-// (its coefficient operand, and the launches' latencies: small problems of 45 us
-// are 10-15 us shorter with tables).  On one B200, tables against tensor cores: 2048 x 64 KiB, 205
-// outputs 2300 / 402 us, 13 outputs 335 / 272, 4 outputs 210 / 268; 256 x 64 KiB,
-// 205 outputs 370 / 139, 13 outputs 81 / 81; 64 x 64 KiB, 24 outputs 69 / 77.
+// 512 B - 1 MiB, where calls routed by them take 0.3 % longer than the faster
+// side's on average (at most 20 %).  The margin of 12 % is that of the least
+// loss.  On one B200, calls with tables against tensor cores: 2048 x 64 KiB, 205
+// outputs 2288 / 373 us, 13 outputs 323 / 240, 4 outputs 194 / 239; 256 x 64 KiB,
+// 205 outputs 359 / 120, 13 outputs 74 / 70; 64 x 64 KiB, 24 outputs 61 / 66;
+// 1024 x 4 KiB, 24 outputs 66 / 43, 2 outputs 36 / 39.
 static bool tensor_better(const p2g_ctx *ctx, const MuladdPlan &table, int nin, int nout, size_t S)
 {
     const int sms = ctx && ctx->sm_count > 0 ? ctx->sm_count : 148;
     int split = 1;
-    return 1.12 * tensor_clocks(sms, nin, nout, S, &split) + 34000.0 < table_clocks(ctx, table, nin, nout, S);
+    return 1.12 * tensor_clocks(sms, nin, nout, S, &split) < table_clocks(ctx, table, nin, nout, S);
 }
 
 MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S)
