@@ -196,6 +196,7 @@ __global__ void __launch_bounds__(256)
                    const uint8_t *const *__restrict__ src, int nin, int T, size_t S,
                    uint32_t *__restrict__ planes, unsigned plane_blocks, const OutputPrep z)
 {
+    let_next_start();
     unsigned b = blockIdx.x;
     if (b < rec_blocks) {
         record_of(c, glog, gexp, cnin, nout, recs, static_cast<size_t>(b) * 256 + threadIdx.x);
@@ -501,6 +502,7 @@ __global__ void __launch_bounds__(WARPS * 32, SMALL ? 2 : 1)
                      uint8_t *const *__restrict__ dst, size_t S, int mode)
 {
     extern __shared__ __align__(128) uint8_t smem[];
+    wait_for_previous();
     int bid = blockIdx.x;
     const int split = bid % nsplit;
     bid /= nsplit;
@@ -754,6 +756,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
                   uint8_t *const *__restrict__ dst, size_t S, int mode)
 {
     extern __shared__ __align__(128) uint8_t smem[];
+    wait_for_previous();
     int bid = blockIdx.x;
     const int split = bid % nsplit;
     bid /= nsplit;
@@ -1024,7 +1027,7 @@ static int launch_zero(cudaStream_t st, uint8_t *const *d_dst, int nout, size_t 
 
 static int launch_kernel(cudaStream_t stream, const MuladdPlan &p, const uint32_t *planes,
                          const uint32_t *d_recs, int nin, int nout, int T,
-                         uint8_t *const *d_dst, size_t S, int mode)
+                         uint8_t *const *d_dst, size_t S, int mode, bool linked = false)
 {
     KernelFn fn = kernel_for(p);
     size_t smem = smem_bytes(p);
@@ -1036,9 +1039,8 @@ static int launch_kernel(cudaStream_t stream, const MuladdPlan &p, const uint32_
         set_error("muladd grid too large");
         return P2G_ERANGE;
     }
-    fn<<<static_cast<unsigned>(grid), p.warps * 32, smem, stream>>>(
-        planes, d_recs, nin, nout, T, p.nblk, p.nsplit, d_dst, S, mode);
-    P2G_CUDA(cudaGetLastError());
+    P2G_CUDA(launch_linked(fn, static_cast<unsigned>(grid), p.warps * 32, smem, stream, linked, planes, d_recs, nin,
+                           nout, T, p.nblk, p.nsplit, d_dst, S, mode));
     return P2G_OK;
 }
 
@@ -1081,7 +1083,7 @@ static int tables_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
     ctx->mark(2);
-    P2G_TRY(launch_kernel(ctx->stream, p, planes, d_recs, nin, nout, T, d_dst, S, mode));
+    P2G_TRY(launch_kernel(ctx->stream, p, planes, d_recs, nin, nout, T, d_dst, S, mode, true));
     ++ctx->launches;
     ctx->mark(3);
     return P2G_OK;

@@ -498,6 +498,7 @@ __global__ void __launch_bounds__(256)
                    unsigned coef_blocks, const uint8_t *const *__restrict__ src, int nin, size_t S, size_t byte0,
                    uint32_t *__restrict__ forms, unsigned pairs, unsigned form_blocks, const OutputPrep z)
 {
+    let_next_start();
     unsigned b = blockIdx.x;
     if (b < coef_blocks) {
         coef_block(p, glog, gexp, b);
@@ -1036,6 +1037,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(c.tmem));
         return;
     }
+    if constexpr (!BATCH)
+        wait_for_previous();
     // Registers: 896 threads x 72 = 64512 at launch; 128 x (56 + 2 x 64 + 4 x
     // 80) = 64512 after the split.
     if (wg == 0) {
@@ -1224,8 +1227,8 @@ int tensor_products(cudaStream_t st, const TensorRun &r, size_t t0, size_t n)
         set_error("tensor multiply-accumulate: grid too large");
         return P2G_ERANGE;
     }
-    tensor_muladd<false><<<static_cast<unsigned>(grid), kThreads, smem, st>>>(a, nullptr, nullptr, nullptr);
-    P2G_CUDA(cudaGetLastError());
+    P2G_CUDA(launch_linked(tensor_muladd<false>, static_cast<unsigned>(grid), kThreads, smem, st, true, a, nullptr,
+                           nullptr, nullptr));
     return P2G_OK;
 }
 
