@@ -1076,18 +1076,19 @@ int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missi
     return rc;
 }
 
-// Steps 1-3 of p2g_repair on slices that all are on the device: queued without
-// waiting for the inversion's status.  A singular matrix sends the last step's
+// Steps 1-3 of p2g_repair on slices that all are on the device, for inversions of
+// one CTA: queued without waiting for the inversion's status.  A singular matrix sends the last step's
 // results to the right-hand sides' scratch, so that the caller's outputs stay
-// as they were.  An inversion of one CTA runs beside the first pass, which does
-// not need it.  (13 of 256 slices of 64 KiB: 107 us; 129 with the inversion, 17 us,
-// and the wait for its status ahead of the passes.)
+// as they were.  The inversion runs beside the first pass, which does not need it.  (13 of 256 slices of 64 KiB: 107 us; 129 with the inversion, 17 us,
+// and the wait for its status ahead of the passes.  Beyond 1 GiB of slices that is
+// below 3 %, and a singular matrix would cost a pass that takes longer than that.)
+constexpr size_t kUnattendedBytes = size_t(1) << 30;
 static int repair_unattended(p2g_ctx *ctx, GjWork &w, size_t m, size_t np, size_t slice_bytes,
                              uint8_t *dp, const ParamLayout &L, const uint32_t *d_exps,
                              const uint32_t *exps, MulOp &op)
 {
     const int n = static_cast<int>(m);
-    const bool side = np && p2g::gj_one_cta(n);
+    const bool side = np != 0;
     if (side)
         P2G_TRY(ensure_side(ctx));
     cudaStream_t main = ctx->stream;
@@ -1154,7 +1155,7 @@ static int repair_passes(p2g_ctx *ctx, size_t m, size_t np, size_t slice_bytes, 
     // 1. A^-1 on the device
     P2G_TRY(ctx->inv.ensure(m * m * 2));
     GjWork w{ctx->gj_M, ctx->gj_status};
-    if (dev && !o_st)
+    if (dev && !o_st && p2g::gj_one_cta(static_cast<int>(m)) && np * slice_bytes <= kUnattendedBytes)
         return repair_unattended(ctx, w, m, np, slice_bytes, dp, L, d_exps, exps, tail.op);
     P2G_TRY(gj_invert(ctx, w, static_cast<int>(m), reinterpret_cast<const uint16_t *>(dp + L.a_off),
                       d_exps, exps, nullptr, ctx->inv.as<uint16_t>()));

@@ -7,9 +7,13 @@
 //
 //     dst[o][x] (^)= XOR_i  coeff(i, o) * src[i][x]      (GF(2^16), 0x1100B)
 //
+// Most problems run on the tensor cores (tensor.cu; the rule between the two is
+// tensor_better below).  This file has the lookup tables for the others, and what
+// the two share: plans, the preparing launch, batches' persistent kernel.
+//
 // Design (bit-sliced tables, "method of four Russians" over GF(2)):
 //   * Inputs are first converted to 16 bit planes per group of 32 symbols
-//     (slices_to_planes).  Multiplication by a constant is GF(2)-linear on the
+//     (planes_of_group).  Multiplication by a constant is GF(2)-linear on the
 //     planes (bitslice.cuh).
 //   * A CTA owns one column tile of 1024 symbols (2 KiB of every slice) and a
 //     block of up to 8*EREG outputs; each warp keeps EREG outputs x 16 planes

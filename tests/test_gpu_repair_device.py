@@ -1,7 +1,7 @@
 """Repairs of slices on the device, whose passes are queued before the
-inversion's outcome is known: results at the sizes where the inversion moves to
-the passes' own stream (above 96 rows), and a singular matrix leaving the
-outputs alone with every kind of plan for the last pass."""
+inversion's outcome is known up to 96 rows: results on both sides of that size,
+and a singular matrix leaving the outputs alone with every kind of plan for the
+last pass."""
 import numpy as np
 import pytest
 
