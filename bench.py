@@ -10,9 +10,10 @@ multiply-accumulate.  One "step" is one full encode of that set.
   e2e     the same through the C ABI with pinned HOST buffers: the 2 GiB H2D
           copy of the sources and the D2H copy of the 205 recovery slices are
           inside the timed region
-  roofline  the multiply-accumulate kernel's integer-issue roofline: 2 LOP3
-          per symbol multiply-accumulate against the LOP3 rate measured on
-          this device, plus its HBM side
+  roofline  the multiply-accumulate kernel's roofline: on the tensor cores 60
+          4-bit multiply-adds per symbol multiply-accumulate against their
+          rate, with lookup tables 2 LOP3 against the LOP3 rate measured on
+          this device; plus its HBM side
   cpu_baseline  the reference's CPU strategy (par2-rs AVX2-Shuffle restated
           in C, all host threads) on the whole set, its recovery slices
           compared with the GPU's byte for byte (gpu_matches_full)
@@ -69,6 +70,15 @@ def peaks():
         d = json.load(open(path))
         return d.get("hbm_gbs", 6650.0), "measured"
     return 6650.0, "fallback"
+
+
+# flops of the tensor-core form per symbol multiply-accumulate: 60 products of bits
+TENSOR_FLOPS = 120.0
+
+
+def tensor_peak(sms):
+    """4-bit multiply-adds of the device's tensor cores, as flops per second."""
+    return 2 * 16384 * (sms or 148) * 1.965e9
 
 
 def probe_int_peak(device):
@@ -315,23 +325,39 @@ def run_ours(args, rank, world):
     macs = k * r * (S // 2)
     int_ops = 2.0 * macs
     alg_bytes = (k + r) * S
-    # the heuristic plan takes the paired form above 104 outputs
-    paired = (plan["tile_symbols"] == 512) if plan else r > 104
-    roofline = {
-        "bound": "int",
-        "kernel": "muladd_paired" if paired else "muladd_bitsliced",
-        "achieved": int_ops / t_kernel / 1e12,
-        "peak": (int_peak or 0) / 1e12,
-        "unit": "Tops/s (2 LOP3 per GF(2^16) symbol MAC)",
-        "frac": (int_ops / t_kernel) / int_peak if int_peak else None,
-        "peak_source": f"LOP3 issue rate measured on this device ({sms} SMs)",
+    # the form that the plan names (without one: the tensor cores, but for problems
+    # of a few outputs)
+    tile = plan["tile_symbols"] if plan else 256 if r > 8 else 1024
+    if tile == 256:
+        roofline = {
+            "bound": "tensor",
+            "kernel": "tensor_muladd",
+            "achieved": TENSOR_FLOPS * macs / t_kernel / 1e12,
+            "peak": tensor_peak(sms) / 1e12,
+            "unit": "Tflop/s (60 4-bit multiply-adds per GF(2^16) symbol MAC)",
+            "frac": TENSOR_FLOPS * macs / t_kernel / tensor_peak(sms),
+            "peak_source": f"16384 multiply-adds per clock and SM at 1965 MHz ({sms} SMs)",
+            # what the lookup tables' bound would make of the same work
+            "lop3_ratio": (int_ops / t_kernel) / int_peak if int_peak else None,
+        }
+    else:
+        roofline = {
+            "bound": "int",
+            "kernel": "muladd_paired" if tile == 512 else "muladd_bitsliced",
+            "achieved": int_ops / t_kernel / 1e12,
+            "peak": (int_peak or 0) / 1e12,
+            "unit": "Tops/s (2 LOP3 per GF(2^16) symbol MAC)",
+            "frac": (int_ops / t_kernel) / int_peak if int_peak else None,
+            "peak_source": f"LOP3 issue rate measured on this device ({sms} SMs)",
+        }
+    roofline.update({
         "kernel_ms": t_kernel * 1e3,
         "alg_bytes": alg_bytes,
         "hbm": {"achieved": alg_bytes / t_kernel / 1e9, "peak": hbm_peak, "unit": "GB/s",
                 "frac": alg_bytes / t_kernel / 1e9 / hbm_peak, "peak_source": peak_kind},
         # ncu DRAM bytes per launch, profiled for the large-encode shape only
         "traffic": traffic_from_profile() if WORKLOAD == WORKLOADS["large_encode"][3] else None,
-    }
+    })
 
     # ---- CPU baseline + bit-exact cross-check of the whole recovery output ----
     cpu = None
@@ -601,12 +627,12 @@ def verify_repair_leg(autotune=True):
     tot, ker = timed(lambda: ctx.repair(k, S, dmg, present, exps, rptr,
                                         [fbase + j * S for j in range(m)], device=True))
     torch.cuda.synchronize(dev)
-    int_peak, _ = probe_int_peak(0)
+    _, sms = probe_int_peak(0)
     macs = m * k * (S // 2)
     out["repair"] = {"ms": tot, "last_muladd_kernel_ms": ker,
                      "source_gbs": k * S / tot / 1e6,
                      "bit_exact": bool(torch.equal(fixed, pristine)),
-                     "int_roofline_frac": (2.0 * macs / (tot * 1e-3)) / int_peak if int_peak else None}
+                     "tensor_roofline_frac": TENSOR_FLOPS * macs / (tot * 1e-3) / tensor_peak(sms)}
     ctx.close()
     del src, rec, fixed, pristine
     torch.cuda.empty_cache()
@@ -1041,13 +1067,12 @@ def batched_leg():
     out["graph_replay"] = {"makespan_ms": ms, "jobs_per_s": len(sets) / (ms * 1e-3),
                            "note": "decode matrices precomputed; device work only"}
     # the multiply-accumulate work of all sets (create: k x r, repair: one
-    # pass of k sources x m outputs) against the LOP3 roofline, per arm
+    # pass of k sources x m outputs) against the tensor cores' rate, per arm
     macs = sum(x["k"] * (x["r"] if x["create"] else x["m"]) * (x["S"] // 2) for x in sets)
-    int_peak, _ = probe_int_peak(0)
+    _, sms = probe_int_peak(0)
     out["symbol_macs"] = macs
     for name in ("plain", "batched", "graph_replay"):
-        if int_peak:
-            out[name]["int_frac"] = 2.0 * macs / (out[name]["makespan_ms"] * 1e-3) / int_peak
+        out[name]["tensor_frac"] = TENSOR_FLOPS * macs / (out[name]["makespan_ms"] * 1e-3) / tensor_peak(sms)
     for b in graphs:
         b.close()
     same = all(torch.equal(x["out_plain"], x["out_batch"]) for x in sets)
