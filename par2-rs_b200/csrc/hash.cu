@@ -389,6 +389,31 @@ int hash_run(p2g_ctx *ctx, const uint8_t *const *d_slices, int n, size_t S, uint
     return P2G_OK;
 }
 
+// Bound by its launch: 36 bytes read and one written a slice.
+__global__ void __launch_bounds__(256)
+    hash_compare_kernel(const uint4 *__restrict__ md5, const uint32_t *__restrict__ crc,
+                        const uint4 *__restrict__ want_md5, const uint32_t *__restrict__ want_crc, int n,
+                        uint8_t *__restrict__ ok)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n)
+        return;
+    const uint4 a = md5[i], b = want_md5[i];
+    ok[i] = crc[i] == want_crc[i] && a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
+}
+
+int hash_compare(cudaStream_t st, const uint8_t *d_md5, const uint32_t *d_crc, const uint8_t *d_want_md5,
+                 const uint32_t *d_want_crc, int n, uint8_t *d_ok)
+{
+    if (n <= 0)
+        return P2G_OK;
+    hash_compare_kernel<<<(n + 255) / 256, 256, 0, st>>>(reinterpret_cast<const uint4 *>(d_md5), d_crc,
+                                                         reinterpret_cast<const uint4 *>(d_want_md5), d_want_crc,
+                                                         n, d_ok);
+    P2G_CUDA(cudaGetLastError());
+    return P2G_OK;
+}
+
 // A group's time is its slices' chain of MD5 blocks whatever else runs, as long
 // as an SM holds no more than about one team per scheduler: four to a CTA, so
 // that the launch leaves the other SMs to the work it runs beside.

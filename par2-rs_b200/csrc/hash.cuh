@@ -13,7 +13,12 @@ size_t hash_smem_bytes();
 int hash_run(p2g_ctx *ctx, const uint8_t *const *d_slices, int n, size_t S, uint8_t *d_md5,
              uint32_t *d_crc);
 
-// Up to 32 slices of one size, hashed by one warp; results at md5 (16-byte
+// ok[i] = 1 where both checksums of slice i are the expected ones, else 0 (md5
+// and want_md5 16-byte aligned).
+int hash_compare(cudaStream_t st, const uint8_t *d_md5, const uint32_t *d_crc, const uint8_t *d_want_md5,
+                 const uint32_t *d_want_crc, int n, uint8_t *d_ok);
+
+// Up to 32 slices of one size, hashed by one team; results at md5 (16-byte
 // aligned, 16 bytes a slice) and crc.
 struct HashWarp {
     const uint8_t *const *slices;

@@ -59,3 +59,20 @@ def test_groups_in_a_batch(ctx):
             assert np.array_equal(res["md5"], want_md5)
             assert np.array_equal(res["crc"], want_crc)
     b.close()
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 1000])
+def test_verdicts(ctx, n):
+    """One wrong bit of an expected checksum is one damaged slice."""
+    S = 70
+    rng = np.random.default_rng(n)
+    a = rng.integers(0, 256, (n, S), dtype=np.uint8)
+    md5, crc = expect(a)
+    bad = np.unique(np.concatenate([[0, n - 1], rng.integers(0, n, 5)]))
+    for t, i in enumerate(bad):
+        if t % 2:
+            crc[i] ^= np.uint32(1 << int(rng.integers(0, 32)))
+        else:
+            md5[i, rng.integers(0, 16)] ^= np.uint8(1 << int(rng.integers(0, 8)))
+    got = ctx.verify_slices([a[i] for i in range(n)], S, md5, crc)
+    assert np.array_equal(np.flatnonzero(~got), bad)
