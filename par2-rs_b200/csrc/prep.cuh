@@ -47,7 +47,7 @@ inline OutputPrep output_prep(uint8_t *const *dst, int n, size_t S, bool zero, c
 // that others do.  (Neither does anything in launches that are not so linked.)
 // What it hides: the launch's latency and the tensor kernel's setup of tensor
 // memory, 2-5 us a call (20 x 4 KiB, 2 outputs 28.1 -> 26.0 us; 256 x 64 KiB,
-// 13 outputs 70.9 -> 67.3; 777 x 150016, 61 outputs 265 -> 260).
+// 13 outputs 70.9 -> 67.3; 777 x 150002, 61 outputs 265 -> 260).
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
