@@ -190,7 +190,8 @@ int p2g_par2_constants(size_t k, uint16_t *out);
  * + StreamingEncoder::{process_block, flush_batch, finalize}
  * (par2_rs.rs:687-902): out[e] = sum_i c_i^{exps[e]} * src[i] for k input
  * slices of slice_bytes (the caller zero-pads the last slice of a file, as
- * creator.rs:386-395 does).  out receives r recovery slice bodies. */
+ * creator.rs:386-395 does).  out receives r recovery slice bodies.  Device
+ * outputs may overlap the sources: all of them are read before one is written. */
 int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_bytes,
                const uint32_t *exps, size_t r, uint8_t *const *out, uint32_t flags);
 

@@ -12,6 +12,7 @@
 #include "hash.cuh"
 #include "invert.cuh"
 #include "muladd.cuh"
+#include "overlap.hpp"
 
 namespace p2g {
 
@@ -276,7 +277,7 @@ static int matrix_muladd(p2g_ctx *ctx, const std::vector<uint8_t *> &src,
     memcpy(h + L.a_off, coeff, nin * nout * 2);
     P2G_TRY(upload_params(ctx, L));
     uint8_t *d = ctx->params.as<uint8_t>();
-    MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes);
+    MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes, slices_overlap(src, dst, bytes));
     P2G_TRY(mulop_matrix(op, ctx->recs, reinterpret_cast<const uint16_t *>(d + L.a_off)));
     P2G_TRY(mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(d + L.src_off), 0,
                       static_cast<int>(nin), reinterpret_cast<uint8_t *const *>(d + L.dst_off), bytes, mode));
@@ -621,7 +622,7 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
     // blocks CTAs) about fills the device, so none leaves SMs idle.
     const size_t tiles = (slice_bytes + 2047) / 2048;
     int slabs = 1;
-    MulOp op = mulop(ctx, static_cast<int>(k), static_cast<int>(r), slice_bytes);
+    MulOp op = mulop(ctx, static_cast<int>(k), static_cast<int>(r), slice_bytes, slices_overlap(s, d, slice_bytes));
     if (groups >= 4 && d_staged) {
         const p2g::MuladdPlan tp =
             op.plan.tensor ? op.plan
@@ -813,7 +814,7 @@ int p2g_mul_slice(p2g_ctx *ctx, uint16_t c, uint16_t *data, size_t n, uint32_t f
     std::vector<uint8_t *> s;
     bool staged = false;
     P2G_TRY(stage(ctx, ctx->in_copy, &in, 1, bytes, dev, true, s, staged));
-    // in place: the planes are taken before the product is stored
+    // in place: the slice is taken before the product is stored (MulOp::in_place)
     P2G_TRY(matrix_muladd(ctx, s, s, &c, bytes, 0));
     if (staged) {
         uint8_t *user = reinterpret_cast<uint8_t *>(data);

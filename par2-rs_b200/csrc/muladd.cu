@@ -1075,8 +1075,11 @@ static int tables_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_
     uint32_t *planes = ctx->planes.as<uint32_t>();
     const size_t groups = static_cast<size_t>(nin) * T * 32;
     const size_t recs = op && op->pending ? static_cast<size_t>(op->nin) * nout : 0;
-    const OutputPrep z = output_prep(d_dst, nout, S, p.nsplit > 1 && mode == 0, op ? op->status : nullptr,
-                                     op ? op->alt : nullptr);
+    // the preparing launch's blocks run in any order: outputs that overlap inputs
+    // are zeroed in a launch of their own, after the inputs' planes are taken
+    const bool zero = p.nsplit > 1 && mode == 0, apart = zero && op && op->in_place;
+    const OutputPrep z =
+        output_prep(d_dst, nout, S, zero && !apart, op ? op->status : nullptr, op ? op->alt : nullptr);
     const unsigned rec_blocks = static_cast<unsigned>((recs + 255) / 256),
                    plane_blocks = static_cast<unsigned>((groups + 255) / 256);
     ctx->mark(1);
@@ -1086,8 +1089,12 @@ static int tables_run(p2g_ctx *ctx, const uint8_t *const *d_src, int nin, uint8_
         z);
     P2G_CUDA(cudaGetLastError());
     ++ctx->launches;
+    if (apart) {
+        P2G_TRY(launch_zero(ctx->stream, d_dst, nout, S));
+        ++ctx->launches;
+    }
     ctx->mark(2);
-    P2G_TRY(launch_kernel(ctx->stream, p, planes, d_recs, nin, nout, T, d_dst, S, mode, true));
+    P2G_TRY(launch_kernel(ctx->stream, p, planes, d_recs, nin, nout, T, d_dst, S, mode, !apart));
     ++ctx->launches;
     ctx->mark(3);
     return P2G_OK;
@@ -1141,12 +1148,17 @@ static bool tensor_better(const p2g_ctx *ctx, const MuladdPlan &table, int nin, 
     return 1.12 * tensor_clocks(sms, nin, nout, S, &split) < table_clocks(ctx, table, nin, nout, S);
 }
 
-MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S)
+MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S, bool in_place)
 {
     MulOp op;
     op.nin = nin;
     op.nout = nout;
     op.S = S;
+    op.in_place = in_place;
+    if (in_place) {
+        op.plan = choose_plan(ctx, nin, nout, S);
+        return op;
+    }
     if (ctx) {
         auto it = ctx->plans.find(plan_key(nin, nout, S));
         if (it != ctx->plans.end()) {

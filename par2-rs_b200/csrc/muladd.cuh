@@ -157,10 +157,15 @@ struct MulOp {
     // to the slices of the device array `alt` (a run with at least one input)
     const int *status = nullptr;
     uint8_t *const *alt = nullptr;
+    bool in_place = false;  // some output overlaps some input
 };
 // Chooses the plan of an nin x nout problem over slices of S bytes (the
 // context's own plan for that shape if it has one, else by the sizes).
-MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S);
+// in_place: an output may overlap an input.  Such a problem always runs on the
+// lookup tables, which take every input whole before anything is written: the
+// tensor cores would take the inputs of a large problem in column chunks, between
+// which outputs are written.
+MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S, bool in_place = false);
 // The coefficients, which go into buf (grown as needed): a device matrix
 // [nout][nin], or consts[i]^exps[o] (the PAR2 encoding matrix,
 // par2_rs.rs:707-719).  The first mulop_run writes them, in the launch that

@@ -1,0 +1,72 @@
+// overlap.hpp -- whether a call's slices overlap others in memory (host only).
+#pragma once
+#include <stddef.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <utility>
+#include <vector>
+
+namespace p2g {
+
+// A set of byte ranges to ask others against.  Slices that lie wholly before or
+// after the set, the usual case, cost two comparisons each; the ranges are sorted
+// and joined only when one does not.
+class ByteRanges {
+  public:
+    void add(const void *p, size_t n)
+    {
+        if (n == 0)
+            return;
+        const uintptr_t b = reinterpret_cast<uintptr_t>(p);
+        r_.push_back({b, b + n});
+        lo_ = std::min(lo_, b);
+        hi_ = std::max(hi_, b + n);
+        joined_ = false;
+    }
+    // Whether [p, p + n) has a byte in common with the set.
+    bool overlaps(const void *p, size_t n)
+    {
+        const uintptr_t b = reinterpret_cast<uintptr_t>(p), e = b + n;
+        if (n == 0 || b >= hi_ || e <= lo_)
+            return false;
+        if (!joined_)
+            join();
+        // the last range that starts before e
+        auto it = std::lower_bound(r_.begin(), r_.end(), std::make_pair(e, uintptr_t(0)));
+        return it != r_.begin() && std::prev(it)->second > b;
+    }
+
+  private:
+    void join()
+    {
+        std::sort(r_.begin(), r_.end());
+        size_t n = 0;
+        for (const auto &x : r_) {
+            if (n && x.first <= r_[n - 1].second)
+                r_[n - 1].second = std::max(r_[n - 1].second, x.second);
+            else
+                r_[n++] = x;
+        }
+        r_.resize(n);
+        joined_ = true;
+    }
+    std::vector<std::pair<uintptr_t, uintptr_t>> r_;
+    uintptr_t lo_ = UINTPTR_MAX, hi_ = 0;
+    bool joined_ = true;
+};
+
+// Whether any of the slices a overlaps any of the slices b, all of n bytes.
+template <class A, class B>
+inline bool slices_overlap(const A &a, const B &b, size_t n)
+{
+    ByteRanges r;
+    for (const auto *p : b)
+        r.add(p, n);
+    for (const auto *p : a)
+        if (r.overlaps(p, n))
+            return true;
+    return false;
+}
+
+}  // namespace p2g
