@@ -235,13 +235,15 @@ int p2g_verify_slices(p2g_ctx *ctx, const uint8_t *const *slices, size_t n, size
                       const uint8_t *md5_expect, const uint32_t *crc_expect, uint8_t *ok_out,
                       uint32_t flags);
 
-/* ---- batches of independent jobs ---------------------------------------
+/* ---- batches of jobs ---------------------------------------------------
  * Many recovery sets of uneven sizes in one execution: per phase ONE
  * persistent kernel takes (job, column tile, output block, input split)
  * items, longest first, from a device queue -- instead of per-set launches
  * that leave most SMs idle for small sets.  No counterpart in par2-rs (it
  * handles one set per process); the per-job work is that of p2g_encode,
- * p2g_repair and p2g_verify_slices. */
+ * p2g_repair and p2g_verify_slices.  CREATE and REPAIR jobs are independent: none
+ * may read or write another's outputs.  A VERIFY job may take slices that other
+ * jobs of the batch write, and gets the checksums of what they wrote. */
 #define P2G_JOB_CREATE 1
 #define P2G_JOB_REPAIR 2
 #define P2G_JOB_VERIFY 3

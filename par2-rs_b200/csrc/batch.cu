@@ -8,8 +8,9 @@
 //   phase A: CREATE jobs (sources -> recovery slices) and the first REPAIR
 //            pass (RHS = recovery ^ V * present, into scratch);
 //   phase B: the second REPAIR pass (missing = A^-1 * RHS).
-// VERIFY jobs are hashed by one launch beside them.  The device work can be
-// captured once into a CUDA graph and replayed.
+// VERIFY jobs are hashed by one launch beside them; slices that other jobs of the
+// batch write, by one after them.  The device work can be captured once into a
+// CUDA graph and replayed.
 #include <string.h>
 
 #include <algorithm>
@@ -21,6 +22,7 @@
 #include "hash.cuh"
 #include "invert.cuh"
 #include "muladd.cuh"
+#include "overlap.hpp"
 
 using namespace p2g;
 
@@ -45,6 +47,7 @@ struct Image {
 struct HashGroup {
     size_t ptr_off;  // device table of slice pointers
     size_t S;
+    bool after;      // slices that the batch's other jobs write: hashed after both phases
     int n;
     size_t out_off;  // into hash buffer: md5 (n*16), then crc (n*4)
     std::vector<std::pair<int, int>> slices;  // (job, slice index) of each entry
@@ -73,7 +76,7 @@ struct p2g_batch {
     int ncopy = 0;
     std::vector<HashGroup> hash;
     size_t hash_warps_off = 0;  // the groups cut into warps' shares (HashWarp)
-    int nhash_warps = 0;
+    int nhash_beside = 0, nhash_after = 0;  // of them, in this order
     size_t hash_bytes = 0;  // MD5 + CRC results of all groups
     DevBuf hash_host;  // pinned
     DevBuf abort_buf;  // device word the persistent kernels poll (p2g_batch_cancel)
@@ -201,8 +204,16 @@ int enqueue(p2g_batch *b)
                        reinterpret_cast<uint8_t *const *>(dp(b, b->copy_dst_off)),
                        reinterpret_cast<const unsigned long long *>(dp(b, b->copy_len_off)),
                        b->ncopy));
-    if (!b->nhash_warps)
-        return enqueue_phases(b);
+    const HashWarp *hash = reinterpret_cast<const HashWarp *>(dp(b, b->hash_warps_off));
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    // slices that the phases write are hashed as they are then
+    auto phases = [&]() -> int {
+        P2G_TRY(enqueue_phases(b));
+        ctx->launches += b->nhash_after > 0;
+        return hash_groups(st, sms, ctx->d_crc, hash + b->nhash_beside, b->nhash_after);
+    };
+    if (!b->nhash_beside)
+        return phases();
     // Verification is bound by the serial chains of its slices, not by the SMs
     // it uses: all sizes in one launch on a stream of its own, beside the rest.
     // (48 uneven sets, nine of them verified: 8.45 ms with one launch per size
@@ -210,11 +221,10 @@ int enqueue(p2g_batch *b)
     // after a failure: a capture must not end with one of them left open.
     P2G_CUDA(cudaEventRecord(ctx->fork_ev, st));
     P2G_CUDA(cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0));
-    int rc = hash_groups(ctx->side_stream, ctx->sm_count > 0 ? ctx->sm_count : 148, ctx->d_crc,
-                         reinterpret_cast<const HashWarp *>(dp(b, b->hash_warps_off)), b->nhash_warps);
+    int rc = hash_groups(ctx->side_stream, sms, ctx->d_crc, hash, b->nhash_beside);
     ++ctx->launches;
     if (rc == P2G_OK)
-        rc = enqueue_phases(b);
+        rc = phases();
     P2G_CUDA(cudaEventRecord(ctx->join_ev, ctx->side_stream));
     P2G_CUDA(cudaStreamWaitEvent(st, ctx->join_ev, 0));
     return rc;
@@ -641,23 +651,35 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
     if (int rc = take(ctx, b->rhs, rhs_bytes + 256))
         return fail(rc);
     std::vector<HashGroup> hg;
+    auto hash_group = [&](size_t S, bool after) {
+        size_t g = 0;
+        while (g < hg.size() && (hg[g].S != S || hg[g].after != after))
+            ++g;
+        if (g == hg.size()) {
+            hg.push_back(HashGroup());
+            hg[g].S = S;
+            hg[g].after = after;
+        }
+        return g;
+    };
+    ByteRanges written;  // by the CREATE and REPAIR jobs
+    for (size_t j = 0; j < njobs; ++j) {
+        const p2g_job &J = jobs[j];
+        for (size_t e = 0; J.kind != P2G_JOB_VERIFY && e < J.n; ++e)
+            written.add(J.out[e] + J.col_begin, (J.col_end ? J.col_end : J.slice_bytes) - J.col_begin);
+    }
     for (size_t j = 0; j < njobs; ++j) {
         p2g_job &J = jobs[j];
         const size_t cb = J.col_begin;
         const size_t S = (J.col_end ? J.col_end : J.slice_bytes) - cb;
         if (J.kind == P2G_JOB_VERIFY) {
-            HashGroup *g = nullptr;
-            for (HashGroup &x : hg)
-                if (x.S == S)
-                    g = &x;
-            if (!g) {
-                hg.push_back(HashGroup());
-                g = &hg.back();
-                g->S = S;
-                g->n = 0;
+            size_t g = 0;
+            for (size_t i = 0; i < J.k; ++i) {
+                const bool after = written.overlaps(J.src[i], S);
+                if (i == 0 || hg[g].after != after)
+                    g = hash_group(S, after);
+                hg[g].slices.push_back({static_cast<int>(j), static_cast<int>(i)});
             }
-            for (size_t i = 0; i < J.k; ++i)
-                g->slices.push_back({static_cast<int>(j), static_cast<int>(i)});
             continue;
         }
         if (J.kind == P2G_JOB_CREATE) {
@@ -973,9 +995,11 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         D.zero_ptr_off = img.put(ph[x].zptr.data(), ph[x].zptr.size() * sizeof(void *));
         D.zero_len_off = img.put(ph[x].zlen.data(), ph[x].zlen.size() * 8);
     }
-    std::stable_sort(hg.begin(), hg.end(), [](const HashGroup &l, const HashGroup &r) { return l.S > r.S; });
+    std::stable_sort(hg.begin(), hg.end(), [](const HashGroup &l, const HashGroup &r) {
+        return l.after != r.after ? r.after : l.S > r.S;
+    });
     size_t hbytes = 0;
-    int hwarps = 0;
+    int hwarps[2] = {0, 0};  // beside, after
     for (HashGroup &g : hg) {
         g.n = static_cast<int>(g.slices.size());
         std::vector<const uint8_t *> ptrs(g.n);
@@ -984,11 +1008,12 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         g.ptr_off = img.put(ptrs.data(), ptrs.size() * sizeof(void *));
         g.out_off = hbytes;
         hbytes += al256(al16(static_cast<size_t>(g.n) * 16) + static_cast<size_t>(g.n) * 4);
-        hwarps += (g.n + 31) / 32;
+        hwarps[g.after] += (g.n + 31) / 32;
     }
-    b->hash_warps_off = img.put(nullptr, hwarps * sizeof(HashWarp));
-    b->nhash_warps = hwarps;
-    if (hwarps)
+    b->hash_warps_off = img.put(nullptr, (hwarps[0] + hwarps[1]) * sizeof(HashWarp));
+    b->nhash_beside = hwarps[0];
+    b->nhash_after = hwarps[1];
+    if (hwarps[0])
         if (int rc = ensure_side(ctx))
             return fail(rc);
     if (int rc = take(ctx, b->hashbuf, hbytes + 256))
