@@ -81,6 +81,14 @@ typedef struct {
 int p2g_set_timing(p2g_ctx *ctx, int enable);
 int p2g_last_timing(p2g_ctx *ctx, p2g_timing *out);
 
+/* How many of a thread's waits on the device may fail their try, over one kernel,
+ * before the kernel gives up (its copies and products end first) and the call
+ * returns P2G_ETIMEOUT, its outputs unspecified; later calls are not affected.
+ * Only the tensor-core kernel waits, for its own CTA's work.  0 restores the
+ * default of 4000000 (2 us each; a healthy kernel needs some thousand).  Applies
+ * to the context's later calls and batches.  No counterpart in par2-rs. */
+int p2g_set_wait_limit(p2g_ctx *ctx, uint32_t tries);
+
 /* Tile shape of the multiply-accumulate kernel for one problem shape:
  * warps per CTA; warps_per_group warps share one group of outputs_per_group
  * outputs (each holding 16 / warps_per_group of the 16 bit planes); output

@@ -870,6 +870,7 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
                 a.nout = p.nout;
                 a.mode = p.mode;
                 a.err = ctx->wait_err;
+                a.tries = ctx->wait_tries;
                 // parts: items of at most half of an SM's share of the phase
                 a.split = 1;
                 const double share = total_clocks / (2.0 * sms);

@@ -571,6 +571,18 @@ int p2g_set_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes,
     return P2G_OK;
 }
 
+int p2g_set_wait_limit(p2g_ctx *ctx, uint32_t tries)
+{
+    clear_error();
+    if (!ctx) {
+        set_error("p2g_set_wait_limit: null context");
+        return P2G_EINVAL;
+    }
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    ctx->wait_tries = tries ? tries : kWaitTries;
+    return P2G_OK;
+}
+
 int p2g_par2_constants(size_t k, uint16_t *out)
 {
     clear_error();

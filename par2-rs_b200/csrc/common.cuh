@@ -49,6 +49,12 @@ struct MuladdPlan {
     bool tensor = false; // tensor-core products (ereg: rows per block, nblk and nsplit apply)
 };
 
+// Failing tries that a thread of a tensor CTA may make over all its waits.  A try
+// suspends it for about 2 us, so that a stuck CTA gives up after 8 s; the waits of a
+// healthy one (8 ms in all for 32000 inputs and 208 outputs) are at most some
+// thousand tries.
+constexpr uint32_t kWaitTries = 4000000;
+
 using PlanKey = std::tuple<int, int, size_t>;  // inputs, outputs, slice bytes
 
 // Device mirrors and recorded products of the shuffle2x hooks (deferred.cu).
@@ -100,6 +106,7 @@ struct p2g_ctx {
     }
     // pinned host word that a kernel sets when a bounded wait gave up
     int *wait_err = nullptr;
+    uint32_t wait_tries = p2g::kWaitTries;  // p2g_set_wait_limit
     // GF(2^16) log / antilog tables on the device (galois/core.rs:49-91)
     uint16_t *d_log = nullptr;
     uint16_t *d_exp = nullptr;

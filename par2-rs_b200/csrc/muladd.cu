@@ -1254,6 +1254,7 @@ int mulop_run(p2g_ctx *ctx, MulOp &op, const uint8_t *const *d_src, int i0, int 
     r.mode = mode;
     r.split = i0 == 0 && n == op.nin && S == op.S ? op.plan.nsplit : tensor_splits(sms, n, op.nout, S);
     r.err = ctx->wait_err;
+    r.tries = ctx->wait_tries;
     // column chunks: whole waves of tile pairs that fit the scratch; smaller
     // ones when the device has no room for that
     const size_t tiles = tensor_tiles(S), pair = tensor_form_bytes(n, 2);

@@ -127,22 +127,20 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes)
 }
 // Waits for a barrier phase.  The loop is inside the asm block (branches that
 // the compiler sees cost ten to twenty clocks each, also when not taken) and
-// bounded: every phase here ends within a millisecond, and each try suspends
-// the thread for a while, so that the count is reached after a few seconds
-// only.  Returns the tries left: 0 if it gave up, after which a role finishes
-// the step at hand (on stale data, all in bounds), raises the error word and
-// ends.
-__device__ __forceinline__ uint32_t bar_wait(uint32_t bar, uint32_t phase)
+// bounded: `left`, a thread's failing tries, serves all of its waits, so that once
+// it is used up each later wait is one try.  A thread that finds it 0 skips its
+// copies, products and arrivals (what it would announce may not be there).  Its
+// warp then leaves its loops, all lanes together, gives what is in flight time to
+// end, raises the error word and goes where the CTA meets.
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t phase, uint32_t &left)
 {
-    uint32_t left;
-    asm volatile("{\n.reg .pred p, q;\n.reg .u32 n;\nmov.u32 n, 4000000;\n"
+    asm volatile("{\n.reg .pred p, q;\n"
                  "WAIT:\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 "@p bra DONE;\nsub.u32 n, n, 1;\nsetp.ne.u32 q, n, 0;\n@q bra WAIT;\n"
-                 "DONE:\nmov.u32 %0, n;\n}"
-                 : "=r"(left)
+                 "@p bra DONE;\nsetp.ne.u32 q, %0, 0;\n@q sub.u32 %0, %0, 1;\n@q bra WAIT;\n"
+                 "DONE:\n}"
+                 : "+r"(left)
                  : "r"(bar), "r"(phase)
                  : "memory");
-    return left;
 }
 // Whether a phase has completed, without waiting.  Asked for some time before
 // the wait, so that the answer's latency passes behind other work.
@@ -157,25 +155,26 @@ __device__ __forceinline__ uint32_t bar_test(uint32_t bar, uint32_t phase)
     return done;
 }
 // The wait that follows a test: no more than a predicate if it was done.
-__device__ __forceinline__ uint32_t bar_wait(uint32_t bar, uint32_t phase, uint32_t done)
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t phase, uint32_t &left, uint32_t done)
 {
-    uint32_t left;
-    asm volatile("{\n.reg .pred p, q;\n.reg .u32 n;\nmov.u32 n, 4000000;\nsetp.ne.u32 p, %3, 0;\n@p bra DONE;\n"
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\n@p bra DONE;\n"
                  "WAIT:\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 "@p bra DONE;\nsub.u32 n, n, 1;\nsetp.ne.u32 q, n, 0;\n@q bra WAIT;\n"
-                 "DONE:\nmov.u32 %0, n;\n}"
-                 : "=r"(left)
+                 "@p bra DONE;\nsetp.ne.u32 q, %0, 0;\n@q sub.u32 %0, %0, 1;\n@q bra WAIT;\n"
+                 "DONE:\n}"
+                 : "+r"(left)
                  : "r"(bar), "r"(phase), "r"(done)
                  : "memory");
-    return left;
 }
-// After a wait gave up: time for copies and products in flight to end before
-// the CTA gives its memory back.
-__device__ __forceinline__ void let_finish()
+// Whether no lane of the warp has given up.
+__device__ __forceinline__ bool all_left(uint32_t left) { return __all_sync(0xffffffffu, left != 0); }
+// By a role that gave up: 2 ms for copies and products in flight (each takes
+// microseconds) to end before the CTA gives its memory back, and the error word.
+__device__ __forceinline__ void gave_up(int *err)
 {
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000ll) {
     }
+    *static_cast<volatile int *>(err) = 1;
 }
 // global -> shared copy of `bytes` (a multiple of 16, both sides aligned)
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
@@ -552,7 +551,7 @@ __device__ __forceinline__ void issue_products(const TensorArgs &a, const CtaWor
     const uint32_t endA = c.ringA * 8;
     uint32_t offB = 0, offA = 0, pa = 0, pb = 0, pd = 0;
     uint64_t b = desc0;
-    uint32_t left = 1;
+    uint32_t left = a.tries;
     auto advance = [&] {
         b += stepB;
         offB += 8;
@@ -567,17 +566,17 @@ __device__ __forceinline__ void issue_products(const TensorArgs &a, const CtaWor
     };
     uint32_t buf = 0;  // 8 * accumulator set
     for (int e = c.e0; e < c.e1; ++e) {
-        left = min(left, bar_wait(c.smem + empty_d(T, 0) + buf, pd));
+        bar_wait(c.smem + empty_d(T, 0) + buf, pd, left);
         const uint32_t d = d0 + (buf >> 2) * c.N;
         for (int n = 1; n < c.ns; ++n) {
             {
                 const uint32_t db = bar_test(c.smem + full_b(0) + offB, pb);
                 const uint32_t da = bar_test(c.smem + full_a(T, 0) + offA, pa);
-                left = min(left, bar_wait(c.smem + full_b(0) + offB, pb, db));
-                left = min(left, bar_wait(c.smem + full_a(T, 0) + offA, pa, da));
+                bar_wait(c.smem + full_b(0) + offB, pb, left, db);
+                bar_wait(c.smem + full_a(T, 0) + offA, pa, left, da);
             }
             tc_fence_after();
-            if (one) {
+            if (one && left != 0) {
                 const uint32_t col = colA + offA * (kStageCols / 8);
                 tc_mma(d, col, b, idesc, sa, sb);
                 tc_mma(d, col + 8, b + step, idesc, sa, sb);
@@ -589,10 +588,10 @@ __device__ __forceinline__ void issue_products(const TensorArgs &a, const CtaWor
             __syncwarp();
             advance();
         }
-        left = min(left, bar_wait(c.smem + full_b(0) + offB, pb));
-        left = min(left, bar_wait(c.smem + full_a(T, 0) + offA, pa));
+        bar_wait(c.smem + full_b(0) + offB, pb, left);
+        bar_wait(c.smem + full_a(T, 0) + offA, pa, left);
         tc_fence_after();
-        if (one) {
+        if (one && left != 0) {
             const uint32_t col = colA + offA * (kStageCols / 8);
 #pragma unroll 1
             for (int q = 0; q < c.last; ++q)
@@ -605,13 +604,9 @@ __device__ __forceinline__ void issue_products(const TensorArgs &a, const CtaWor
         advance();
         pd ^= buf == static_cast<uint32_t>(c.dbuf) * 8;
         buf ^= c.dbuf * 8;
-        if (left == 0)
-            break;
     }
-    if (left == 0) {
-        let_finish();
-        *a.err = 1;
-    }
+    if (!all_left(left))
+        gave_up(a.err);
 }
 
 // ---- copies of the B stages
@@ -622,12 +617,12 @@ __device__ __forceinline__ void copy_b(const TensorArgs &a, const CtaWork &c)
     const uint32_t last_bytes = c.last * 2 * c.N * 16;
     const uint32_t ring = c.smem + kOffB;
     uint32_t off = 0, ph = 1, dst = ring;
-    uint32_t left = 1;
-    for (int e = c.e0; e < c.e1 && left; ++e) {
+    uint32_t left = a.tries;
+    for (int e = c.e0; e < c.e1; ++e) {
         const uint4 *src = cb + static_cast<size_t>(e) * a.cwords * c.N;
-        for (int n = 0; n < c.ns && left; ++n) {
-            left = bar_wait(c.smem + empty_b(0) + off, ph);
-            if (one) {
+        for (int n = 0; n < c.ns; ++n) {
+            bar_wait(c.smem + empty_b(0) + off, ph, left);
+            if (one && left != 0) {
                 const uint32_t bytes = n == c.ns - 1 ? last_bytes : c.slotB;
                 bar_expect(c.smem + full_b(0) + off, bytes);
                 bulk_copy(dst, src, bytes, c.smem + full_b(0) + off);
@@ -642,10 +637,8 @@ __device__ __forceinline__ void copy_b(const TensorArgs &a, const CtaWork &c)
             ph ^= wrap;
         }
     }
-    if (left == 0) {
-        let_finish();
-        *a.err = 1;
-    }
+    if (!all_left(left))
+        gave_up(a.err);
 }
 
 // ---- copies of the tile pair's form words: a slot holds four stages of one
@@ -655,9 +648,9 @@ __device__ __forceinline__ void copy_forms(const TensorArgs &a, const CtaWork &c
     const bool one = elect_one();
     const uint32_t plane = c.ns * kFormBytes;  // bytes of one form of one pair
     const uint8_t *ft = reinterpret_cast<const uint8_t *>(a.forms) + static_cast<size_t>(c.pair) * kForms * plane;
-    uint32_t off = 0, d = c.smem + kOffF, ph = 1, left = 1;
+    uint32_t off = 0, d = c.smem + kOffF, ph = 1, left = a.tries;
     uint32_t next = c_prod.forms[c.e0];
-    for (int e = c.e0; e < c.e1 && left; ++e) {
+    for (int e = c.e0; e < c.e1; ++e) {
         const uint32_t t = next;
         next = c_prod.forms[min(e + 1, kProds - 1)];
         const uint32_t nf = (t >> 16) & 0xFF, step = (4u >> (nf >> 1)) * kFormBytes;
@@ -665,8 +658,8 @@ __device__ __forceinline__ void copy_forms(const TensorArgs &a, const CtaWork &c
         const uint8_t *f1 = ft + static_cast<size_t>((t >> 8) & 0xFF) * plane;
         for (uint32_t at = 0; at < plane; at += step) {
             const uint32_t bytes = min(step, plane - at);
-            left = min(left, bar_wait(c.smem + empty_f(0) + off, ph));
-            if (one) {
+            bar_wait(c.smem + empty_f(0) + off, ph, left);
+            if (one && left != 0) {
                 const uint32_t bar = c.smem + full_f(0) + off;
                 bar_expect(bar, nf * bytes);
                 bulk_copy(d, f0 + at, bytes, bar);
@@ -687,10 +680,8 @@ __device__ __forceinline__ void copy_forms(const TensorArgs &a, const CtaWork &c
             ph ^= wrap;
         }
     }
-    if (left == 0) {
-        let_finish();
-        *a.err = 1;
-    }
+    if (!all_left(left))
+        gave_up(a.err);
 }
 
 // ---- the A operand of a tile: row = lane of tensor memory = symbol
@@ -707,7 +698,7 @@ __device__ __forceinline__ void generate_product(GenState &g)
 {
     constexpr int kPer = 4 / NF;  // stages per slot
     for (int n = 0; n < g.ns; n += kPer) {
-        g.left = min(g.left, bar_wait(g.fullF + g.sf * 8, g.pf));
+        bar_wait(g.fullF + g.sf * 8, g.pf, g.left);
         const uint32_t F = g.ring + g.sf * kSlotF;
 #pragma unroll
         for (int s = 0; s < kPer; ++s) {
@@ -730,7 +721,7 @@ __device__ __forceinline__ void generate_product(GenState &g)
                     o[2] = w[j] & 0x44444444u;
                     o[3] = (w[j] >> 1) & 0x44444444u;
                 }
-                g.left = min(g.left, bar_wait(g.emptyA + g.offA, g.pa, doneA));
+                bar_wait(g.emptyA + g.offA, g.pa, g.left, doneA);
                 tc_fence_after();
                 const uint32_t col = g.lanes + g.offA * (kStageCols / 8);
 #pragma unroll
@@ -739,7 +730,7 @@ __device__ __forceinline__ void generate_product(GenState &g)
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (g.first)
+                if (g.first && g.left != 0)
                     bar_arrive(g.fullA + g.offA);
                 g.offA += 8;
                 const bool wrapA = g.offA == g.endA;
@@ -747,7 +738,7 @@ __device__ __forceinline__ void generate_product(GenState &g)
                 g.pa ^= wrapA;
             }
         }
-        if (g.first)
+        if (g.first && g.left != 0)
             bar_arrive(g.emptyF + g.sf * 8);
         const bool wrap = ++g.sf == kRingF;
         g.sf = wrap ? 0 : g.sf;
@@ -769,7 +760,7 @@ __device__ __forceinline__ void generate_a(const TensorArgs &a, const CtaWork &c
     g.emptyF = c.smem + empty_f(0);
     g.sf = 0;
     g.pf = 0;
-    g.left = 1;
+    g.left = a.tries;
     g.ns = c.ns;
     g.first = lane == 0;
     uint32_t next = c_prod.forms[c.e0];
@@ -782,10 +773,9 @@ __device__ __forceinline__ void generate_a(const TensorArgs &a, const CtaWork &c
             generate_product<2>(g);
         else
             generate_product<4>(g);
-        if (!__all_sync(0xffffffffu, g.left != 0)) {
-            if (lane == 0)
-                *a.err = 1;
-            break;
+        if (!all_left(g.left)) {
+            gave_up(a.err);
+            return;
         }
     }
 }
@@ -860,7 +850,8 @@ __device__ __forceinline__ void read_products(const TensorArgs &a, const CtaWork
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             acc[q][j] = 0;
-    uint32_t pd = 0, left = 1, buf = 0;
+    uint32_t pd = 0, left = a.tries, buf = 0;
+    bool whole = true;
     int run = 1;  // products since the accumulators of this set were set, this one included
     for (int e = c.e0; e < c.e1; ++e) {
         // parities of sums over all products since then (see the head of this
@@ -868,7 +859,7 @@ __device__ __forceinline__ void read_products(const TensorArgs &a, const CtaWork
         const bool end = run == span || e + nbuf >= c.e1;
         const uint32_t w = (end ? c_prod.w[e] : c_prod.w[e] ^ c_prod.w[e + nbuf]) * 0x10001u;
         const uint32_t col = d + (buf >> 2) * c.N;
-        left = min(left, bar_wait(c.smem + full_d(t, 0) + buf, pd));
+        bar_wait(c.smem + full_d(t, 0) + buf, pd, left);
         tc_fence_after();
 #pragma unroll
         for (int q0 = 0; q0 < G; q0 += kBatch) {
@@ -900,10 +891,11 @@ __device__ __forceinline__ void read_products(const TensorArgs &a, const CtaWork
             run = run == span ? 1 : run + 1;
         }
         buf ^= c.dbuf * 8;
-        if (!__all_sync(0xffffffffu, left != 0)) {
-            if (lane == 0)
-                *a.err = 1;
-            return;
+        if (!all_left(left)) {
+            // stores nothing more, but still meets the others below
+            gave_up(a.err);
+            whole = false;
+            break;
         }
     }
     // The sums go through shared memory (the form ring is idle once both tiles'
@@ -915,6 +907,7 @@ __device__ __forceinline__ void read_products(const TensorArgs &a, const CtaWork
     const int per = (a.nout + a.nblk - 1) / a.nblk;
     const int nrows = min(per, a.nout - c.nb * per);
     const size_t off = a.byte0 + (static_cast<size_t>(2 * c.pair + t) * kTensorM + lane * 4) * 2;
+    const size_t end = whole ? a.S : 0;
     const int mode = a.split > 1 ? 2 : a.mode;
     constexpr int kHalf = 4;  // column groups per exchange
     static_assert(kHalf * 8 * kTensorM * 4 <= kRingF * kSlotF / 4, "exchange fits a quarter of the form ring");
@@ -936,7 +929,7 @@ __device__ __forceinline__ void read_products(const TensorArgs &a, const CtaWork
 #pragma unroll 1
             for (int hi = 0; hi < 2; ++hi) {
                 const int o = col0 + (q0 * 8 + p) * 2 + hi;
-                if (o >= nrows || off >= a.S)
+                if (o >= nrows || off >= end)
                     continue;
                 const uint32_t sel = hi ? 0x7632u : 0x5410u;
                 store_symbols(a.dst[c.nb * per + o] + off, a.S - off,
@@ -1222,6 +1215,7 @@ int tensor_products(cudaStream_t st, const TensorRun &r, size_t t0, size_t n)
     a.mode = r.mode;
     a.split = std::max(1, std::min(r.split, kProds));
     a.err = r.err;
+    a.tries = r.tries;
     const long long grid = static_cast<long long>((n + 1) / 2) * nblk * a.split;
     if (grid > 0x7fffffffLL) {
         set_error("tensor multiply-accumulate: grid too large");

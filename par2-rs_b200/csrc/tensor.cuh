@@ -52,6 +52,7 @@ struct TensorRun {
     int mode;     // 0 stores, 1 XORs
     int split;    // parts of the work; above 1 they are XORed atomically into dst
     int *err;     // device-visible word, set when a bounded wait gave up
+    uint32_t tries;  // of a thread's waits (kWaitTries)
 };
 inline size_t tensor_tiles(size_t S) { return (S / 2 + kTensorM - 1) / kTensorM; }
 // The forms of tiles [t0, t0 + n), the coefficient operand (r.coef, of the whole
@@ -76,6 +77,7 @@ struct TensorArgs {
     int rows, nblk, nout, mode;
     int split;  // parts of the 60 products (above 1: partial results are XORed atomically)
     int *err;
+    uint32_t tries;
 };
 // One CTA's work: a tile pair, an output block and a part of the products.
 struct TensorItem {

@@ -44,6 +44,7 @@ SIGNATURES = [
     ("p2g_set_timing", _I, [_P, _I]),
     ("p2g_last_timing", _I, [_P, _P]),
     ("p2g_autotune", _I, [_P, _S, _S, _S, _I, _P]),
+    ("p2g_set_wait_limit", _I, [_P, _U32]),
     ("p2g_set_plan", _I, [_P, _S, _S, _S, _P]),
     ("p2g_strategy_info", _I, [_P, _P, _P]),
     ("p2g_mul_slice", _I, [_P, _U16, _P, _S, _U32]),
@@ -249,6 +250,11 @@ class Context:
         t = Timing()
         check(lib().p2g_last_timing(self.h, ctypes.byref(t)))
         return t
+
+    def set_wait_limit(self, tries=0):
+        """Failing tries of a device thread's waits before a kernel gives up and
+        the call raises Par2GpuError with code ETIMEOUT (0: the default)."""
+        check(lib().p2g_set_wait_limit(self.h, tries))
 
     def autotune(self, nin, nout, slice_bytes, reps=2):
         """Time the kernel's tile shapes for this problem shape and keep the
