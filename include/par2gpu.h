@@ -290,7 +290,10 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags,
                      p2g_batch **out);
 /* Runs (or replays) the batch and waits for it; fills statuses and hashes. */
 int p2g_batch_run(p2g_batch *batch);
-/* Starts the batch without waiting; p2g_batch_wait completes it. */
+/* Starts the batch without waiting; p2g_batch_wait completes it.  A batch whose
+ * kernels gave up on a wait returns P2G_ETIMEOUT from its own p2g_batch_wait, with
+ * the status of its jobs P2G_ETIMEOUT and their outputs unspecified; calls and
+ * other batches of the context do not report it. */
 int p2g_batch_launch(p2g_batch *batch);
 int p2g_batch_poll(p2g_batch *batch, int *done);
 int p2g_batch_wait(p2g_batch *batch);

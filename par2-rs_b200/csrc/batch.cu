@@ -79,6 +79,7 @@ struct p2g_batch {
     int nhash_beside = 0, nhash_after = 0;  // of them, in this order
     size_t hash_bytes = 0;  // MD5 + CRC results of all groups
     DevBuf hash_host;  // pinned
+    int *wait_err = nullptr;  // in hparams, past the tables: set when a wait gave up
     DevBuf abort_buf;  // device word the persistent kernels poll (p2g_batch_cancel)
     int *abort_dev = nullptr;
     std::atomic<bool> cancelled{false};
@@ -869,7 +870,6 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
                 a.nblk = tensor_blocks(p.nout);
                 a.nout = p.nout;
                 a.mode = p.mode;
-                a.err = ctx->wait_err;
                 a.tries = ctx->wait_tries;
                 // parts: items of at most half of an SM's share of the phase
                 a.split = 1;
@@ -1021,6 +1021,10 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         return fail(rc);
     if (int rc = take(ctx, b->params, img.bytes.size() + 256))
         return fail(rc);
+    if (int rc = take(ctx, b->hparams, al256(img.bytes.size()) + 256))
+        return fail(rc);
+    b->wait_err = reinterpret_cast<int *>(b->hparams.as<uint8_t>() + al256(img.bytes.size()));
+    *b->wait_err = 0;
     uint8_t *base = b->params.as<uint8_t>();
     auto rebase = [&](const void *off) { return base + reinterpret_cast<uintptr_t>(off); };
     for (int x = 0; x < 2; ++x) {
@@ -1042,8 +1046,10 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
                 q.consts = reinterpret_cast<const uint16_t *>(rebase(q.consts));
                 q.exps = reinterpret_cast<const uint32_t *>(rebase(q.exps));
             }
-        for (TensorArgs &q : ph[x].tp)
+        for (TensorArgs &q : ph[x].tp) {
             q.dst = reinterpret_cast<uint8_t *const *>(rebase(q.dst));
+            q.err = b->wait_err;
+        }
         auto table = [&](size_t off, const auto &v) {
             if (!v.empty())
                 memcpy(img.bytes.data() + off, v.data(), v.size() * sizeof(v[0]));
@@ -1072,8 +1078,6 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
             return fail(rc);
     b->hash = hg;
     b->hash_bytes = hbytes;
-    if (int rc = take(ctx, b->hparams, img.bytes.size() + 256))
-        return fail(rc);
     memcpy(b->hparams.p, img.bytes.data(), img.bytes.size());
     if (cudaMemcpyAsync(b->params.p, b->hparams.p, img.bytes.size(), cudaMemcpyHostToDevice,
                         ctx->stream) != cudaSuccess ||
@@ -1124,9 +1128,11 @@ int p2g_batch_launch(p2g_batch *b)
         m = false;
     ctx->mark(0);
     b->cancelled = false;
-    for (size_t j = 0; j < b->njobs; ++j)  // a cancelled run's statuses (singular jobs keep theirs)
-        if (b->jobs[j].status == P2G_ECANCELED)
+    for (size_t j = 0; j < b->njobs; ++j)  // an earlier run's statuses (singular jobs keep theirs)
+        if (b->jobs[j].status == P2G_ECANCELED || b->jobs[j].status == P2G_ETIMEOUT)
             b->jobs[j].status = P2G_OK;
+    if (!b->launched)
+        *b->wait_err = 0;
     if (b->exec) {
         P2G_CUDA(cudaGraphLaunch(b->exec, ctx->stream));
         ctx->launches = 1;
@@ -1172,7 +1178,12 @@ int p2g_batch_wait(p2g_batch *b)
     P2G_CUDA(cudaEventSynchronize(b->done));
     P2G_CUDA(cudaGetLastError());
     b->launched = false;
-    P2G_TRY(check_waits(ctx));
+    if (const int rc = check_waits(b->wait_err)) {
+        for (size_t j = 0; j < b->njobs; ++j)
+            if (b->jobs[j].status == P2G_OK)
+                b->jobs[j].status = rc;
+        return rc;
+    }
     if (b->cancelled) {
         for (size_t j = 0; j < b->njobs; ++j)
             b->jobs[j].status = P2G_ECANCELED;

@@ -207,6 +207,7 @@ static void begin(p2g_ctx *ctx)
     ctx->launches = 0;
     for (bool &m : ctx->ev_marked)
         m = false;
+    *ctx->wait_err = 0;
     ctx->mark(0);
 }
 
@@ -221,16 +222,12 @@ static float elapsed(p2g_ctx *ctx, int a, int b)
     return ms;
 }
 
-// After a synchronisation: P2G_ETIMEOUT if a kernel's bounded wait gave up.
-int check_waits(p2g_ctx *ctx)
+int check_waits(const volatile int *word)
 {
-    volatile int *err = ctx->wait_err;
-    if (err && *err) {
-        *err = 0;
-        set_error("a bounded wait on the device gave up");
-        return P2G_ETIMEOUT;
-    }
-    return P2G_OK;
+    if (*word == 0)
+        return P2G_OK;
+    set_error("a bounded wait on the device gave up");
+    return P2G_ETIMEOUT;
 }
 
 int ensure_side(p2g_ctx *ctx)
@@ -249,7 +246,7 @@ static int finish(p2g_ctx *ctx)
     ctx->mark(4);
     P2G_CUDA(cudaStreamSynchronize(ctx->stream));
     P2G_CUDA(cudaGetLastError());
-    P2G_TRY(check_waits(ctx));
+    P2G_TRY(check_waits(ctx->wait_err));
     ctx->last = p2g_timing{};
     ctx->last.launches = ctx->launches;
     if (ctx->timing) {
@@ -520,6 +517,7 @@ int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int 
     MuladdPlan p;
     float ms = 0.f;
     int tried = 0;
+    *ctx->wait_err = 0;
     P2G_TRY(muladd_autotune(ctx, static_cast<int>(nin), static_cast<int>(nout), slice_bytes,
                             reps, &p, &ms, &tried));
     if (p.tensor) {

@@ -104,7 +104,9 @@ struct p2g_ctx {
             ev_marked[idx] = true;
         }
     }
-    // pinned host word that a kernel sets when a bounded wait gave up
+    // pinned host word that a kernel of the running call sets when a bounded wait
+    // gave up (batches and the shuffle2x state, whose kernels outlive a call, have
+    // words of their own)
     int *wait_err = nullptr;
     uint32_t wait_tries = p2g::kWaitTries;  // p2g_set_wait_limit
     // GF(2^16) log / antilog tables on the device (galois/core.rs:49-91)
@@ -139,8 +141,9 @@ struct p2g_ctx {
 namespace p2g {
 // Frees the shuffle2x state (mirrors, staging, pool) of a context.
 void deferred_release(p2g_ctx *ctx);
-// After a synchronisation: P2G_ETIMEOUT if a kernel's bounded wait gave up.
-int check_waits(p2g_ctx *ctx);
+// After a synchronisation: P2G_ETIMEOUT if a kernel's bounded wait gave up and set
+// the word, which whoever queues the kernels clears before it does.
+int check_waits(const volatile int *word);
 // Creates the context's side stream and its events on first use.
 int ensure_side(p2g_ctx *ctx);
 }  // namespace p2g

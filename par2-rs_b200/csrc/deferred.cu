@@ -203,6 +203,10 @@ struct Deferred {
     int par_next = 0;
 
     cudaMemPool_t pool = nullptr;
+
+    // pinned word that a recorded launch sets when a wait gave up: it stays set
+    // until no accumulator is left, since any of them may be wrong
+    int *wait_err = nullptr;
 };
 
 namespace {
@@ -246,6 +250,10 @@ int setup(p2g_ctx *ctx, Deferred *&out)
             cudaEventCreateWithFlags(&d->stage_ev[i], cudaEventDisableTiming) != cudaSuccess)
             rc = P2G_ENOMEM;
     }
+    if (rc == P2G_OK && cudaMallocHost(&d->wait_err, sizeof(int)) != cudaSuccess)
+        rc = P2G_ENOMEM;
+    if (rc == P2G_OK)
+        *d->wait_err = 0;
     for (int i = 0; i < 2 && rc == P2G_OK; ++i) {
         d->hpar[i].pinned = true;
         if (cudaEventCreateWithFlags(&d->par_ev[i], cudaEventDisableTiming) != cudaSuccess)
@@ -419,6 +427,7 @@ int launch_group(p2g_ctx *ctx, Deferred *d, const std::vector<uint8_t *> &srcs,
     P2G_CUDA(cudaMemcpyAsync(dp, h, total, cudaMemcpyHostToDevice, ctx->stream));
     P2G_CUDA(cudaEventRecord(d->par_ev[slot], ctx->stream));
     MulOp op = mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), bytes);
+    op.wait_err = d->wait_err;
     P2G_TRY(mulop_matrix(op, ctx->recs, reinterpret_cast<const uint16_t *>(dp + co)));
     return mulop_run(ctx, op, reinterpret_cast<const uint8_t *const *>(dp + so), 0, static_cast<int>(nin),
                      reinterpret_cast<uint8_t *const *>(dp + dso), bytes, 1);
@@ -665,7 +674,7 @@ int record(p2g_ctx *ctx, uint16_t *const *dsts, size_t ndst, const uint16_t *con
         sp[i] = back[i].data();
     }
     P2G_CUDA(cudaStreamSynchronize(ctx->stream));
-    P2G_TRY(check_waits(ctx));
+    P2G_TRY(check_waits(d->wait_err));
     wlock.unlock();
     lock.unlock();
     std::vector<uint16_t> rows(unprep.size() * nsrc);
@@ -715,6 +724,8 @@ void deferred_release(p2g_ctx *ctx)
     }
     if (d->upload_ev)
         cudaEventDestroy(d->upload_ev);
+    if (d->wait_err)
+        cudaFreeHost(d->wait_err);
     (void)cudaGetLastError();
     delete d;
     ctx->deferred = nullptr;
@@ -819,9 +830,10 @@ int p2g_finish_shuffle2x(p2g_ctx *ctx, uint16_t *data, size_t n)
     P2G_CUDA(cudaMemcpyAsync(data, m.dev, std::min(n * 2, m.bytes), cudaMemcpyDeviceToHost,
                              ctx->stream));
     P2G_CUDA(cudaStreamSynchronize(ctx->stream));
-    P2G_TRY(check_waits(ctx));
+    const int waited = check_waits(d->wait_err);
     P2G_TRY(retire(ctx, d, static_cast<uint32_t>(id)));
     if (d->live_dsts == 0) {
+        *d->wait_err = 0;
         // no accumulator left: the remaining sources' mirrors go too
         std::vector<uint32_t> rest;
         for (const auto &kv : d->by_host)
@@ -829,7 +841,7 @@ int p2g_finish_shuffle2x(p2g_ctx *ctx, uint16_t *data, size_t n)
         for (uint32_t r : rest)
             P2G_TRY(retire(ctx, d, r));
     }
-    return P2G_OK;
+    return waited;
 }
 
 }  // extern "C"

@@ -1253,7 +1253,7 @@ int mulop_run(p2g_ctx *ctx, MulOp &op, const uint8_t *const *d_src, int i0, int 
     r.coef = op.coef;
     r.mode = mode;
     r.split = i0 == 0 && n == op.nin && S == op.S ? op.plan.nsplit : tensor_splits(sms, n, op.nout, S);
-    r.err = ctx->wait_err;
+    r.err = op.wait_err ? op.wait_err : ctx->wait_err;
     r.tries = ctx->wait_tries;
     // column chunks: whole waves of tile pairs that fit the scratch; smaller
     // ones when the device has no room for that
@@ -1514,6 +1514,7 @@ int muladd_autotune(p2g_ctx *ctx, int nin, int nout, size_t S, int reps, MuladdP
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     P2G_TRY(rc);
+    P2G_TRY(check_waits(ctx->wait_err));
     ctx->plans[plan_key(nin, nout, S)] = best_p;
     *best = best_p;
     *best_ms = best_t;

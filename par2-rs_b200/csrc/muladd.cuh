@@ -158,6 +158,7 @@ struct MulOp {
     const int *status = nullptr;
     uint8_t *const *alt = nullptr;
     bool in_place = false;  // some output overlaps some input
+    int *wait_err = nullptr;  // raised when a wait gives up (null: the context's word)
 };
 // Chooses the plan of an nin x nout problem over slices of S bytes (the
 // context's own plan for that shape if it has one, else by the sizes).
