@@ -1137,7 +1137,9 @@ static int repair_unattended(p2g_ctx *ctx, GjWork &w, size_t m, size_t np, size_
     int singular = 0;
     if (rc == P2G_OK) {
         rc = finish(ctx);
-        singular = *ctx->hparams.as<int>();
+        // the status has arrived unless the wait itself failed
+        if (rc == P2G_OK || rc == P2G_ETIMEOUT)
+            singular = *ctx->hparams.as<int>();
     } else {
         // what is queued ends before the call does; a singular matrix is the
         // answer also when a later step failed

@@ -1,0 +1,230 @@
+// Failing CUDA calls, on the host: this program defines the runtime's functions that
+// the library uses (its own definitions come first in the dynamic linker's order),
+// over host memory and without running a kernel, and lets chosen ones fail.  Copies
+// back to the host land when their stream is waited for, as on a device.
+// Usage: test_faults CASE
+#include <cuda_runtime.h>
+#include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
+
+#include <map>
+#include <mutex>
+#include <vector>
+
+#include "../../par2-rs_b200/csrc/common.cuh"
+
+// ---- the runtime -----------------------------------------------------------
+
+namespace {
+std::mutex g_mu;
+std::map<void *, size_t> g_device;  // live device allocations
+size_t g_used = 0, g_room = size_t(1) << 40;
+int g_fail_syncs = 0;  // cudaStreamSynchronize calls that fail from now on
+struct Copy {
+    void *dst;
+    const void *src;
+    size_t n;
+};
+std::vector<Copy> g_pending;
+
+void land()
+{
+    for (const Copy &c : g_pending)
+        memcpy(c.dst, c.src, c.n);
+    g_pending.clear();
+}
+}  // namespace
+
+extern "C" {
+cudaError_t cudaMalloc(void **p, size_t n)
+{
+    std::lock_guard<std::mutex> l(g_mu);
+    if (g_used + n > g_room)
+        return cudaErrorMemoryAllocation;
+    *p = aligned_alloc(256, (n + 255) / 256 * 256);
+    memset(*p, 0, n < 65536 ? n : 65536);  // larger ones are not read by the cases
+    g_device[*p] = n;
+    g_used += n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p)
+{
+    std::lock_guard<std::mutex> l(g_mu);
+    land();
+    g_used -= g_device[p];
+    g_device.erase(p);
+    free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void **p, size_t n)
+{
+    *p = calloc(1, n);
+    return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMallocHost(p, n); }
+cudaError_t cudaFreeHost(void *p)
+{
+    free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t)
+{
+    std::lock_guard<std::mutex> l(g_mu);
+    if (k == cudaMemcpyDeviceToHost)
+        g_pending.push_back({d, s, n});
+    else
+        memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind)
+{
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy2DAsync(void *d, size_t dp, const void *s, size_t sp, size_t w, size_t h, cudaMemcpyKind,
+                              cudaStream_t)
+{
+    for (size_t i = 0; i < h; ++i)
+        memcpy(static_cast<char *>(d) + i * dp, static_cast<const char *>(s) + i * sp, w);
+    return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t)
+{
+    memset(d, v, n);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t)
+{
+    std::lock_guard<std::mutex> l(g_mu);
+    if (g_fail_syncs > 0) {
+        --g_fail_syncs;
+        return cudaErrorUnknown;
+    }
+    land();
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t)
+{
+    std::lock_guard<std::mutex> l(g_mu);
+    land();
+    return cudaSuccess;
+}
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t)
+{
+    *ms = 1.f;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDeviceCount(int *n)
+{
+    *n = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int *d)
+{
+    *d = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp *p, int)
+{
+    memset(p, 0, sizeof *p);
+    p->major = 10;
+    p->multiProcessorCount = 148;
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int)
+{
+    *v = 10;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *, int, size_t, unsigned)
+{
+    *n = 1;
+    return cudaSuccess;
+}
+const char *cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no error" : "injected"; }
+#define OK(name, ...) \
+    cudaError_t name(__VA_ARGS__) { return cudaSuccess; }
+OK(cudaGetLastError, void)
+OK(cudaSetDevice, int)
+OK(cudaStreamDestroy, cudaStream_t)
+OK(cudaStreamWaitEvent, cudaStream_t, cudaEvent_t, unsigned)
+OK(cudaEventDestroy, cudaEvent_t)
+OK(cudaEventRecord, cudaEvent_t, cudaStream_t)
+OK(cudaEventQuery, cudaEvent_t)
+OK(cudaFuncSetAttribute, const void *, cudaFuncAttribute, int)
+OK(cudaLaunchKernel, const void *, dim3, dim3, void **, size_t, cudaStream_t)
+OK(cudaLaunchKernelExC, const cudaLaunchConfig_t *, const void *, void **)
+#undef OK
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned)
+{
+    static char stream;
+    *s = reinterpret_cast<cudaStream_t>(&stream);
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned)
+{
+    static char event;
+    *e = reinterpret_cast<cudaEvent_t>(&event);
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e, 0); }
+}
+
+// ---- the cases -------------------------------------------------------------
+
+#define CHECK(c)                                                                        \
+    do {                                                                                \
+        if (!(c)) {                                                                     \
+            printf("%s:%d: %s (last error: %s)\n", __FILE__, __LINE__, #c, p2g_last_error()); \
+            return 1;                                                                   \
+        }                                                                               \
+    } while (0)
+
+// A "device" buffer of n slices of S bytes and their addresses.
+static std::vector<uint8_t *> slices(size_t n, size_t S)
+{
+    void *p = nullptr;
+    cudaMalloc(&p, n * S);
+    std::vector<uint8_t *> v(n);
+    for (size_t i = 0; i < n; ++i)
+        v[i] = static_cast<uint8_t *>(p) + i * S;
+    return v;
+}
+
+// The last wait of a device repair fails: the call reports that, not a singular
+// matrix read from a word that never arrived.
+static int repair_sync(p2g_ctx *ctx)
+{
+    const size_t k = 60, m = 5, S = 4096;
+    const auto present = slices(k - m, S), rec = slices(m, S), out = slices(m, S);
+    uint64_t missing[m];
+    uint32_t exps[m];
+    for (size_t i = 0; i < m; ++i) {
+        missing[i] = 3 * i;
+        exps[i] = static_cast<uint32_t>(i);
+    }
+    auto repair = [&] {
+        return p2g_repair(ctx, k, S, missing, m, present.data(), exps, rec.data(), out.data(), P2G_DEVICE_PTRS);
+    };
+    CHECK(repair() == P2G_OK);
+    g_fail_syncs = 1;
+    CHECK(repair() == P2G_ECUDA);
+    CHECK(strstr(p2g_last_error(), "cudaStreamSynchronize"));
+    CHECK(repair() == P2G_OK);
+    return 0;
+}
+
+int main(int argc, char **argv)
+{
+    p2g_ctx *ctx = nullptr;
+    CHECK(p2g_create(0, &ctx) == P2G_OK);
+    int rc = 2;
+    if (argc == 2 && !strcmp(argv[1], "repair_sync"))
+        rc = repair_sync(ctx);
+    if (rc == 0) {
+        CHECK(p2g_destroy(ctx) == P2G_OK);
+        printf("ok\n");
+    }
+    return rc;
+}
