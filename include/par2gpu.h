@@ -333,9 +333,9 @@ int p2g_batch_destroy(p2g_batch *batch);
 int p2g_batch_autotune(p2g_ctx *ctx, int reps, int *forms_out, float *ms_out);
 /* Pins the form per class (P2G_BATCH_CLASSES entries; -1, or forms NULL,
  * restores the heuristic: small tables up to 24 outputs, paired above 104,
- * wide between, the tensor cores where they are estimated to be faster; no
- * problem of a context with pinned forms uses the tensor cores).  P2G_EINVAL
- * for the small form on a class above 24 outputs. */
+ * wide between, the tensor cores where they are estimated to be faster; while
+ * any class has a pinned form, no problem of the context's batches uses the
+ * tensor cores).  P2G_EINVAL for the small form on a class above 24 outputs. */
 int p2g_batch_set_forms(p2g_ctx *ctx, const int *forms);
 
 /* Size of the fixed device scratch array behind p2g_encode_noalloc. */

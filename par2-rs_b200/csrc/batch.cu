@@ -1279,9 +1279,11 @@ int p2g_batch_set_forms(p2g_ctx *ctx, const int *forms)
             return P2G_EINVAL;
         }
     }
-    for (int c = 0; c < 8; ++c)
+    ctx->batch_pinned = false;
+    for (int c = 0; c < 8; ++c) {
         ctx->batch_forms[c] = forms ? forms[c] : -1;
-    ctx->batch_pinned = forms != nullptr;
+        ctx->batch_pinned = ctx->batch_pinned || ctx->batch_forms[c] != -1;
+    }
     return P2G_OK;
 }
 

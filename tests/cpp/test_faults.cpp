@@ -10,6 +10,7 @@
 
 #include <map>
 #include <mutex>
+#include <string>
 #include <vector>
 
 #include "../../par2-rs_b200/csrc/common.cuh"
@@ -27,6 +28,27 @@ struct Copy {
     size_t n;
 };
 std::vector<Copy> g_pending;
+
+// launches by kernel (the library registers its kernels before main starts)
+std::map<const void *, std::string> &kernels()
+{
+    static std::map<const void *, std::string> m;
+    return m;
+}
+std::map<std::string, int> g_launches;
+cudaError_t launched(const void *fn)
+{
+    ++g_launches[kernels()[fn]];
+    return cudaSuccess;
+}
+int launches(const char *part)
+{
+    int n = 0;
+    for (const auto &x : g_launches)
+        if (x.first.find(part) != std::string::npos)
+            n += x.second;
+    return n;
+}
 
 void land()
 {
@@ -153,9 +175,24 @@ OK(cudaEventDestroy, cudaEvent_t)
 OK(cudaEventRecord, cudaEvent_t, cudaStream_t)
 OK(cudaEventQuery, cudaEvent_t)
 OK(cudaFuncSetAttribute, const void *, cudaFuncAttribute, int)
-OK(cudaLaunchKernel, const void *, dim3, dim3, void **, size_t, cudaStream_t)
-OK(cudaLaunchKernelExC, const cudaLaunchConfig_t *, const void *, void **)
 #undef OK
+cudaError_t cudaLaunchKernel(const void *fn, dim3, dim3, void **, size_t, cudaStream_t) { return launched(fn); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *fn, void **) { return launched(fn); }
+void **__cudaRegisterFatBinary(void *)
+{
+    static void *handle;
+    return &handle;
+}
+void __cudaRegisterFatBinaryEnd(void **) {}
+void __cudaUnregisterFatBinary(void **) {}
+void __cudaRegisterFunction(void **, const char *host, char *, const char *name, int, uint3 *, uint3 *, dim3 *, dim3 *,
+                            int *)
+{
+    kernels()[host] = name;
+}
+void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
+unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void *) { return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3 *, dim3 *, size_t *, void *) { return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned)
 {
     static char stream;
@@ -215,6 +252,46 @@ static int repair_sync(p2g_ctx *ctx)
     return 0;
 }
 
+// A batch of one CREATE job; returns p2g_batch_create's or p2g_batch_run's code.
+static int run_create(p2g_ctx *ctx, const std::vector<uint8_t *> &src, const std::vector<uint8_t *> &out, size_t S)
+{
+    std::vector<uint32_t> exps(out.size());
+    for (size_t i = 0; i < exps.size(); ++i)
+        exps[i] = static_cast<uint32_t>(i);
+    p2g_job J = {};
+    J.kind = P2G_JOB_CREATE;
+    J.k = src.size();
+    J.slice_bytes = S;
+    J.src = src.data();
+    J.n = out.size();
+    J.exps = exps.data();
+    J.out = out.data();
+    p2g_batch *b = nullptr;
+    if (const int rc = p2g_batch_create(ctx, &J, 1, 0, &b))
+        return rc;
+    const int rc = p2g_batch_run(b);
+    p2g_batch_destroy(b);
+    return rc;
+}
+
+// Forms that are all -1 are the heuristic's, tensor cores included, as NULL is.
+static int forms(p2g_ctx *ctx)
+{
+    const size_t S = 65536;
+    const auto src = slices(2000, S), out = slices(100, S);
+    const int none[P2G_BATCH_CLASSES] = {-1, -1, -1, -1, -1, -1, -1, -1};
+    const int one[P2G_BATCH_CLASSES] = {-1, -1, -1, P2G_FORM_WIDE, -1, -1, -1, -1};
+    const int *tries[] = {nullptr, none, one, none};
+    for (const int *f : tries) {
+        CHECK(p2g_batch_set_forms(ctx, f) == P2G_OK);
+        g_launches.clear();
+        CHECK(run_create(ctx, src, out, S) == P2G_OK);
+        CHECK(launches("tensor_muladd") == (f == one ? 0 : 1));
+        CHECK(launches("muladd_persistent") == (f == one ? 1 : 0));
+    }
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -222,6 +299,8 @@ int main(int argc, char **argv)
     int rc = 2;
     if (argc == 2 && !strcmp(argv[1], "repair_sync"))
         rc = repair_sync(ctx);
+    if (argc == 2 && !strcmp(argv[1], "forms"))
+        rc = forms(ctx);
     if (rc == 0) {
         CHECK(p2g_destroy(ctx) == P2G_OK);
         printf("ok\n");
