@@ -1305,7 +1305,6 @@ int p2g_batch_autotune(p2g_ctx *ctx, int reps, int *forms_out, float *ms_out)
         set_error("p2g_batch_autotune: cudaEventCreate failed");
         return P2G_ECUDA;
     }
-    ctx->batch_pinned = false;
     // representative outputs per class pair, ten inputs per output (a set
     // of 10 % redundancy)
     static const int kOut[4] = {8, 64, 160, 420};
@@ -1330,6 +1329,10 @@ int p2g_batch_autotune(p2g_ctx *ctx, int reps, int *forms_out, float *ms_out)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    // from here on the forms are the tuner's (after a failure some are still those
+    // that the caller pinned)
+    if (rc == P2G_OK)
+        ctx->batch_pinned = false;
     return rc;
 }
 

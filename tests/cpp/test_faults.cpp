@@ -292,6 +292,22 @@ static int forms(p2g_ctx *ctx)
     return 0;
 }
 
+// A batch tuner that fails leaves the pinned forms pinned.
+static int tune_fails(p2g_ctx *ctx)
+{
+    const size_t S = 65536;
+    const auto src = slices(2000, S), out = slices(100, S);
+    const int wide[P2G_BATCH_CLASSES] = {0, 0, 0, 0, 0, 0, 0, 0};
+    CHECK(p2g_batch_set_forms(ctx, wide) == P2G_OK);
+    g_room = g_used + (1 << 20);
+    CHECK(p2g_batch_autotune(ctx, 1, nullptr, nullptr) == P2G_ENOMEM);
+    g_room = size_t(1) << 40;
+    g_launches.clear();
+    CHECK(run_create(ctx, src, out, S) == P2G_OK);
+    CHECK(launches("tensor_muladd") == 0 && launches("muladd_persistent") == 1);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -299,6 +315,8 @@ int main(int argc, char **argv)
     int rc = 2;
     if (argc == 2 && !strcmp(argv[1], "repair_sync"))
         rc = repair_sync(ctx);
+    if (argc == 2 && !strcmp(argv[1], "tune_fails"))
+        rc = tune_fails(ctx);
     if (argc == 2 && !strcmp(argv[1], "forms"))
         rc = forms(ctx);
     if (rc == 0) {
