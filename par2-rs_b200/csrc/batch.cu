@@ -780,7 +780,9 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         return take(ctx, b->recs, rec_need + 256);
     };
     if (scratch() != P2G_OK) {
-        // the tensor cores' operands take up to twice the planes' room
+        // the tensor cores' operands take several times the planes' room; what of it
+        // could be had goes back first
+        b->planes.release();
         for (Prob &p : probs)
             p.tensor = false;
         clear_error();

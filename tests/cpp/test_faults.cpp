@@ -308,6 +308,28 @@ static int tune_fails(p2g_ctx *ctx)
     return 0;
 }
 
+// A batch whose tensor-core operands do not fit falls back to the tables, also where
+// the first of the two buffers did fit (and would leave no room for the tables').
+static int batch_room(p2g_ctx *&ctx)
+{
+    const size_t S = 65536;
+    const auto src = slices(2000, S), out = slices(100, S);
+    // forms 252 MB and coefficients 6.9 MB; planes 131 MB and records 6.4 MB; each
+    // with a quarter of headroom
+    for (const size_t mb : {1000, 318, 200}) {
+        g_room = g_used + mb * 1000000;
+        g_launches.clear();
+        CHECK(run_create(ctx, src, out, S) == P2G_OK);
+        CHECK(launches("tensor_muladd") == (mb == 1000 ? 1 : 0));
+        CHECK(launches("muladd_persistent") == (mb == 1000 ? 0 : 1));
+        // a fresh context: no spare buffers
+        CHECK(p2g_destroy(ctx) == P2G_OK);
+        g_room = size_t(1) << 40;
+        CHECK(p2g_create(0, &ctx) == P2G_OK);
+    }
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -317,6 +339,8 @@ int main(int argc, char **argv)
         rc = repair_sync(ctx);
     if (argc == 2 && !strcmp(argv[1], "tune_fails"))
         rc = tune_fails(ctx);
+    if (argc == 2 && !strcmp(argv[1], "batch_room"))
+        rc = batch_room(ctx);
     if (argc == 2 && !strcmp(argv[1], "forms"))
         rc = forms(ctx);
     if (rc == 0) {
