@@ -1505,7 +1505,11 @@ int muladd_autotune(p2g_ctx *ctx, int nin, int nout, size_t S, int reps, MuladdP
                 tensor_split = ns;
             }
         }
-        if (rc == P2G_OK && tensor_ms < best_t + planes_ms) {
+        if (rc == P2G_ENOMEM) {
+            // no room for the tensor cores' operands: the table plans stand
+            clear_error();
+            rc = P2G_OK;
+        } else if (rc == P2G_OK && tensor_ms < best_t + planes_ms) {
             best_p = op.plan;
             best_p.nsplit = tensor_split;
             best_t = tensor_ms;

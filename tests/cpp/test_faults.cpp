@@ -330,6 +330,20 @@ static int batch_room(p2g_ctx *&ctx)
     return 0;
 }
 
+// An autotuner without room for the tensor cores' operands tunes the tables.
+static int tune_room(p2g_ctx *ctx)
+{
+    // planes 134 MB and records 6.3 MB; coefficients for the tensor cores 31 MB
+    p2g_plan plan;
+    g_room = g_used + 150000000;
+    CHECK(p2g_autotune(ctx, 65535, 1, 64, 1, &plan) == P2G_OK);
+    CHECK(plan.tile_symbols == 1024 && !strcmp(p2g_last_error(), ""));
+    // less than the tables take is still an error
+    g_room = g_used + (1 << 20);
+    CHECK(p2g_autotune(ctx, 65535, 30, 4096, 1, &plan) == P2G_ENOMEM);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -341,6 +355,8 @@ int main(int argc, char **argv)
         rc = tune_fails(ctx);
     if (argc == 2 && !strcmp(argv[1], "batch_room"))
         rc = batch_room(ctx);
+    if (argc == 2 && !strcmp(argv[1], "tune_room"))
+        rc = tune_room(ctx);
     if (argc == 2 && !strcmp(argv[1], "forms"))
         rc = forms(ctx);
     if (rc == 0) {
