@@ -288,6 +288,12 @@ typedef struct p2g_batch p2g_batch;
  * pointers are device pointers; `jobs` must outlive the batch. */
 int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags,
                      p2g_batch **out);
+/* Device scratch that a job of these sizes takes in a batch, apart from its slices:
+ * converted slices and coefficients on the lookup tables or, where the tensor cores
+ * may take it, in their larger form, and a REPAIR's right-hand sides (VERIFY: the
+ * checksums; n unused).  A batch takes the sum over its jobs, the buffers a quarter
+ * larger than needed when they are allocated.  0 for sizes that no job can have. */
+size_t p2g_batch_job_bytes(int kind, size_t k, size_t n, size_t slice_bytes);
 /* Runs (or replays) the batch and waits for it; fills statuses and hashes. */
 int p2g_batch_run(p2g_batch *batch);
 /* Starts the batch without waiting; p2g_batch_wait completes it.  A batch whose

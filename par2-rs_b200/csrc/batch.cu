@@ -255,16 +255,19 @@ int split_for(double unit, double target, int nin, size_t S)
     return std::max(1, static_cast<int>(ns));
 }
 
-// The tile form for a problem: the context's tuned form for its class if
-// there is one, else small tables up to 24 outputs, the paired form above
-// 104 (one table build per input serves up to 208 outputs) and the 8 + 8
-// tables over 1024-symbol tiles between.
+// The tile form for a problem without a tuned or pinned one: small tables up to 24
+// outputs, the paired form above 104 (one table build per input serves up to 208
+// outputs) and the 8 + 8 tables over 1024-symbol tiles between.
+int default_form(int nout)
+{
+    return nout <= 24 ? kFormSmall : nout > 104 ? kFormPaired : kFormWide;
+}
+
+// The tile form for a problem: the context's for its class if there is one.
 int form_for(const p2g_ctx *ctx, int nout, size_t S)
 {
     const int f = ctx->batch_forms[batch_class(nout, S)];
-    if (batch_form_valid(f, nout))
-        return f;
-    return nout <= 24 ? kFormSmall : nout > 104 ? kFormPaired : kFormWide;
+    return batch_form_valid(f, nout) ? f : default_form(nout);
 }
 
 // SM clocks per 256 symbols of a problem in the persistent kernel, planes
@@ -273,6 +276,12 @@ int form_for(const p2g_ctx *ctx, int nout, size_t S)
 double table_pair_clocks(int nin, int nout)
 {
     return nin * (nout <= 24 ? 160.0 + 13.0 * nout : 300.0 + 9.7 * nout);
+}
+
+// Clocks that the tensor cores save per 256 symbols of a problem, less the margin.
+double tensor_gain(int nin, int nout)
+{
+    return table_pair_clocks(nin, nout) - 1.12 * tensor_pair_clocks(nin, nout);
 }
 
 // Marks the problems of a phase that the tensor cores take: those they are
@@ -287,7 +296,7 @@ void mark_tensor(const p2g_ctx *ctx, std::vector<Prob> &probs, int phase)
         if (p.phase != phase)
             continue;
         const double pairs = static_cast<double>((p.S + 511) / 512);
-        const double gain = table_pair_clocks(p.nin, p.nout) - 1.12 * tensor_pair_clocks(p.nin, p.nout);
+        const double gain = tensor_gain(p.nin, p.nout);
         p.tensor = gain > 0 && !ctx->batch_pinned;
         if (p.tensor)
             saved += gain * pairs / sms;
@@ -438,6 +447,32 @@ int tune_class(p2g_ctx *ctx, int cls, int nin, int nout, size_t S, int copies, i
 }  // namespace
 
 extern "C" {
+
+size_t p2g_batch_job_bytes(int kind, size_t k, size_t n, size_t slice_bytes)
+{
+    const bool repair = kind == P2G_JOB_REPAIR;
+    if (kind == P2G_JOB_VERIFY)
+        return k * 20;
+    if ((kind != P2G_JOB_CREATE && !repair) || k == 0 || k > 65535 || n == 0 || n > (repair ? k : 65535))
+        return 0;
+    Prob p{};
+    p.nin = static_cast<int>(k);
+    p.nout = static_cast<int>(n);
+    p.S = slice_bytes;
+    p.form = default_form(p.nout);
+    // on the tables, and on the tensor cores where those may take a pass: a REPAIR's
+    // two take the same buffers in turn
+    size_t planes = planes_need(p), recs = recs_need(p);
+    p.tensor = true;
+    for (const size_t nin : {repair ? k - n : k, repair ? n : k}) {
+        p.nin = static_cast<int>(nin);
+        if (nin == 0 || tensor_gain(p.nin, p.nout) <= 0)
+            continue;
+        planes = std::max(planes, planes_need(p));
+        recs = std::max(recs, recs_need(p));
+    }
+    return planes + recs + (repair ? n * al16(slice_bytes) : 0);
+}
 
 int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, p2g_batch **out)
 {

@@ -63,6 +63,7 @@ SIGNATURES = [
     ("p2g_muladd_shuffle2x", _I, [_P, _P, _P, _S, _U16]),
     ("p2g_muladd_region_shuffle2x", _I, [_P, _P, _S, _P, _S, _P, _S, _S]),
     ("p2g_finish_shuffle2x", _I, [_P, _P, _S]),
+    ("p2g_batch_job_bytes", _S, [_I, _S, _S, _S]),
     ("p2g_batch_create", _I, [_P, _P, _S, _U32, _P]),
     ("p2g_batch_run", _I, [_P]),
     ("p2g_batch_launch", _I, [_P]),
@@ -157,6 +158,11 @@ def par2_constants(k):
     out = np.zeros(k, np.uint16)
     check(lib().p2g_par2_constants(k, out.ctypes.data))
     return out
+
+
+def batch_job_bytes(kind, k, n, slice_bytes):
+    """Device scratch of a job in a batch, apart from its slices (no GPU needed)."""
+    return lib().p2g_batch_job_bytes(kind, k, n, slice_bytes)
 
 
 def encode_noalloc(stream, srcs, slice_bytes, exps, outs):

@@ -26,7 +26,7 @@ import time
 
 import numpy as np
 
-from . import JOB_CREATE, JOB_REPAIR, JOB_VERIFY, Batch
+from . import JOB_CREATE, JOB_REPAIR, JOB_VERIFY, Batch, batch_job_bytes
 
 TILE = 2048
 
@@ -61,15 +61,13 @@ class ServedJob:
         return self.k * self.n * cols // 2
 
     def scratch_bytes(self):
-        """What admission reserves: outputs, bit planes (whole 2 KiB tiles),
-        coefficient records (96 bytes per pair up to 24 outputs, else 32)
-        and, for a repair, the right-hand sides of its first pass."""
+        """What admission reserves: the outputs, and what the library takes for
+        the job in a batch (its slices in the form that the kernel of its sizes
+        reads, coefficients, a repair's right-hand sides)."""
         if self.kind == "verify":
-            return self.k * 20
-        planes = self.k * (-(-self.S // 2048) * 2048)
-        records = self.k * self.n * (96 if self.n <= 24 else 32)
-        rhs = self.n * self.S if self.kind == "repair" else 0
-        return self.n * self.S + planes + records + rhs
+            return batch_job_bytes(JOB_VERIFY, self.k, 0, self.S)
+        kind = JOB_REPAIR if self.kind == "repair" else JOB_CREATE
+        return self.n * self.S + batch_job_bytes(kind, self.k, self.n, self.S)
 
 
 class _DeviceRoom:

@@ -2,7 +2,7 @@
 // the library uses (its own definitions come first in the dynamic linker's order),
 // over host memory and without running a kernel, and lets chosen ones fail.  Copies
 // back to the host land when their stream is waited for, as on a device.
-// Usage: test_faults CASE
+// Usage: test_faults CASE [ARGUMENT...]
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -222,10 +222,11 @@ cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e,
 static std::vector<uint8_t *> slices(size_t n, size_t S)
 {
     void *p = nullptr;
-    cudaMalloc(&p, n * S);
+    const size_t pitch = (S + 15) / 16 * 16;
+    cudaMalloc(&p, n * pitch);
     std::vector<uint8_t *> v(n);
     for (size_t i = 0; i < n; ++i)
-        v[i] = static_cast<uint8_t *>(p) + i * S;
+        v[i] = static_cast<uint8_t *>(p) + i * pitch;
     return v;
 }
 
@@ -344,6 +345,42 @@ static int tune_room(p2g_ctx *ctx)
     return 0;
 }
 
+// Prints the device bytes that a batch of one job takes, without the quarter of
+// headroom of its large buffers.
+static int job_bytes(p2g_ctx *ctx, const char *kind, size_t k, size_t n, size_t S)
+{
+    const bool repair = !strcmp(kind, "repair");
+    const auto src = slices(k, S), rec = slices(n, S), out = slices(n, S);
+    std::vector<uint32_t> exps(n);
+    std::vector<uint64_t> missing(n);
+    for (size_t i = 0; i < n; ++i) {
+        exps[i] = static_cast<uint32_t>(i);
+        missing[i] = i;
+    }
+    p2g_job J = {};
+    J.kind = repair ? P2G_JOB_REPAIR : P2G_JOB_CREATE;
+    J.k = k;
+    J.slice_bytes = S;
+    J.src = src.data();
+    J.n = n;
+    J.exps = exps.data();
+    J.missing = missing.data();
+    J.recovery = rec.data();
+    J.out = out.data();
+    // scratch of the context that a first batch grows (decode matrices) stays
+    p2g_batch *b = nullptr;
+    CHECK(p2g_batch_create(ctx, &J, 1, 0, &b) == P2G_OK);
+    p2g_batch_destroy(b);
+    for (p2g::DevBuf &d : ctx->spare)
+        d.release();
+    ctx->spare.clear();
+    const size_t before = g_used;
+    CHECK(p2g_batch_create(ctx, &J, 1, 0, &b) == P2G_OK);
+    printf("%zu\n", (g_used - before) / 5 * 4);
+    p2g_batch_destroy(b);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -357,6 +394,9 @@ int main(int argc, char **argv)
         rc = batch_room(ctx);
     if (argc == 2 && !strcmp(argv[1], "tune_room"))
         rc = tune_room(ctx);
+    if (argc == 6 && !strcmp(argv[1], "job_bytes"))
+        rc = job_bytes(ctx, argv[2], strtoull(argv[3], nullptr, 10), strtoull(argv[4], nullptr, 10),
+                       strtoull(argv[5], nullptr, 10));
     if (argc == 2 && !strcmp(argv[1], "forms"))
         rc = forms(ctx);
     if (rc == 0) {
