@@ -244,6 +244,7 @@ def run_ours(args, rank, world):
     plan = None
     if not args.no_autotune:
         plan = ctx.autotune(k, r, S).as_dict()
+    used = ctx.get_plan(k, r, S).as_dict()
 
     def barrier():
         if world > 1:
@@ -325,9 +326,7 @@ def run_ours(args, rank, world):
     macs = k * r * (S // 2)
     int_ops = 2.0 * macs
     alg_bytes = (k + r) * S
-    # the form that the plan names (without one: the tensor cores, but for problems
-    # of a few outputs)
-    tile = plan["tile_symbols"] if plan else 256 if r > 8 else 1024
+    tile = used["tile_symbols"]  # the kernel that the timed steps ran
     if tile == 256:
         roofline = {
             "bound": "tensor",
@@ -1002,12 +1001,13 @@ def batched_leg():
                              "out": x["t_out_batch"]})
         return jobs
 
-    # groups whose scratch (bit planes + records) fits the budget
+    # groups whose scratch fits the budget
     budget = 48 << 30
     groups, cur, used = [], [], 0
     for x in sets:
         n = x["r"] if x["create"] else x["m"]
-        need = x["k"] * x["S"] + x["k"] * n * 64
+        need = par2gpu.batch_job_bytes(par2gpu.JOB_CREATE if x["create"] else par2gpu.JOB_REPAIR,
+                                       x["k"], n, x["S"])
         if cur and used + need > budget:
             groups.append(cur)
             cur, used = [], 0

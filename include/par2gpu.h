@@ -127,6 +127,10 @@ typedef struct {
 int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int reps,
                  p2g_plan *best);
 
+/* The plan that a call of this shape uses now: the tuned or pinned one, else the
+ * heuristic's (ms 0). */
+int p2g_get_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, p2g_plan *plan);
+
 /* Pins the plan for one shape (P2G_EINVAL if the shape is not compiled or
  * does not cover nout outputs).  Problems of at most 24 outputs run the
  * small-output kernel (three smaller lookup tables per input), compiled for

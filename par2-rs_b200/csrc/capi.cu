@@ -500,6 +500,14 @@ int p2g_last_timing(p2g_ctx *ctx, p2g_timing *out)
     return P2G_OK;
 }
 
+static p2g_plan plan_of(const MuladdPlan &p, float ms)
+{
+    if (p.tensor)
+        return p2g_plan{16, p.ereg, 16, p.nblk, p.nsplit, ms, 256, kTensorStage};
+    return p2g_plan{p.warps, p.paired ? 2 * p.ereg : p.ereg, p.psplit, p.nblk, p.nsplit, ms,
+                    p.paired ? 512 : 1024, p.stage};
+}
+
 int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int reps,
                  p2g_plan *best)
 {
@@ -520,12 +528,24 @@ int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int 
     *ctx->wait_err = 0;
     P2G_TRY(muladd_autotune(ctx, static_cast<int>(nin), static_cast<int>(nout), slice_bytes,
                             reps, &p, &ms, &tried));
-    if (p.tensor) {
-        *best = p2g_plan{16, p.ereg, 16, p.nblk, p.nsplit, ms, 256, kTensorStage};
-        return P2G_OK;
+    *best = plan_of(p, ms);
+    return P2G_OK;
+}
+
+int p2g_get_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, p2g_plan *plan)
+{
+    clear_error();
+    if (!ctx || !plan || nin == 0 || nout == 0 || slice_bytes == 0 || slice_bytes % 2) {
+        set_error("p2g_get_plan: null argument, or an empty or odd-sized problem");
+        return P2G_EINVAL;
     }
-    *best = p2g_plan{p.warps, p.paired ? 2 * p.ereg : p.ereg, p.psplit, p.nblk, p.nsplit, ms,
-                     p.paired ? 512 : 1024, p.stage};
+    if (nin > 65535 || nout > 65535) {
+        set_error("p2g_get_plan: %zu x %zu beyond 65535", nin, nout);
+        return P2G_ERANGE;
+    }
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    P2G_CUDA(cudaSetDevice(ctx->device));
+    *plan = plan_of(mulop(ctx, static_cast<int>(nin), static_cast<int>(nout), slice_bytes).plan, 0.f);
     return P2G_OK;
 }
 

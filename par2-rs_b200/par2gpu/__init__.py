@@ -45,6 +45,7 @@ SIGNATURES = [
     ("p2g_last_timing", _I, [_P, _P]),
     ("p2g_autotune", _I, [_P, _S, _S, _S, _I, _P]),
     ("p2g_set_wait_limit", _I, [_P, _U32]),
+    ("p2g_get_plan", _I, [_P, _S, _S, _S, _P]),
     ("p2g_set_plan", _I, [_P, _S, _S, _S, _P]),
     ("p2g_strategy_info", _I, [_P, _P, _P]),
     ("p2g_mul_slice", _I, [_P, _U16, _P, _S, _U32]),
@@ -267,6 +268,12 @@ class Context:
         fastest as this context's plan for it; returns the Plan."""
         p = Plan()
         check(lib().p2g_autotune(self.h, nin, nout, slice_bytes, reps, ctypes.byref(p)))
+        return p
+
+    def get_plan(self, nin, nout, slice_bytes):
+        """The Plan that a call of this shape uses now (tuned, pinned or heuristic)."""
+        p = Plan()
+        check(lib().p2g_get_plan(self.h, nin, nout, slice_bytes, ctypes.byref(p)))
         return p
 
     def batch_autotune(self, reps=2):

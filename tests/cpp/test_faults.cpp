@@ -381,6 +381,36 @@ static int job_bytes(p2g_ctx *ctx, const char *kind, size_t k, size_t n, size_t 
     return 0;
 }
 
+// The plan that p2g_get_plan names is the one that calls run.
+static int get_plan(p2g_ctx *ctx)
+{
+    struct {
+        size_t k, r, S;
+    } const shapes[] = {{20, 2, 4096}, {2048, 205, 1 << 16}, {2048, 4, 1 << 16}, {256, 13, 1 << 16}, {64, 24, 1 << 16},
+                        {64, 120, 1 << 12}, {400, 150, 4096}};
+    for (const auto &x : shapes) {
+        const auto src = slices(x.k, x.S), out = slices(x.r, x.S);
+        std::vector<uint32_t> exps(x.r);
+        p2g_plan p;
+        for (int pinned = 0; pinned < 2; ++pinned) {
+            CHECK(p2g_get_plan(ctx, x.k, x.r, x.S, &p) == P2G_OK);
+            g_launches.clear();
+            CHECK(p2g_encode(ctx, src.data(), x.k, x.S, exps.data(), x.r, out.data(), P2G_DEVICE_PTRS) == P2G_OK);
+            CHECK(launches("tensor_muladd") == (p.tile_symbols == 256));
+            CHECK(launches("muladd_paired") == (p.tile_symbols == 512));
+            CHECK(launches("muladd_bitsliced") == (p.tile_symbols == 1024));
+            p.input_splits = 3;
+            CHECK(p2g_set_plan(ctx, x.k, x.r, x.S, &p) == P2G_OK);
+            p2g_plan q;
+            CHECK(p2g_get_plan(ctx, x.k, x.r, x.S, &q) == P2G_OK);
+            CHECK(!memcmp(&p, &q, sizeof p));
+        }
+    }
+    p2g_plan p;
+    CHECK(p2g_get_plan(ctx, 0, 1, 64, &p) == P2G_EINVAL && p2g_get_plan(ctx, 65536, 1, 64, &p) == P2G_ERANGE);
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -397,6 +427,8 @@ int main(int argc, char **argv)
     if (argc == 6 && !strcmp(argv[1], "job_bytes"))
         rc = job_bytes(ctx, argv[2], strtoull(argv[3], nullptr, 10), strtoull(argv[4], nullptr, 10),
                        strtoull(argv[5], nullptr, 10));
+    if (argc == 2 && !strcmp(argv[1], "get_plan"))
+        rc = get_plan(ctx);
     if (argc == 2 && !strcmp(argv[1], "forms"))
         rc = forms(ctx);
     if (rc == 0) {
