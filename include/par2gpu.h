@@ -140,7 +140,8 @@ int p2g_get_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, p2g_
  * (tile_symbols 512: 8 warps x 14-26 even, 12 warps x 16 outputs per
  * warp; with inputs_per_stage 2: 8 warps x 14/18/22/26, 12 warps x 16), and
  * problems of any size the tensor-core kernel (tile_symbols 256, one shape per
- * output count: ceil(nout / 208) blocks of equal size rounded up to 16). */
+ * output count: ceil(nout / 208) blocks of equal size rounded up to 16).  Calls
+ * whose outputs overlap their inputs run on the lookup tables whatever the plan. */
 int p2g_set_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes,
                  const p2g_plan *plan);
 
@@ -162,7 +163,8 @@ int p2g_muladd(p2g_ctx *ctx, uint16_t *dst, const uint16_t *src, size_t n, uint1
  * target of gf_muladd_block_regions (galois/region/mod.rs:195-242):
  *   dsts[d][off .. off+len) ^= sum_s coeff_rows[d][s] * srcs[s][off .. off+len)
  * with coeff_rows[d] an array of nsrc coefficients (coefficients[dst][src]),
- * off and len in u16 units. */
+ * off and len in u16 units.  Device destinations may overlap the sources: all of
+ * them are read before one is written. */
 int p2g_muladd_region(p2g_ctx *ctx, uint16_t *const *dsts, size_t ndst,
                       const uint16_t *const *srcs, size_t nsrc,
                       const uint16_t *const *coeff_rows, size_t off_u16, size_t len_u16,

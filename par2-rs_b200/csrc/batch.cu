@@ -272,7 +272,9 @@ int form_for(const p2g_ctx *ctx, int nout, size_t S)
 
 // SM clocks per 256 symbols of a problem in the persistent kernel, planes
 // included, from launches of many waves: per input 160 + 13 per output with the
-// small tables, else 300 + 9.7 per output.
+// small tables, else 300 + 9.7 per output.  (A quarter of table_clocks' figures for
+// 1024 symbols in muladd.cu, 460 + 52 and 1020 + 39 per output, and 45 for the
+// planes: a refit of one is one of the other.)
 double table_pair_clocks(int nin, int nout)
 {
     return nin * (nout <= 24 ? 160.0 + 13.0 * nout : 300.0 + 9.7 * nout);
