@@ -133,9 +133,9 @@ __device__ void load_exp_table(uint16_t *sexp, const uint16_t *__restrict__ gexp
 // thread) when A is singular.  Each elimination step takes the logs of the
 // pivot row (lrow, 2n entries) and of the row factors (fcol) once, so every
 // product of the row updates is one lookup in the shared antilog table sexp.
-__device__ bool cta_gauss_jordan(uint16_t *S, int n, int ld, uint32_t *fcol, uint32_t *lrow,
-                                 const uint16_t *sexp, const uint16_t *__restrict__ glog,
-                                 const uint16_t *__restrict__ gexp)
+__device__ __forceinline__ bool cta_gauss_jordan(uint16_t *S, int n, int ld, uint32_t *fcol, uint32_t *lrow,
+                                                 const uint16_t *sexp, const uint16_t *__restrict__ glog,
+                                                 const uint16_t *__restrict__ gexp)
 {
     __shared__ int piv;
     const int tid = threadIdx.x, nt = blockDim.x, w2 = 2 * n;
@@ -221,7 +221,11 @@ __global__ void __launch_bounds__(kGjThreads)
         S[idx] = M[static_cast<size_t>(r) * W + j];
     }
     __syncthreads();
-    if (!cta_gauss_jordan(S, m, 2 * m, fcol, lrow, copied ? sexp : gexp, glog, gexp)) {
+    // two calls: through one pointer to either table the lookups are generic loads
+    // (96 x 96 1.20 ms that way, 1.12 this; 51 x 51 284 and 272 us)
+    const bool regular = copied ? cta_gauss_jordan(S, m, 2 * m, fcol, lrow, sexp, glog, gexp)
+                                : cta_gauss_jordan(S, m, 2 * m, fcol, lrow, gexp, glog, gexp);
+    if (!regular) {
         if (threadIdx.x == 0)
             *status = 1;
         return;
