@@ -1132,7 +1132,7 @@ static int repair_unattended(p2g_ctx *ctx, GjWork &w, size_t m, size_t np, size_
             ctx->stream = ctx->side_stream;
         }
         const int inverted = gj_invert(ctx, w, n, reinterpret_cast<const uint16_t *>(dp + L.a_off),
-                                       d_exps, exps, nullptr, ctx->inv.as<uint16_t>());
+                                       d_exps, exps, nullptr, ctx->inv.as<uint16_t>(), side);
         ctx->stream = main;
         P2G_TRY(inverted);
         inverting = true;

@@ -837,12 +837,20 @@ static bool exps_are_run(const uint32_t *exps, int m, uint32_t *s)
     return true;
 }
 
+// An inversion that is waited for goes to one CTA up to this size: its chain grows
+// with m squared, the launches' with its logarithm (a call that reads the matrix
+// back, one CTA against launches: m = 48 79 / 82 us, 56 80 / 84, 64 86 / 84, 96 124 /
+// 97, 128 176 / 102).  One that runs beside other work takes one CTA as far as that
+// goes, since what counts there is the launches (64 of 640 slices of 64 KiB 211 / 226,
+// 96 of 960 263 / 266).
+constexpr int kVdmOneCta = 56;
+
 static int vdm_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x, const uint32_t *d_exps,
-                      uint32_t s, uint16_t *d_inv, int ld)
+                      uint32_t s, uint16_t *d_inv, int ld, bool beside = false)
 {
     const size_t vec = (static_cast<size_t>(m) * 2 + 255) & ~static_cast<size_t>(255);
     P2G_TRY(w.status.ensure(256 + 5 * vec));
-    if (m <= kVdmSmall)
+    if (m <= (beside ? kVdmSmall : kVdmOneCta))
         return launch_vdm_small(ctx, SmallInverse{d_x, d_exps, d_inv, w.status.as<int>(), s, m, ld}, nullptr, 1);
     P2G_TRY(w.M.ensure(static_cast<size_t>(m) * m * 2 + 16));
     uint8_t *aux = w.status.as<uint8_t>();
@@ -1107,13 +1115,13 @@ static int woodbury_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x,
 
 
 int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uint32_t *d_exps,
-              const uint32_t *h_exps, const uint16_t *d_A, uint16_t *d_inv)
+              const uint32_t *h_exps, const uint16_t *d_A, uint16_t *d_inv, bool beside)
 {
     if (m <= 0)
         return P2G_OK;
     uint32_t s = 0;
     if (!d_A && h_exps && exps_are_run(h_exps, m, &s))
-        return vdm_invert(ctx, w, m, d_cmiss, d_exps, s, d_inv, m);
+        return vdm_invert(ctx, w, m, d_cmiss, d_exps, s, d_inv, m, beside);
     WoodburyPlan wp;
     if (!d_A && h_exps && m > kSmallM && plan_woodbury(h_exps, m, &wp))
         return woodbury_invert(ctx, w, m, d_cmiss, wp, d_inv);

@@ -16,8 +16,9 @@ struct GjWork {
 // (row-major m x m).  h_exps (optional) is a host copy of the exponents: when
 // they are a permutation of consecutive values, the closed-form Vandermonde
 // inverse replaces the elimination.  Singularity is reported by gj_status.
+// beside: it runs beside other work, on few SMs and in few launches if it can.
 int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uint32_t *d_exps,
-              const uint32_t *h_exps, const uint16_t *d_A, uint16_t *d_inv);
+              const uint32_t *h_exps, const uint16_t *d_A, uint16_t *d_inv, bool beside = false);
 
 // Inverses that the closed form makes in one CTA each, in one launch: m
 // consecutive exponents from s on, in any order (small_inverse says whether and

@@ -411,6 +411,52 @@ static int get_plan(p2g_ctx *ctx)
     return 0;
 }
 
+// Closed-form inverses: one CTA up to 56 rows where the call waits for them, up to 96
+// beside a repair's first pass, up to 128 where repairs of a batch share the launch.
+static int inverse_routes(p2g_ctx *ctx)
+{
+    const size_t S = 4096;
+    for (const size_t m : {1, 56, 57, 96, 97, 128, 129}) {
+        const size_t k = 3 * m + 5;
+        std::vector<uint64_t> missing(m);
+        std::vector<uint32_t> exps(m);
+        std::vector<uint16_t> inv(m * m);
+        for (size_t i = 0; i < m; ++i) {
+            missing[i] = 2 * i;
+            exps[i] = static_cast<uint32_t>(i);
+        }
+        const auto present = slices(k - m, S), rec = slices(m, S), out = slices(m, S);
+        g_launches.clear();
+        CHECK(p2g_reconstruction_matrix(ctx, k, missing.data(), m, exps.data(), inv.data()) == P2G_OK);
+        CHECK(launches("vdm_small") == (m <= 56) && launches("vdm_quotients") == (m > 56));
+        g_launches.clear();
+        CHECK(p2g_repair(ctx, k, S, missing.data(), m, present.data(), exps.data(), rec.data(), out.data(),
+                         P2G_DEVICE_PTRS) == P2G_OK);
+        CHECK(launches("vdm_small") == (m <= 96) && launches("vdm_quotients") == (m > 96));
+        p2g_job jobs[2] = {};
+        for (p2g_job &J : jobs) {
+            J.kind = P2G_JOB_REPAIR;
+            J.k = k;
+            J.slice_bytes = S;
+            J.src = present.data();
+            J.n = m;
+            J.exps = exps.data();
+            J.missing = missing.data();
+            J.recovery = rec.data();
+            J.out = out.data();
+        }
+        for (const int n : {1, 2}) {
+            p2g_batch *b = nullptr;
+            g_launches.clear();
+            CHECK(p2g_batch_create(ctx, jobs, n, 0, &b) == P2G_OK);
+            const bool one = m <= (n == 1 ? 56 : 128);
+            CHECK(launches("vdm_small") == one && launches("vdm_quotients") == (one ? 0 : n));
+            p2g_batch_destroy(b);
+        }
+    }
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -427,6 +473,8 @@ int main(int argc, char **argv)
     if (argc == 6 && !strcmp(argv[1], "job_bytes"))
         rc = job_bytes(ctx, argv[2], strtoull(argv[3], nullptr, 10), strtoull(argv[4], nullptr, 10),
                        strtoull(argv[5], nullptr, 10));
+    if (argc == 2 && !strcmp(argv[1], "inverse_routes"))
+        rc = inverse_routes(ctx);
     if (argc == 2 && !strcmp(argv[1], "get_plan"))
         rc = get_plan(ctx);
     if (argc == 2 && !strcmp(argv[1], "forms"))

@@ -10,7 +10,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 BIN = os.path.join(HERE, "cpp", "_build", "test_faults")
 
 
-@pytest.mark.parametrize("case", ["repair_sync", "forms", "tune_fails", "batch_room", "tune_room", "get_plan"])
+@pytest.mark.parametrize("case", ["repair_sync", "forms", "tune_fails", "batch_room", "tune_room", "get_plan",
+                                  "inverse_routes"])
 def test_failing_call(case):
     subprocess.run(["make", "-s", "-C", os.path.join(HERE, "cpp")], check=True)
     r = subprocess.run([BIN, case], capture_output=True, text=True, timeout=120)
