@@ -127,8 +127,9 @@ typedef struct {
 int p2g_autotune(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, int reps,
                  p2g_plan *best);
 
-/* The plan that a call of this shape uses now: the tuned or pinned one, else the
- * heuristic's (ms 0). */
+/* The plan that a call of this shape on device slices uses now: the tuned or pinned
+ * one, else the heuristic's (ms 0).  (From host memory a call without a tuned or
+ * pinned plan also weighs the parts in which its inputs come up.) */
 int p2g_get_plan(p2g_ctx *ctx, size_t nin, size_t nout, size_t slice_bytes, p2g_plan *plan);
 
 /* Pins the plan for one shape (P2G_EINVAL if the shape is not compiled or

@@ -639,7 +639,10 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
     const bool dev = flags & P2G_DEVICE_PTRS;
     // Host sources are copied in groups on the copy stream while the kernel
     // accumulates the groups already on the device (XOR into the outputs).
-    const int groups = (!dev && k >= 128) ? static_cast<int>(std::min<size_t>(p2g_ctx::kPipe, k / 64)) : 1;
+    int groups = 1;
+    MulOp op;
+    if (!dev)
+        op = mulop_upload(ctx, static_cast<int>(k), static_cast<int>(r), slice_bytes, &groups);
     std::vector<uint8_t *> s, d;
     bool s_staged = false, d_staged = false;
     P2G_TRY(stage(ctx, ctx->in_copy, src, k, slice_bytes, dev, groups == 1, s, s_staged));
@@ -652,7 +655,8 @@ int p2g_encode(p2g_ctx *ctx, const uint8_t *const *src, size_t k, size_t slice_b
     // blocks CTAs) about fills the device, so none leaves SMs idle.
     const size_t tiles = (slice_bytes + 2047) / 2048;
     int slabs = 1;
-    MulOp op = mulop(ctx, static_cast<int>(k), static_cast<int>(r), slice_bytes, slices_overlap(s, d, slice_bytes));
+    if (dev)
+        op = mulop(ctx, static_cast<int>(k), static_cast<int>(r), slice_bytes, slices_overlap(s, d, slice_bytes));
     if (groups >= 4 && d_staged) {
         const p2g::MuladdPlan tp =
             op.plan.tensor ? op.plan
@@ -1001,8 +1005,10 @@ int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missi
     // slices: present data and recovery inputs, outputs.  Host present
     // slices (128 or more) go up in groups on the copy stream instead, while
     // the inversion and the earlier groups' multiply-accumulate run.
-    const int groups =
-        (!dev && np >= 128) ? static_cast<int>(std::min<size_t>(p2g_ctx::kPipe, np / 64)) : 1;
+    RepairTail tail;
+    int groups = 1;
+    tail.op = dev ? mulop(ctx, static_cast<int>(np), static_cast<int>(m), slice_bytes)
+                  : mulop_upload(ctx, static_cast<int>(np), static_cast<int>(m), slice_bytes, &groups);
     std::vector<uint8_t *> ps, os;
     bool p_st = false, o_st = false;
     P2G_TRY(stage(ctx, ctx->in_copy, present, np, slice_bytes, dev, groups == 1, ps, p_st));
@@ -1019,8 +1025,6 @@ int p2g_repair(p2g_ctx *ctx, size_t k, size_t slice_bytes, const uint64_t *missi
     // (as in p2g_encode): what remains after the last upload is one slab's
     // passes and read-back instead of the whole second pass and the
     // read-back of every output.  Slabs about fill the device each.
-    RepairTail tail;
-    tail.op = mulop(ctx, static_cast<int>(np), static_cast<int>(m), slice_bytes);
     const size_t tiles = (slice_bytes + 2047) / 2048;
     if (groups >= 4 && o_st) {
         // the last kTailGroups groups (measured on 2048 x 1 MiB, m = 205:

@@ -1173,6 +1173,45 @@ MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S, bool in_place)
     return op;
 }
 
+// Up to 16 parts of 64 inputs or more hide the work behind the uploads.  Two things
+// are different on the tensor cores, where a part costs at least a stage of 256 inputs:
+//   * Where a part's columns do not fill the SMs, its products are dealt over
+//     several CTAs and its time is latency, whatever its inputs: 4 parts at most.
+//     (Encodes from pinned memory in 16 parts, 4 parts, and 16 with tables: 1487 x 10716
+//     B, 185 outputs 1421 / 516 / 1287 us; 2000 x 4 KiB, 200 outputs 431 / 246 / 1118;
+//     10000 x 4 KiB, 200 outputs 912 / 878 / 2154.)
+//   * Where the last part's product follows its upload in one piece (callers cut it
+//     into column slabs if there are 4 parts and two waves of columns), the tables
+//     take the problem if they end 4 % sooner by the estimates, at 55 GB/s up.  (256 x
+//     64 KiB, 13 outputs, tensor cores and tables: 421 / 402 us; 200 x 200 KiB, 40
+//     outputs 1171 / 1119; with slabs 600 x 256 KiB, 24 outputs 3004 / 3111.)
+MulOp mulop_upload(const p2g_ctx *ctx, int nin, int nout, size_t S, int *parts)
+{
+    MulOp op = mulop(ctx, nin, nout, S);
+    const int most = nin >= 128 ? std::min(p2g_ctx::kPipe, nin / 64) : 1;
+    *parts = most;
+    if (!op.plan.tensor || most == 1)
+        return op;
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : 148;
+    const size_t columns = (tensor_tiles(S) + 1) / 2 * tensor_blocks(nout);
+    if (tensor_splits(sms, (nin + most - 1) / most, nout, S) > 1)
+        *parts = std::min(most, 4);
+    if ((*parts >= 4 && 2 * columns >= 3 * static_cast<size_t>(sms)) || ctx->plans.count(plan_key(nin, nout, S)))
+        return op;
+    // the last part's product ends the call, unless all of them take longer
+    const double upload = static_cast<double>(nin) * static_cast<double>(S) * (1.9 / 55);
+    auto ends = [&](int g, double part) { return std::max(upload / g + g * part, upload + part); };
+    auto inputs = [&](int g) { return (nin + g - 1) / g; };
+    int split = 1;
+    const double tensor = ends(*parts, tensor_clocks(sms, inputs(*parts), nout, S, &split));
+    const MuladdPlan p = choose_plan(ctx, inputs(most), nout, S);
+    if (1.04 * ends(most, table_clocks(ctx, p, inputs(most), nout, S)) < tensor) {
+        op.plan = choose_plan(ctx, nin, nout, S);
+        *parts = most;
+    }
+    return op;
+}
+
 static int mulop_coefs(MulOp &op, DevBuf &buf, const CoefSource &c)
 {
     P2G_TRY(buf.ensure(op.plan.tensor ? tensor_coef_bytes(op.nin, op.nout) : record_bytes(op.nin, op.nout)));

@@ -167,6 +167,9 @@ struct MulOp {
 // tensor cores would take the inputs of a large problem in column chunks, between
 // which outputs are written.
 MulOp mulop(const p2g_ctx *ctx, int nin, int nout, size_t S, bool in_place = false);
+// mulop for inputs that come up from the host, in *parts parts that are each
+// multiplied when they have come (1: all of them at once).
+MulOp mulop_upload(const p2g_ctx *ctx, int nin, int nout, size_t S, int *parts);
 // The coefficients, which go into buf (grown as needed): a device matrix
 // [nout][nin], or consts[i]^exps[o] (the PAR2 encoding matrix,
 // par2_rs.rs:707-719).  The first mulop_run writes them, in the launch that

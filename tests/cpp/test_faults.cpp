@@ -457,6 +457,50 @@ static int inverse_routes(p2g_ctx *ctx)
     return 0;
 }
 
+// Inputs from the host: problems that upload in many small parts are not multiplied
+// in as many tensor-core launches, and go to the tables where those end sooner; where
+// the link is what takes the time, the parts stay as many as they can.
+static int upload_parts(p2g_ctx *ctx)
+{
+    struct {
+        size_t k, r, S;
+        int least, most;  // tensor_muladd launches of an encode
+    } const shapes[] = {{1487, 185, 10716, 1, 8},  {200, 40, 200 << 10, 0, 0},  {256, 13, 64 << 10, 0, 0},
+                        {1024, 102, 65536, 10, 32}, {100, 30, 64 << 10, 0, 1}};
+    for (const auto &x : shapes) {
+        std::vector<uint8_t> in(x.k * x.S), back(x.r * x.S);
+        std::vector<const uint8_t *> src(x.k);
+        std::vector<uint8_t *> out(x.r);
+        std::vector<uint32_t> exps(x.r);
+        std::vector<uint64_t> missing(x.r);
+        for (size_t i = 0; i < x.k; ++i)
+            src[i] = in.data() + i * x.S;
+        for (size_t i = 0; i < x.r; ++i) {
+            out[i] = back.data() + i * x.S;
+            exps[i] = static_cast<uint32_t>(i);
+            missing[i] = i;
+        }
+        g_launches.clear();
+        CHECK(p2g_encode(ctx, src.data(), x.k, x.S, exps.data(), x.r, out.data(), 0) == P2G_OK);
+        const int n = launches("tensor_muladd");
+        CHECK(n >= x.least && n <= x.most);
+        CHECK(n > 0 || launches("muladd_") > 0);
+        // a pinned plan is kept, whatever the parts
+        p2g_plan p;
+        CHECK(p2g_get_plan(ctx, x.k, x.r, x.S, &p) == P2G_OK);
+        CHECK(p2g_set_plan(ctx, x.k, x.r, x.S, &p) == P2G_OK);
+        g_launches.clear();
+        CHECK(p2g_encode(ctx, src.data(), x.k, x.S, exps.data(), x.r, out.data(), 0) == P2G_OK);
+        CHECK((launches("tensor_muladd") > 0) == (p.tile_symbols == 256));
+        g_launches.clear();
+        CHECK(p2g_repair(ctx, x.k, x.S, missing.data(), x.r, src.data(), exps.data(), src.data(), out.data(), 0) ==
+              P2G_OK);
+        // and one launch for the second pass, or one a slab
+        CHECK(launches("tensor_muladd") <= 2 * x.most + 2);
+    }
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     p2g_ctx *ctx = nullptr;
@@ -473,6 +517,8 @@ int main(int argc, char **argv)
     if (argc == 6 && !strcmp(argv[1], "job_bytes"))
         rc = job_bytes(ctx, argv[2], strtoull(argv[3], nullptr, 10), strtoull(argv[4], nullptr, 10),
                        strtoull(argv[5], nullptr, 10));
+    if (argc == 2 && !strcmp(argv[1], "upload_parts"))
+        rc = upload_parts(ctx);
     if (argc == 2 && !strcmp(argv[1], "inverse_routes"))
         rc = inverse_routes(ctx);
     if (argc == 2 && !strcmp(argv[1], "get_plan"))

@@ -11,7 +11,7 @@ BIN = os.path.join(HERE, "cpp", "_build", "test_faults")
 
 
 @pytest.mark.parametrize("case", ["repair_sync", "forms", "tune_fails", "batch_room", "tune_room", "get_plan",
-                                  "inverse_routes"])
+                                  "inverse_routes", "upload_parts"])
 def test_failing_call(case):
     subprocess.run(["make", "-s", "-C", os.path.join(HERE, "cpp")], check=True)
     r = subprocess.run([BIN, case], capture_output=True, text=True, timeout=120)
