@@ -569,9 +569,9 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
             return fail(rc);
         std::vector<uint8_t> h;
         // inverses of one CTA each, all in one launch after the others (48 sets
-        // with 19 small repairs: one by one 0.9 ms, mostly uploads and launches); not
-        // for one alone, which takes the faster way for its size (128 of 640 slices
-        // of 4 KiB: 358 us in one CTA, 308 in launches)
+        // with 19 small repairs: one by one 0.9 ms, mostly uploads and launches); one
+        // alone only if that is the faster way for its size (128 of 640 slices of 4
+        // KiB: 358 us in one CTA, 293 in launches)
         size_t nsmall = 0;
         for (size_t j = 0; j < njobs; ++j) {
             uint32_t s = 0;
@@ -599,7 +599,7 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
             par2_constants(J.k, c.data());
             const size_t m = J.n;
             uint32_t s = 0;
-            if (nsmall > 1 && small_inverse(J.exps, static_cast<int>(m), &s)) {
+            if (small_inverse(J.exps, static_cast<int>(m), &s, nsmall == 1)) {
                 std::vector<uint16_t> x(m);
                 for (size_t q = 0; q < m; ++q)
                     x[q] = c[J.missing[q]];

@@ -1214,9 +1214,9 @@ int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uin
     return P2G_OK;
 }
 
-bool small_inverse(const uint32_t *h_exps, int m, uint32_t *s)
+bool small_inverse(const uint32_t *h_exps, int m, uint32_t *s, bool alone)
 {
-    return m > 0 && m <= kVdmSmall && exps_are_run(h_exps, m, s);
+    return m > 0 && m <= (alone ? kVdmOneCta : kVdmSmall) && exps_are_run(h_exps, m, s);
 }
 
 int small_inverses(p2g_ctx *ctx, const SmallInverse *d_items, int n)

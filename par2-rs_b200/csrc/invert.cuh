@@ -22,8 +22,9 @@ int gj_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_cmiss, const uin
 
 // Inverses that the closed form makes in one CTA each, in one launch: m
 // consecutive exponents from s on, in any order (small_inverse says whether and
-// finds s); x are the missing slices' constants, ld the row stride of inv and
-// *status becomes 1 where the matrix is singular, else 0.
+// finds s; `alone`: whether it is also the faster way for a single one); x are the
+// missing slices' constants, ld the row stride of inv and *status becomes 1 where
+// the matrix is singular, else 0.
 struct SmallInverse {
     const uint16_t *x;
     const uint32_t *exps;
@@ -32,7 +33,7 @@ struct SmallInverse {
     uint32_t s;
     int m, ld;
 };
-bool small_inverse(const uint32_t *h_exps, int m, uint32_t *s);
+bool small_inverse(const uint32_t *h_exps, int m, uint32_t *s, bool alone = false);
 int small_inverses(p2g_ctx *ctx, const SmallInverse *d_items, int n);
 
 // Whether an inversion of m rows runs in one CTA, without the multiply-accumulate
