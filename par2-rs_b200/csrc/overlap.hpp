@@ -56,23 +56,29 @@ class ByteRanges {
     bool joined_ = true;
 };
 
-// Whether any of the slices a overlaps any of the slices b, all of n bytes.  Tables
-// that lie apart as a whole, which nearly all do, cost a minimum and a maximum a
-// slice (20 and 2 slices 0.09 -> 0.02 us, 256 and 13 0.52 -> 0.27, 2048 and 205 3.8 ->
-// 2.4).
+// Whether any of the slices a (usually the more) overlaps any of the slices b, all of n
+// bytes.  Where all of a lie apart from b's address range, which is nearly always, a
+// slice costs two subtractions and two logic operations on vectors (256 and 13 slices
+// 0.52 us by ranges, 0.14 so; 2048 and 205 3.8 us, 1.0).
 template <class A, class B>
 inline bool slices_overlap(const A &a, const B &b, size_t n)
 {
-    auto bounds = [](const auto &t) {
-        uintptr_t lo = UINTPTR_MAX, hi = 0;
-        for (const auto *p : t) {
-            lo = std::min(lo, reinterpret_cast<uintptr_t>(p));
-            hi = std::max(hi, reinterpret_cast<uintptr_t>(p));
-        }
-        return std::make_pair(lo, hi);
-    };
-    const auto x = bounds(a), y = bounds(b);
-    if (x.second + n <= y.first || y.second + n <= x.first)
+    if (a.empty() || b.empty() || n == 0)
+        return false;
+    uintptr_t lo = UINTPTR_MAX, hi = 0;
+    for (const auto *p : b) {
+        lo = std::min(lo, reinterpret_cast<uintptr_t>(p));
+        hi = std::max(hi, reinterpret_cast<uintptr_t>(p));
+    }
+    // p overlaps [lo, hi + n) if x = p - (lo - n + 1) < width: the top bit of
+    // (x - width) & ~x, addresses and widths being below 2^63
+    const uintptr_t first = lo - n + 1, width = hi + n - first;
+    uintptr_t near = 0;
+    for (const auto *p : a) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(p) - first;
+        near |= (x - width) & ~x;
+    }
+    if (near >> 63 == 0)
         return false;
     ByteRanges r;
     for (const auto *p : b)
