@@ -839,11 +839,11 @@ static bool exps_are_run(const uint32_t *exps, int m, uint32_t *s)
 
 // An inversion that is waited for goes to one CTA up to this size: its chain grows
 // with m squared, the launches' with its logarithm (a call that reads the matrix
-// back, one CTA against launches: m = 48 79 / 82 us, 56 80 / 84, 64 86 / 84, 96 124 /
-// 97, 128 176 / 102).  One that runs beside other work takes one CTA as far as that
+// back, one CTA against launches: m = 48 79 / 82 us, 60 77 / 79, 64 80 / 79, 65 88 / 84,
+// 96 124 / 97, 128 176 / 102).  One that runs beside other work takes one CTA as far as that
 // goes, since what counts there is the launches (64 of 640 slices of 64 KiB 211 / 226,
 // 96 of 960 263 / 266).
-constexpr int kVdmOneCta = 56;
+constexpr int kVdmOneCta = 64;
 
 static int vdm_invert(p2g_ctx *ctx, GjWork &w, int m, const uint16_t *d_x, const uint32_t *d_exps,
                       uint32_t s, uint16_t *d_inv, int ld, bool beside = false)

@@ -411,12 +411,12 @@ static int get_plan(p2g_ctx *ctx)
     return 0;
 }
 
-// Closed-form inverses: one CTA up to 56 rows where the call waits for them, up to 96
+// Closed-form inverses: one CTA up to 64 rows where the call waits for them, up to 96
 // beside a repair's first pass, up to 128 where repairs of a batch share the launch.
 static int inverse_routes(p2g_ctx *ctx)
 {
     const size_t S = 4096;
-    for (const size_t m : {1, 56, 57, 96, 97, 128, 129}) {
+    for (const size_t m : {1, 64, 65, 96, 97, 128, 129}) {
         const size_t k = 3 * m + 5;
         std::vector<uint64_t> missing(m);
         std::vector<uint32_t> exps(m);
@@ -428,7 +428,7 @@ static int inverse_routes(p2g_ctx *ctx)
         const auto present = slices(k - m, S), rec = slices(m, S), out = slices(m, S);
         g_launches.clear();
         CHECK(p2g_reconstruction_matrix(ctx, k, missing.data(), m, exps.data(), inv.data()) == P2G_OK);
-        CHECK(launches("vdm_small") == (m <= 56) && launches("vdm_quotients") == (m > 56));
+        CHECK(launches("vdm_small") == (m <= 64) && launches("vdm_quotients") == (m > 64));
         g_launches.clear();
         CHECK(p2g_repair(ctx, k, S, missing.data(), m, present.data(), exps.data(), rec.data(), out.data(),
                          P2G_DEVICE_PTRS) == P2G_OK);
@@ -449,7 +449,7 @@ static int inverse_routes(p2g_ctx *ctx)
             p2g_batch *b = nullptr;
             g_launches.clear();
             CHECK(p2g_batch_create(ctx, jobs, n, 0, &b) == P2G_OK);
-            const bool one = m <= (n == 1 ? 56 : 128);
+            const bool one = m <= (n == 1 ? 64 : 128);
             CHECK(launches("vdm_small") == one && launches("vdm_quotients") == (one ? 0 : n));
             p2g_batch_destroy(b);
         }

@@ -22,7 +22,7 @@ def up(a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
 
 
-@pytest.mark.parametrize("m", [55, 56, 57, 64, 96])
+@pytest.mark.parametrize("m", [56, 63, 64, 65, 96])
 def test_matrix(ctx, m):
     rng = np.random.default_rng(m)
     k = 3 * m
@@ -33,7 +33,7 @@ def test_matrix(ctx, m):
     assert np.array_equal(ctx.reconstruction_matrix(k, missing, exps), want)
 
 
-@pytest.mark.parametrize("m", [56, 57, 96])
+@pytest.mark.parametrize("m", [64, 65, 96])
 def test_repair_and_lone_job(ctx, m):
     import par2gpu
     import torch
