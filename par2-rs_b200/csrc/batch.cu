@@ -708,20 +708,40 @@ int p2g_batch_create(p2g_ctx *ctx, p2g_job *jobs, size_t njobs, uint32_t flags, 
         }
         return g;
     };
-    ByteRanges written;  // by the CREATE and REPAIR jobs
+    // what the CREATE and REPAIR jobs write: the address range, and the slices' own
+    // ranges when a verification first comes near it (64 jobs, a third of them
+    // verifications: 50 us of 1.5 ms less than by the slices' ranges alone)
+    uintptr_t wlo = UINTPTR_MAX, wend = 0;
     for (size_t j = 0; j < njobs; ++j) {
         const p2g_job &J = jobs[j];
-        for (size_t e = 0; J.kind != P2G_JOB_VERIFY && e < J.n; ++e)
-            written.add(J.out[e] + J.col_begin, (J.col_end ? J.col_end : J.slice_bytes) - J.col_begin);
+        if (J.kind == P2G_JOB_VERIFY || J.n == 0)
+            continue;
+        Bounds r;
+        r.add(J.out, J.n);
+        wlo = std::min(wlo, r.lo + J.col_begin);
+        wend = std::max<uintptr_t>(wend, r.hi + (J.col_end ? J.col_end : J.slice_bytes));
     }
+    ByteRanges written;
+    bool listed = false;
+    auto list_written = [&] {
+        for (size_t j = 0; j < njobs && !listed; ++j) {
+            const p2g_job &J = jobs[j];
+            for (size_t e = 0; J.kind != P2G_JOB_VERIFY && e < J.n; ++e)
+                written.add(J.out[e] + J.col_begin, (J.col_end ? J.col_end : J.slice_bytes) - J.col_begin);
+        }
+        listed = true;
+    };
     for (size_t j = 0; j < njobs; ++j) {
         p2g_job &J = jobs[j];
         const size_t cb = J.col_begin;
         const size_t S = (J.col_end ? J.col_end : J.slice_bytes) - cb;
         if (J.kind == P2G_JOB_VERIFY) {
+            const bool near = any_in(J.src, J.k, S, wlo, wend);
+            if (near)
+                list_written();
             size_t g = 0;
             for (size_t i = 0; i < J.k; ++i) {
-                const bool after = written.overlaps(J.src[i], S);
+                const bool after = near && written.overlaps(J.src[i], S);
                 if (i == 0 || hg[g].after != after)
                     g = hash_group(S, after);
                 hg[g].slices.push_back({static_cast<int>(j), static_cast<int>(i)});

@@ -56,29 +56,46 @@ class ByteRanges {
     bool joined_ = true;
 };
 
+// The addresses from the first slice's to the last one's of a table.
+struct Bounds {
+    uintptr_t lo = UINTPTR_MAX, hi = 0;
+    template <class T>
+    void add(const T *const *t, size_t count)
+    {
+        for (size_t i = 0; i < count; ++i) {
+            lo = std::min(lo, reinterpret_cast<uintptr_t>(t[i]));
+            hi = std::max(hi, reinterpret_cast<uintptr_t>(t[i]));
+        }
+    }
+};
+
+// Whether any of `count` slices of n bytes has a byte in [lo, end): p does if x = p -
+// (lo - n + 1) < width, that is the top bit of (x - width) & ~x, addresses and widths
+// being below 2^63 (so written for the compiler's vectors: 0.4 ns a slice).
+template <class T>
+inline bool any_in(const T *const *t, size_t count, size_t n, uintptr_t lo, uintptr_t end)
+{
+    if (lo >= end || n == 0)
+        return false;
+    const uintptr_t first = lo - n + 1, width = end - first;
+    uintptr_t near = 0;
+    for (size_t i = 0; i < count; ++i) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(t[i]) - first;
+        near |= (x - width) & ~x;
+    }
+    return near >> 63 != 0;
+}
+
 // Whether any of the slices a (usually the more) overlaps any of the slices b, all of n
-// bytes.  Where all of a lie apart from b's address range, which is nearly always, a
-// slice costs two subtractions and two logic operations on vectors (256 and 13 slices
-// 0.52 us by ranges, 0.14 so; 2048 and 205 3.8 us, 1.0).
+// bytes.  Where all of a lie apart from b's address range, which is nearly always, that
+// is all there is to compare (256 and 13 slices 0.52 us by ranges, 0.14 so; 2048 and 205
+// 3.8 us, 1.0).
 template <class A, class B>
 inline bool slices_overlap(const A &a, const B &b, size_t n)
 {
-    if (a.empty() || b.empty() || n == 0)
-        return false;
-    uintptr_t lo = UINTPTR_MAX, hi = 0;
-    for (const auto *p : b) {
-        lo = std::min(lo, reinterpret_cast<uintptr_t>(p));
-        hi = std::max(hi, reinterpret_cast<uintptr_t>(p));
-    }
-    // p overlaps [lo, hi + n) if x = p - (lo - n + 1) < width: the top bit of
-    // (x - width) & ~x, addresses and widths being below 2^63
-    const uintptr_t first = lo - n + 1, width = hi + n - first;
-    uintptr_t near = 0;
-    for (const auto *p : a) {
-        const uintptr_t x = reinterpret_cast<uintptr_t>(p) - first;
-        near |= (x - width) & ~x;
-    }
-    if (near >> 63 == 0)
+    Bounds y;
+    y.add(b.data(), b.size());
+    if (b.empty() || !any_in(a.data(), a.size(), n, y.lo, y.hi + n))
         return false;
     ByteRanges r;
     for (const auto *p : b)
